@@ -29,8 +29,10 @@
 //   * windows that do not overlap (stride >= kernel in every dimension):
 //     one thread per window recomputes its winner and writes each element
 //     of the window's cell once (read X and dY once, write dX once);
-//   * overlapping windows: one thread per input element visits the windows
-//     that contain it in output order, the order of Owl's `+=` sequence.
+//   * overlapping windows: a block owns a tile of input elements, computes
+//     each window that touches it once (winner and dY, or dY / count) into
+//     shared memory, and every element then adds the windows that contain it
+//     in output order, the order of Owl's `+=` sequence.
 // A max window in which no element beats -inf routes its gradient to flat
 // element 0 in Owl; such windows are detected on the device and element 0
 // is then rebuilt by an ordered fix-up pass.
@@ -83,6 +85,25 @@ struct OutDecode {
 OutDecode make_out_decode(const PG &g, int64_t cv) {
   return OutDecode{make_fastdiv((uint32_t)cv), make_fastdiv((uint32_t)g.OD),
                    make_fastdiv((uint32_t)g.OR), make_fastdiv((uint32_t)g.OC)};
+}
+
+struct OutPos {
+  uint32_t p, cv;  // output pixel and channel vector
+  int b, oc, orr, od;
+};
+
+__device__ __forceinline__ OutPos out_pos(const OutDecode &dec, uint32_t idx) {
+  OutPos o;
+  o.p = fdiv(idx, dec.cv);
+  o.cv = idx - o.p * dec.cv.d;
+  const uint32_t t1 = fdiv(o.p, dec.od);
+  o.od = (int)(o.p - t1 * dec.od.d);
+  const uint32_t t2 = fdiv(t1, dec.orr);
+  o.orr = (int)(t1 - t2 * dec.orr.d);
+  const uint32_t t3 = fdiv(t2, dec.oc);
+  o.oc = (int)(t2 - t3 * dec.oc.d);
+  o.b = (int)t3;
+  return o;
 }
 
 template <typename T, int V>
@@ -222,6 +243,7 @@ template <typename T, int V, int MODE, bool ARG>
 __global__ void __launch_bounds__(256) pool_fwd_kernel(PG g, const T *__restrict__ x,
                                                        T *__restrict__ y,
                                                        int64_t *__restrict__ argmax) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched with launch_pdl
   const int64_t CV = g.Ch / V;
   const int64_t total = g.B * g.OC * g.OR * g.OD * CV;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -291,6 +313,7 @@ __global__ void __launch_bounds__(256) pool_bwd_cell_kernel(PG g, const T *__res
                                                             T *__restrict__ dx,
                                                             unsigned long long ticket) {
   asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched with launch_pdl
   const int64_t CV = g.Ch / V;
   const int64_t total = g.B * g.OC * g.OR * g.OD * CV;
   bool degen = false;
@@ -340,65 +363,81 @@ __global__ void __launch_bounds__(256) pool_bwd_cell_kernel(PG g, const T *__res
 
 // ---- fixed-window fast paths ----------------------------------------------
 
-// Windows of compile-time size KC x KR x KD that lie wholly inside the input
-// (no padding, (O-1)*s + k <= I in every dimension): the taps are constant
-// strides apart, every tap of a window is loaded before the reduction, and
-// nothing is clipped.  Same scan order and comparisons as the general path.
+// Windows of compile-time size KC x KR x KD: a window wholly inside the input
+// has its taps constant strides apart and loads them all before the
+// reduction; one that the border clips (SAME padding) walks its in-range taps
+// as the general kernel does.  Same scan order and comparisons either way.
+// HBM-bound.  3x3 stride 2 SAME on [16;112;112;64] (64 MB): 22.6 us when its
+// clipped windows sent every window to the general kernel, 13.8 us here.
 template <typename T, int V, int KC, int KR, int KD, int MODE, bool ARG>
 __global__ void __launch_bounds__(256) pool_fwd_fixed_kernel(PG g, OutDecode dec,
                                                              const T *__restrict__ x,
                                                              T *__restrict__ y,
                                                              int64_t *__restrict__ argmax) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched with launch_pdl
   constexpr int N = KC * KR * KD;
   const uint32_t total = (uint32_t)(g.B * g.OC * g.OR * g.OD * (g.Ch / V));
   const int64_t sd = g.Ch, sr = g.ID * g.Ch, sc = g.IR * g.ID * g.Ch;
   for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += gridDim.x * blockDim.x) {
-    const uint32_t p32 = fdiv(idx, dec.cv);
-    const int64_t cv = idx - p32 * dec.cv.d, p = p32;
-    const uint32_t t1 = fdiv(p32, dec.od);
-    const int od = (int)(p32 - t1 * dec.od.d);
-    const uint32_t t2 = fdiv(t1, dec.orr);
-    const int orr = (int)(t1 - t2 * dec.orr.d);
-    const uint32_t t3 = fdiv(t2, dec.oc);
-    const int oc = (int)(t2 - t3 * dec.oc.d);
-    const int64_t b = t3;
-    const int64_t base = b * g.IC * sc + (int64_t)oc * g.sc * sc + (int64_t)orr * g.sr * sr +
-                         (int64_t)od * g.sd * sd + cv * V;
-    T v[N][V];
-#pragma unroll
-    for (int a = 0; a < KC; ++a)
-#pragma unroll
-      for (int bb = 0; bb < KR; ++bb)
-#pragma unroll
-        for (int c = 0; c < KD; ++c)
-          load_vec<T, V>(x + base + a * sc + bb * sr + c * sd, v[(a * KR + bb) * KD + c]);
+    const OutPos o = out_pos(dec, idx);
+    const int64_t cv = o.cv, p = o.p;
+    const int c0 = o.oc * g.sc - g.pc, r0 = o.orr * g.sr - g.pr, d0 = o.od * g.sd - g.pd;
+    const int64_t xbase = (int64_t)o.b * g.IC * sc;
     T out[V];
-    if (MODE == POOL_MAX) {
-      int bt[V];
+    int bt[V];
+    if (c0 >= 0 && c0 + KC <= g.IC && r0 >= 0 && r0 + KR <= g.IR && d0 >= 0 &&
+        d0 + KD <= g.ID) {
+      const int64_t base = xbase + c0 * sc + r0 * sr + d0 * sd + cv * V;
+      T v[N][V];
 #pragma unroll
-      for (int i = 0; i < V; ++i) { out[i] = T(-INFINITY); bt[i] = -1; }
+      for (int a = 0; a < KC; ++a)
 #pragma unroll
-      for (int u = 0; u < N; ++u)
+        for (int bb = 0; bb < KR; ++bb)
 #pragma unroll
-        for (int i = 0; i < V; ++i)
-          if (out[i] < v[u][i]) { out[i] = v[u][i]; bt[i] = u; }
-      if (ARG) {
+          for (int c = 0; c < KD; ++c)
+            load_vec<T, V>(x + base + a * sc + bb * sr + c * sd, v[(a * KR + bb) * KD + c]);
+      if (MODE == POOL_MAX) {
 #pragma unroll
-        for (int i = 0; i < V; ++i) {
-          const int a = bt[i] / (KR * KD), bb = bt[i] / KD % KR, c = bt[i] % KD;
-          argmax[p * g.Ch + cv * V + i] = bt[i] < 0 ? -1 : base + a * sc + bb * sr + c * sd + i;
+        for (int i = 0; i < V; ++i) { out[i] = T(-INFINITY); bt[i] = -1; }
+#pragma unroll
+        for (int u = 0; u < N; ++u)
+#pragma unroll
+          for (int i = 0; i < V; ++i)
+            if (out[i] < v[u][i]) { out[i] = v[u][i]; bt[i] = u; }
+        if (ARG) {
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            const int a = bt[i] / (KR * KD), bb = bt[i] / KD % KR, c = bt[i] % KD;
+            argmax[p * g.Ch + cv * V + i] =
+                bt[i] < 0 ? -1 : base + a * sc + bb * sr + c * sd + i;
+          }
         }
+      } else {
+#pragma unroll
+        for (int i = 0; i < V; ++i) out[i] = T(0);
+#pragma unroll
+        for (int u = 0; u < N; ++u)
+#pragma unroll
+          for (int i = 0; i < V; ++i) out[i] += v[u][i];
+#pragma unroll
+        for (int i = 0; i < V; ++i) out[i] = div_count(out[i], N);
       }
     } else {
+      const Box w = window_box(g, o.oc, o.orr, o.od);
+      if (MODE == POOL_MAX) {
+        window_max<T, V, 1>(x, xbase + cv * V, g, w, out, bt);
+        if (ARG) {
 #pragma unroll
-      for (int i = 0; i < V; ++i) out[i] = T(0);
+          for (int i = 0; i < V; ++i)
+            argmax[p * g.Ch + cv * V + i] =
+                bt[i] < 0 ? -1 : tap_offset(g, xbase, w, bt[i]) + cv * V + i;
+        }
+      } else {
+        window_sum<T, V, 1>(x, xbase + cv * V, g, w, out);
 #pragma unroll
-      for (int u = 0; u < N; ++u)
-#pragma unroll
-        for (int i = 0; i < V; ++i) out[i] += v[u][i];
-#pragma unroll
-      for (int i = 0; i < V; ++i) out[i] = div_count(out[i], N);
+        for (int i = 0; i < V; ++i) out[i] = div_count(out[i], w.n);
+      }
     }
     store_vec<T, V>(y + p * g.Ch + cv * V, out);
   }
@@ -413,23 +452,17 @@ __global__ void __launch_bounds__(256) pool_bwd_tile_kernel(PG g, OutDecode dec,
                                                             T *__restrict__ dx,
                                                             unsigned long long ticket) {
   asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched with launch_pdl
   constexpr int N = KC * KR * KD;
   const uint32_t total = (uint32_t)(g.B * g.OC * g.OR * g.OD * (g.Ch / V));
   const int64_t sd = g.Ch, sr = g.ID * g.Ch, sc = g.IR * g.ID * g.Ch;
   bool degen = false;
   for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += gridDim.x * blockDim.x) {
-    const uint32_t p32 = fdiv(idx, dec.cv);
-    const int64_t cv = idx - p32 * dec.cv.d, p = p32;
-    const uint32_t t1 = fdiv(p32, dec.od);
-    const int od = (int)(p32 - t1 * dec.od.d);
-    const uint32_t t2 = fdiv(t1, dec.orr);
-    const int orr = (int)(t1 - t2 * dec.orr.d);
-    const uint32_t t3 = fdiv(t2, dec.oc);
-    const int oc = (int)(t2 - t3 * dec.oc.d);
-    const int64_t b = t3;
-    const int64_t base = b * g.IC * sc + (int64_t)oc * KC * sc + (int64_t)orr * KR * sr +
-                         (int64_t)od * KD * sd + cv * V;
+    const OutPos o = out_pos(dec, idx);
+    const int64_t cv = o.cv, p = o.p;
+    const int64_t base = (int64_t)o.b * g.IC * sc + (int64_t)o.oc * KC * sc +
+                         (int64_t)o.orr * KR * sr + (int64_t)o.od * KD * sd + cv * V;
     T gv[V];
     load_vec<T, V>(dy + p * g.Ch + cv * V, gv);
     int bt[V];
@@ -497,6 +530,7 @@ __global__ void __launch_bounds__(256) pool_bwd_gather_kernel(PG g, const T *__r
                                                               T *__restrict__ dx,
                                                               unsigned long long ticket) {
   asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched with launch_pdl
   const int64_t CV = g.Ch / V;
   const int64_t total = g.B * g.IC * g.IR * g.ID * CV;
   bool degen = false;
@@ -542,6 +576,380 @@ __global__ void __launch_bounds__(256) pool_bwd_gather_kernel(PG g, const T *__r
     store_vec<T, V>(dx + xbase + (((int64_t)ic * g.IR + ir) * g.ID + id) * g.Ch + cv * V, acc);
   }
   if (MODE == POOL_MAX && degen) raise_mark(ticket);
+}
+
+// The tile of an overlapping backward: TC x TR x TD input elements (powers of
+// two) by CVB channel vectors; at most NWC x NWR x NWD windows touch it.
+struct OverTile {
+  int lc, lr, ld;          // log2 of the tile's extents
+  int CVB, n_cb;           // channel vectors per block, blocks of them
+  int n_c, n_r, n_d;       // tiles along each axis
+  int NWR, NWD, NW;        // window box of a tile (rows, dpts; all)
+  FastDiv nwr, nwd, cvb;
+  FastDiv sc, sr, sd;      // strides
+};
+
+// First and last window (output position) of one axis that covers any input
+// position of [i0, i1); s > 0.
+__device__ __forceinline__ void tile_windows(int i0, int i1, const FastDiv &s, int p, int k,
+                                             int O, int &lo, int &hi) {
+  const int num = i0 + p - k + 1;
+  lo = num <= 0 ? 0 : (int)fdiv((uint32_t)num + s.d - 1, s);
+  const int top = i1 - 1 + p;
+  hi = top < 0 ? -1 : min((int)fdiv((uint32_t)top, s), O - 1);
+}
+
+// Backward with overlapping windows.  One block owns a tile of input elements
+// of one batch entry and a run of channel vectors.  Phase 1 computes every
+// window that touches the tile once: its winning tap (one byte a channel) and
+// dY for max, dY / count for average, both into shared memory.  Phase 2 visits
+// for each element the windows that contain it in output order, as Owl's
+// scatter loop adds them, so the float sum is Owl's `+=` sequence without
+// atomics.  Bound: HBM (x, dy, dx once) plus L1 re-reads of x, k/s windows an
+// axis.  Recomputing each window once per element it contains (one thread per
+// element, no tile) took 315 us (max) and 80 us (average) for 3x3 stride 2 on
+// [16;112;112;64]; with the tiles 65 and 43 us, and with the compile-time windows
+// of the next kernel 31.5 and 16.0 us (HBM floor 17 and 9.5).
+template <typename T, int V, int MODE>
+__global__ void __launch_bounds__(256) pool_bwd_over_kernel(PG g, OverTile tl,
+                                                            const T *__restrict__ x,
+                                                            const T *__restrict__ dy,
+                                                            T *__restrict__ dx,
+                                                            unsigned long long ticket) {
+  extern __shared__ __align__(16) unsigned char over_smem[];
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched with launch_pdl
+  T *gbuf = reinterpret_cast<T *>(over_smem);                  // [NW][CVB][V]
+  uint8_t *code = over_smem + (size_t)tl.NW * tl.CVB * V * sizeof(T);  // [NW][CVB][V]
+  // block -> (batch, tile, channel block); channel blocks innermost
+  unsigned q = blockIdx.x;
+  const int cb = (int)(q % tl.n_cb); q /= tl.n_cb;
+  const int td = (int)(q % tl.n_d); q /= tl.n_d;
+  const int tr = (int)(q % tl.n_r); q /= tl.n_r;
+  const int tc = (int)(q % tl.n_c);
+  const int64_t b = q / tl.n_c;
+  const int i0c = tc << tl.lc, i0r = tr << tl.lr, i0d = td << tl.ld;
+  const int i1c = min(i0c + (1 << tl.lc), (int)g.IC), i1r = min(i0r + (1 << tl.lr), (int)g.IR),
+            i1d = min(i0d + (1 << tl.ld), (int)g.ID);
+  const int CV = (int)(g.Ch / V);
+  const int cv0 = cb * tl.CVB, ncv = min(tl.CVB, CV - cv0);
+  const int64_t xbase = b * g.IC * g.IR * g.ID * g.Ch, ybase = b * g.OC * g.OR * g.OD * g.Ch;
+  int wc0, wc1, wr0, wr1, wd0, wd1;
+  tile_windows(i0c, i1c, tl.sc, g.pc, (int)g.KC, (int)g.OC, wc0, wc1);
+  tile_windows(i0r, i1r, tl.sr, g.pr, (int)g.KR, (int)g.OR, wr0, wr1);
+  tile_windows(i0d, i1d, tl.sd, g.pd, (int)g.KD, (int)g.OD, wd0, wd1);
+  // threads: lane cv within the block's channel vectors, groups over windows
+  const int grp = (int)fdiv(threadIdx.x, tl.cvb), cvl = (int)threadIdx.x - grp * tl.CVB;
+  const int n_grp = (int)fdiv(blockDim.x, tl.cvb);
+  const bool on = grp < n_grp && cvl < ncv;
+  bool degen = false;
+  if (on) {
+    for (int w = grp; w < tl.NW; w += n_grp) {
+      const int t = (int)fdiv((uint32_t)w, tl.nwd), kd = w - t * tl.NWD;
+      const int kc = (int)fdiv((uint32_t)t, tl.nwr), kr = t - kc * tl.NWR;
+      const int oc = wc0 + kc, orr = wr0 + kr, od = wd0 + kd;
+      if (oc > wc1 || orr > wr1 || od > wd1) continue;
+      const Box wb = window_box(g, oc, orr, od);
+      T gv[V];
+      load_vec<T, V>(dy + ybase + (((int64_t)oc * g.OR + orr) * g.OD + od) * g.Ch +
+                         (int64_t)(cv0 + cvl) * V, gv);
+      const int at = (w * tl.CVB + cvl) * V;
+      if (MODE == POOL_MAX) {
+        T best[V];
+        int bt[V];
+        window_max<T, V, kChunk + 1>(x, xbase + (int64_t)(cv0 + cvl) * V, g, wb, best, bt);
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          degen |= bt[i] < 0;
+          code[at + i] = bt[i] < 0 ? 255 : (uint8_t)bt[i];
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < V; ++i) gv[i] = div_count(gv[i], wb.n);
+      }
+      store_vec<T, V>(gbuf + at, gv);
+    }
+  }
+  if (MODE == POOL_MAX && degen) raise_mark(ticket);
+  __syncthreads();
+  if (!on) return;
+  const int ne = 1 << (tl.lc + tl.lr + tl.ld);
+  for (int e = grp; e < ne; e += n_grp) {
+    const int id = i0d + (e & ((1 << tl.ld) - 1));
+    const int ir = i0r + ((e >> tl.ld) & ((1 << tl.lr) - 1));
+    const int ic = i0c + (e >> (tl.ld + tl.lr));
+    if (ic >= i1c || ir >= i1r || id >= i1d) continue;
+    int oc0, oc1, or0, or1, od0, od1;
+    tile_windows(ic, ic + 1, tl.sc, g.pc, (int)g.KC, (int)g.OC, oc0, oc1);
+    tile_windows(ir, ir + 1, tl.sr, g.pr, (int)g.KR, (int)g.OR, or0, or1);
+    tile_windows(id, id + 1, tl.sd, g.pd, (int)g.KD, (int)g.OD, od0, od1);
+    T acc[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) acc[i] = T(0);
+    for (int oc = oc0; oc <= oc1; ++oc) {
+      const int cs = max(oc * g.sc - g.pc, 0);
+      for (int orr = or0; orr <= or1; ++orr) {
+        const int rs = orr * g.sr - g.pr;
+        const int r0 = max(rs, 0), nr = min(rs + (int)g.KR, (int)g.IR) - r0;
+        for (int od = od0; od <= od1; ++od) {
+          const int at = ((((oc - wc0) * tl.NWR + (orr - wr0)) * tl.NWD + (od - wd0)) * tl.CVB +
+                          cvl) * V;
+          T gv[V];
+#pragma unroll
+          for (int i = 0; i < V; ++i) gv[i] = gbuf[at + i];
+          if (MODE == POOL_AVG) {
+#pragma unroll
+            for (int i = 0; i < V; ++i) acc[i] += gv[i];
+          } else {
+            const int ds = od * g.sd - g.pd;
+            const int d0 = max(ds, 0), nd = min(ds + (int)g.KD, (int)g.ID) - d0;
+            const int mine = ((ic - cs) * nr + (ir - r0)) * nd + (id - d0);
+#pragma unroll
+            for (int i = 0; i < V; ++i)
+              if (code[at + i] == mine) acc[i] += gv[i];
+          }
+        }
+      }
+    }
+    store_vec<T, V>(dx + xbase + (((int64_t)ic * g.IR + ir) * g.ID + id) * g.Ch +
+                        (int64_t)(cv0 + cvl) * V, acc);
+  }
+}
+
+// The same for compile-time windows K and strides S: input positions come in
+// blocks of S an axis (i + p = a*S + j), and the D + 1 windows a-D .. a, D =
+// (K-1)/S, are the ones that touch block a, element j lying in window a-d when
+// j + d*S < K.  A thread of phase 2 reads its block's windows once from shared
+// memory for all the block's elements, with no division and no per-element
+// window range: 3x3 stride 2 on [16;112;112;64] 31.5 us (max) and 16.0 us (average)
+// against 65 and 43 in the runtime-window kernel above.  Codes number the whole
+// window's taps (clipped ones too).
+template <typename T, int V, int KC, int KR, int KD, int SC, int SR, int SD, int MODE>
+__global__ void __launch_bounds__(256) pool_bwd_over_fixed_kernel(PG g, OverTile tl,
+                                                                  const T *__restrict__ x,
+                                                                  const T *__restrict__ dy,
+                                                                  T *__restrict__ dx,
+                                                                  unsigned long long ticket) {
+  extern __shared__ __align__(16) unsigned char over_smem[];
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched with launch_pdl
+  constexpr int DC = (KC - 1) / SC, DR = (KR - 1) / SR, DD = (KD - 1) / SD;
+  constexpr int N = KC * KR * KD;
+  static_assert(N < 255 && V == 4, "byte codes, four to a word");
+  T *gbuf = reinterpret_cast<T *>(over_smem);  // [NW][CVB][V]
+  uint32_t *code = reinterpret_cast<uint32_t *>(over_smem + (size_t)tl.NW * tl.CVB * V * sizeof(T));
+  unsigned q = blockIdx.x;
+  const int cb = (int)(q % tl.n_cb); q /= tl.n_cb;
+  const int td = (int)(q % tl.n_d); q /= tl.n_d;
+  const int tr = (int)(q % tl.n_r); q /= tl.n_r;
+  const int tc = (int)(q % tl.n_c);
+  const int64_t b = q / tl.n_c;
+  const int a0c = tc << tl.lc, a0r = tr << tl.lr, a0d = td << tl.ld;  // first blocks of the tile
+  const int cv0 = cb * tl.CVB, ncv = min(tl.CVB, (int)(g.Ch / V) - cv0);
+  const int64_t sd = g.Ch, sr = g.ID * g.Ch, sc = g.IR * g.ID * g.Ch;
+  const int64_t xbase = b * g.IC * sc, ybase = b * g.OC * g.OR * g.OD * g.Ch;
+  const int grp = (int)fdiv(threadIdx.x, tl.cvb), cvl = (int)threadIdx.x - grp * tl.CVB;
+  const int n_grp = (int)fdiv(blockDim.x, tl.cvb);
+  const bool on = grp < n_grp && cvl < ncv;
+  const int64_t ch = (int64_t)(cv0 + cvl) * V;
+  bool degen = false;
+  if (on) {
+    for (int w = grp; w < tl.NW; w += n_grp) {
+      const int t = (int)fdiv((uint32_t)w, tl.nwd), kd = w - t * tl.NWD;
+      const int kc = (int)fdiv((uint32_t)t, tl.nwr), kr = t - kc * tl.NWR;
+      const int oc = a0c - DC + kc, orr = a0r - DR + kr, od = a0d - DD + kd;
+      const int at = w * tl.CVB + cvl;
+      if ((unsigned)oc >= (unsigned)g.OC || (unsigned)orr >= (unsigned)g.OR ||
+          (unsigned)od >= (unsigned)g.OD) {
+        // no such window: a code that no tap has, and dY / count zero for
+        // average (skipped in phase 2 by the same test)
+        if (MODE == POOL_MAX) code[at] = 0xffffffffu;
+        continue;
+      }
+      T gv[V];
+      load_vec<T, V>(dy + ybase + (((int64_t)oc * g.OR + orr) * g.OD + od) * g.Ch + ch, gv);
+      const int c0 = oc * SC - g.pc, r0 = orr * SR - g.pr, d0 = od * SD - g.pd;
+      const bool full = c0 >= 0 && c0 + KC <= g.IC && r0 >= 0 && r0 + KR <= g.IR && d0 >= 0 &&
+                        d0 + KD <= g.ID;
+      if (MODE == POOL_MAX) {
+        T best[V];
+        int bt[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) { best[i] = T(-INFINITY); bt[i] = 255; }
+        const T *xw = x + xbase + c0 * sc + r0 * sr + d0 * sd + ch;
+        if (full) {
+          T v[N][V];
+#pragma unroll
+          for (int a = 0; a < KC; ++a)
+#pragma unroll
+            for (int bb = 0; bb < KR; ++bb)
+#pragma unroll
+              for (int c = 0; c < KD; ++c)
+                load_vec<T, V>(xw + a * sc + bb * sr + c * sd, v[(a * KR + bb) * KD + c]);
+#pragma unroll
+          for (int u = 0; u < N; ++u)
+#pragma unroll
+            for (int i = 0; i < V; ++i)
+              if (best[i] < v[u][i]) { best[i] = v[u][i]; bt[i] = u; }
+        } else {
+          for (int a = 0; a < KC; ++a)
+            for (int bb = 0; bb < KR; ++bb)
+              for (int c = 0; c < KD; ++c) {
+                if ((unsigned)(c0 + a) >= (unsigned)g.IC || (unsigned)(r0 + bb) >= (unsigned)g.IR ||
+                    (unsigned)(d0 + c) >= (unsigned)g.ID)
+                  continue;
+                T v[V];
+                load_vec<T, V>(xw + a * sc + bb * sr + c * sd, v);
+#pragma unroll
+                for (int i = 0; i < V; ++i)
+                  if (best[i] < v[i]) { best[i] = v[i]; bt[i] = (a * KR + bb) * KD + c; }
+              }
+        }
+        uint32_t word = 0;
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          degen |= bt[i] == 255;
+          word |= (uint32_t)bt[i] << (8 * i);
+        }
+        code[at] = word;
+      } else {
+        int n = N;
+        if (!full) n = window_box(g, oc, orr, od).n;
+#pragma unroll
+        for (int i = 0; i < V; ++i) gv[i] = div_count(gv[i], n);
+      }
+      store_vec<T, V>(gbuf + (size_t)at * V, gv);
+    }
+  }
+  if (MODE == POOL_MAX && degen) raise_mark(ticket);
+  __syncthreads();
+  if (!on) return;
+  const int nblk = 1 << (tl.lc + tl.lr + tl.ld);
+  for (int e = grp; e < nblk; e += n_grp) {
+    const int bd = e & ((1 << tl.ld) - 1), br = (e >> tl.ld) & ((1 << tl.lr) - 1),
+              bc = e >> (tl.ld + tl.lr);
+    const int ic0 = (a0c + bc) * SC - g.pc, ir0 = (a0r + br) * SR - g.pr,
+              id0 = (a0d + bd) * SD - g.pd;
+    if (ic0 >= g.IC || ir0 >= g.IR || id0 >= g.ID) continue;
+    T acc[SC * SR * SD][V];
+#pragma unroll
+    for (int j = 0; j < SC * SR * SD; ++j)
+#pragma unroll
+      for (int i = 0; i < V; ++i) acc[j][i] = T(0);
+#pragma unroll
+    for (int wc = 0; wc <= DC; ++wc)
+#pragma unroll
+      for (int wr = 0; wr <= DR; ++wr)
+#pragma unroll
+        for (int wd = 0; wd <= DD; ++wd) {  // window a - D + w: output order
+          const int at = (((bc + wc) * tl.NWR + (br + wr)) * tl.NWD + (bd + wd)) * tl.CVB + cvl;
+          if (MODE == POOL_AVG) {
+            const int oc = a0c + bc + wc - DC, orr = a0r + br + wr - DR, od = a0d + bd + wd - DD;
+            if ((unsigned)oc >= (unsigned)g.OC || (unsigned)orr >= (unsigned)g.OR ||
+                (unsigned)od >= (unsigned)g.OD)
+              continue;
+          }
+          const uint32_t word = MODE == POOL_MAX ? code[at] : 0u;
+          T gv[V];
+          // (a window that does not exist has codes that no element matches;
+          // its dY slot is never added)
+#pragma unroll
+          for (int i = 0; i < V; ++i) gv[i] = gbuf[(size_t)at * V + i];
+#pragma unroll
+          for (int jc = 0; jc < SC; ++jc)
+#pragma unroll
+            for (int jr = 0; jr < SR; ++jr)
+#pragma unroll
+              for (int jd = 0; jd < SD; ++jd) {
+                const int kc = jc + (DC - wc) * SC, kr = jr + (DR - wr) * SR,
+                          kd = jd + (DD - wd) * SD;
+                if (kc >= KC || kr >= KR || kd >= KD) continue;
+                const int mine = (kc * KR + kr) * KD + kd;
+                T(&o)[V] = acc[(jc * SR + jr) * SD + jd];
+#pragma unroll
+                for (int i = 0; i < V; ++i) {
+                  if (MODE == POOL_AVG) o[i] += gv[i];
+                  else if (((word >> (8 * i)) & 0xffu) == (uint32_t)mine) o[i] += gv[i];
+                }
+              }
+        }
+    T *out = dx + xbase + ic0 * sc + ir0 * sr + id0 * sd + ch;
+#pragma unroll
+    for (int jc = 0; jc < SC; ++jc)
+#pragma unroll
+      for (int jr = 0; jr < SR; ++jr)
+#pragma unroll
+        for (int jd = 0; jd < SD; ++jd)
+          if ((unsigned)(ic0 + jc) < (unsigned)g.IC && (unsigned)(ir0 + jr) < (unsigned)g.IR &&
+              (unsigned)(id0 + jd) < (unsigned)g.ID)
+            store_vec<T, V>(out + jc * sc + jr * sr + jd * sd, acc[(jc * SR + jr) * SD + jd]);
+  }
+}
+
+// The tile of an overlapping backward over V-element vectors of `es` bytes
+// each; false when the window has too many taps for a one-byte code, an
+// index does not fit 31 bits, or no tile fits shared memory (the per-element
+// kernel then runs).  Larger tiles compute fewer windows twice; the tile is
+// halved along its longest axis while fewer than two blocks an SM would run
+// or its windows take more than 48 KB.
+//
+// `fixed`: the tile is counted in blocks of the stride (the compile-time
+// kernel), and the blocks of an axis are the (I - 1 + p) / s + 1 that hold its
+// positions; otherwise in single elements.
+bool plan_over(const PG &g, int V, size_t es, bool fixed, OverTile &t, int64_t &blocks,
+               size_t &smem) {
+  const int64_t big = int64_t(1) << 30;
+  if (g.KC * g.KR * g.KD > 254 || g.IC >= big || g.IR >= big || g.ID >= big || g.pc >= big ||
+      g.pr >= big || g.pd >= big || g.KC >= big || g.KR >= big || g.KD >= big)
+    return false;
+  const int64_t CV = g.Ch / V;
+  t.CVB = (int)std::min<int64_t>(CV, 16);
+  t.n_cb = (int)ceil_div(CV, t.CVB);
+  auto l2 = [](int64_t n, int most) {
+    int l = 0;
+    while (l < most && (int64_t(1) << l) < n) ++l;
+    return l;
+  };
+  const int64_t EC = fixed ? (g.IC - 1 + g.pc) / g.sc + 1 : g.IC,
+                ER = fixed ? (g.IR - 1 + g.pr) / g.sr + 1 : g.IR,
+                ED = fixed ? (g.ID - 1 + g.pd) / g.sd + 1 : g.ID;
+  const int most = fixed && std::max(g.sc, g.sr) > 1 ? 3 : 4;
+  if (ED == 1) {
+    t.ld = 0; t.lr = l2(ER, most); t.lc = l2(EC, most);
+  } else {
+    t.ld = l2(ED, most - 1); t.lr = l2(ER, most - 1); t.lc = l2(EC, most - 1);
+  }
+  auto wins = [fixed](int tile, int64_t k, int s, int64_t O) {
+    return fixed ? tile + (k - 1) / s : std::min<int64_t>(O, (tile + k - 2) / s + 1);
+  };
+  while (true) {
+    t.n_c = (int)ceil_div(EC, int64_t(1) << t.lc);
+    t.n_r = (int)ceil_div(ER, int64_t(1) << t.lr);
+    t.n_d = (int)ceil_div(ED, int64_t(1) << t.ld);
+    const int64_t nwc = wins(1 << t.lc, g.KC, g.sc, g.OC), nwr = wins(1 << t.lr, g.KR, g.sr, g.OR),
+                  nwd = wins(1 << t.ld, g.KD, g.sd, g.OD);
+    blocks = g.B * t.n_c * t.n_r * t.n_d * t.n_cb;
+    const int64_t need = nwc * nwr * nwd * t.CVB * V * (int64_t)(es + 1);
+    const bool fits = need <= 48 * 1024;
+    const int longest = std::max(t.lc, std::max(t.lr, t.ld));
+    if (fits && (blocks >= 2 * 152 || t.lc + t.lr + t.ld <= 4 || longest == 0)) {
+      if (blocks >= (int64_t(1) << 31)) return false;
+      t.NWR = (int)nwr; t.NWD = (int)nwd; t.NW = (int)(nwc * nwr * nwd);
+      smem = (size_t)need;
+      break;
+    }
+    if (longest == 0) return false;
+    if (t.lc == longest) --t.lc;
+    else if (t.lr == longest) --t.lr;
+    else --t.ld;
+  }
+  t.nwr = make_fastdiv((uint32_t)t.NWR);
+  t.nwd = make_fastdiv((uint32_t)t.NWD);
+  t.cvb = make_fastdiv((uint32_t)t.CVB);
+  t.sc = make_fastdiv((uint32_t)g.sc);
+  t.sr = make_fastdiv((uint32_t)g.sr);
+  t.sd = make_fastdiv((uint32_t)g.sd);
+  return true;
 }
 
 // Ordered rebuild of dX[0] for max-pool backward when some window selected
@@ -618,16 +1026,6 @@ int vec_width(int64_t ch, const void *a, const void *b, const void *c) {
   return 1;
 }
 
-// Every window lies wholly inside the input: no padding and the last
-// window ends at or before the input's end, in every dimension.
-bool interior(const PG &g) {
-  auto ok = [](int64_t I, int64_t K, int64_t O, int s, int p) {
-    return p == 0 && (O - 1) * s + K <= I;
-  };
-  return ok(g.IC, g.KC, g.OC, g.sc, g.pc) && ok(g.IR, g.KR, g.OR, g.sr, g.pr) &&
-         ok(g.ID, g.KD, g.OD, g.sd, g.pd);
-}
-
 // Windows tile the input exactly: stride = kernel, no padding, O*s = I.
 bool exact_tiling(const PG &g) {
   auto ok = [](int64_t I, int64_t K, int64_t O, int s, int p) {
@@ -645,14 +1043,16 @@ template <typename T, int V, int KC, int KR, int KD>
 void fwd_fixed(const PG &g, PoolMode mode, const T *x, T *y, int64_t *arg, int grid,
                cudaStream_t s) {
   const OutDecode d = make_out_decode(g, g.Ch / V);
+  int64_t *none = nullptr;
   if (mode == POOL_AVG)
-    pool_fwd_fixed_kernel<T, V, KC, KR, KD, POOL_AVG, false>
-        <<<grid, 256, 0, s>>>(g, d, x, y, nullptr);
+    launch_pdl(pool_fwd_fixed_kernel<T, V, KC, KR, KD, POOL_AVG, false>, dim3(grid), dim3(256),
+               0, s, g, d, x, y, none);
   else if (arg)
-    pool_fwd_fixed_kernel<T, V, KC, KR, KD, POOL_MAX, true><<<grid, 256, 0, s>>>(g, d, x, y, arg);
+    launch_pdl(pool_fwd_fixed_kernel<T, V, KC, KR, KD, POOL_MAX, true>, dim3(grid), dim3(256), 0,
+               s, g, d, x, y, arg);
   else
-    pool_fwd_fixed_kernel<T, V, KC, KR, KD, POOL_MAX, false>
-        <<<grid, 256, 0, s>>>(g, d, x, y, nullptr);
+    launch_pdl(pool_fwd_fixed_kernel<T, V, KC, KR, KD, POOL_MAX, false>, dim3(grid), dim3(256),
+               0, s, g, d, x, y, none);
 }
 
 // The fixed-window kernels index outputs with 32-bit fast division.
@@ -661,24 +1061,27 @@ bool small_output(const PG &g, int V) {
 }
 
 // Fixed-window kernels exist for the widest vector of each type (16 bytes)
-// and the common window shapes 2x2, 3x3 and 2x2x2.
+// and the common window shapes 2x2, 3x3, 2x2x2 and 3x3x3.
 
 template <typename T, int V>
 int fwd_launch(const PG &g, PoolMode mode, const T *x, T *y, int64_t *arg, cudaStream_t s) {
   int grid = grid_for(g.B * g.OC * g.OR * g.OD * (g.Ch / V));
-  const bool fixed = V == kWide<T> && interior(g) && small_output(g, V);
+  const bool fixed = V == kWide<T> && small_output(g, V);
+  int64_t *none = nullptr;
   if (fixed && window_is(g, 2, 2, 1)) {
     fwd_fixed<T, V, 2, 2, 1>(g, mode, x, y, arg, grid, s);
   } else if (fixed && window_is(g, 3, 3, 1)) {
     fwd_fixed<T, V, 3, 3, 1>(g, mode, x, y, arg, grid, s);
   } else if (fixed && window_is(g, 2, 2, 2)) {
     fwd_fixed<T, V, 2, 2, 2>(g, mode, x, y, arg, grid, s);
+  } else if (fixed && window_is(g, 3, 3, 3)) {
+    fwd_fixed<T, V, 3, 3, 3>(g, mode, x, y, arg, grid, s);
   } else if (mode == POOL_AVG) {
-    pool_fwd_kernel<T, V, POOL_AVG, false><<<grid, 256, 0, s>>>(g, x, y, nullptr);
+    launch_pdl(pool_fwd_kernel<T, V, POOL_AVG, false>, dim3(grid), dim3(256), 0, s, g, x, y, none);
   } else if (arg) {
-    pool_fwd_kernel<T, V, POOL_MAX, true><<<grid, 256, 0, s>>>(g, x, y, arg);
+    launch_pdl(pool_fwd_kernel<T, V, POOL_MAX, true>, dim3(grid), dim3(256), 0, s, g, x, y, arg);
   } else {
-    pool_fwd_kernel<T, V, POOL_MAX, false><<<grid, 256, 0, s>>>(g, x, y, nullptr);
+    launch_pdl(pool_fwd_kernel<T, V, POOL_MAX, false>, dim3(grid), dim3(256), 0, s, g, x, y, none);
   }
   OWL_CHECK_LAUNCH("pool_fwd_kernel");
   return kOk;
@@ -704,11 +1107,43 @@ void bwd_tile(const PG &g, PoolMode mode, const T *x, const T *dy, T *dx,
               unsigned long long ticket, int grid, cudaStream_t s) {
   const OutDecode d = make_out_decode(g, g.Ch / V);
   if (mode == POOL_AVG)
-    pool_bwd_tile_kernel<T, V, KC, KR, KD, POOL_AVG>
-        <<<grid, 256, 0, s>>>(g, d, x, dy, dx, ticket);
+    launch_pdl(pool_bwd_tile_kernel<T, V, KC, KR, KD, POOL_AVG>, dim3(grid), dim3(256), 0, s, g,
+               d, x, dy, dx, ticket);
   else
-    pool_bwd_tile_kernel<T, V, KC, KR, KD, POOL_MAX>
-        <<<grid, 256, 0, s>>>(g, d, x, dy, dx, ticket);
+    launch_pdl(pool_bwd_tile_kernel<T, V, KC, KR, KD, POOL_MAX>, dim3(grid), dim3(256), 0, s, g,
+               d, x, dy, dx, ticket);
+}
+
+template <typename T, int V, int KC, int KR, int KD, int SC, int SR, int SD>
+bool bwd_over_fixed(const PG &g, PoolMode mode, const T *x, const T *dy, T *dx,
+                    unsigned long long ticket, cudaStream_t s) {
+  OverTile tl;
+  int64_t blocks = 0;
+  size_t smem = 0;
+  if (!window_is(g, KC, KR, KD) || g.sc != SC || g.sr != SR || g.sd != SD ||
+      !plan_over(g, V, sizeof(T), true, tl, blocks, smem))
+    return false;
+  if (mode == POOL_AVG)
+    launch_pdl(pool_bwd_over_fixed_kernel<T, V, KC, KR, KD, SC, SR, SD, POOL_AVG>,
+               dim3((unsigned)blocks), dim3(256), smem, s, g, tl, x, dy, dx, ticket);
+  else
+    launch_pdl(pool_bwd_over_fixed_kernel<T, V, KC, KR, KD, SC, SR, SD, POOL_MAX>,
+               dim3((unsigned)blocks), dim3(256), smem, s, g, tl, x, dy, dx, ticket);
+  return true;
+}
+
+// The overlapping windows that networks use, in float32 with 16-byte channel
+// vectors: 3x3 stride 2 and 1, 2x2 stride 1, 3x3x3 stride 2.
+template <typename T, int V>
+bool bwd_over_common(const PG &g, PoolMode mode, const T *x, const T *dy, T *dx,
+                     unsigned long long ticket, cudaStream_t s) {
+  if constexpr (std::is_same_v<T, float> && V == 4) {
+    return bwd_over_fixed<T, V, 3, 3, 1, 2, 2, 1>(g, mode, x, dy, dx, ticket, s) ||
+           bwd_over_fixed<T, V, 3, 3, 1, 1, 1, 1>(g, mode, x, dy, dx, ticket, s) ||
+           bwd_over_fixed<T, V, 2, 2, 1, 1, 1, 1>(g, mode, x, dy, dx, ticket, s) ||
+           bwd_over_fixed<T, V, 3, 3, 3, 2, 2, 2>(g, mode, x, dy, dx, ticket, s);
+  }
+  return false;
 }
 
 template <typename T, int V>
@@ -722,16 +1157,32 @@ int bwd_launch(const PG &g, PoolMode mode, const T *x, const T *dy, T *dx,
     else if (tile && window_is(g, 2, 2, 2))
       bwd_tile<T, V, 2, 2, 2>(g, mode, x, dy, dx, ticket, grid, s);
     else if (mode == POOL_AVG)
-      pool_bwd_cell_kernel<T, V, POOL_AVG><<<grid, 256, 0, s>>>(g, x, dy, dx, ticket);
+      launch_pdl(pool_bwd_cell_kernel<T, V, POOL_AVG>, dim3(grid), dim3(256), 0, s, g, x, dy, dx,
+                 ticket);
     else
-      pool_bwd_cell_kernel<T, V, POOL_MAX><<<grid, 256, 0, s>>>(g, x, dy, dx, ticket);
+      launch_pdl(pool_bwd_cell_kernel<T, V, POOL_MAX>, dim3(grid), dim3(256), 0, s, g, x, dy, dx,
+                 ticket);
     OWL_CHECK_LAUNCH("pool_bwd_cell_kernel");
   } else {
+    OverTile tl;
+    int64_t blocks = 0;
+    size_t smem = 0;
     int grid = grid_for(g.B * g.IC * g.IR * g.ID * (g.Ch / V));
-    if (mode == POOL_AVG)
-      pool_bwd_gather_kernel<T, V, POOL_AVG><<<grid, 256, 0, s>>>(g, x, dy, dx, ticket);
+    if (bwd_over_common<T, V>(g, mode, x, dy, dx, ticket, s)) {
+      // launched
+    } else if (plan_over(g, V, sizeof(T), false, tl, blocks, smem)) {
+      if (mode == POOL_AVG)
+        launch_pdl(pool_bwd_over_kernel<T, V, POOL_AVG>, dim3((unsigned)blocks), dim3(256), smem,
+                   s, g, tl, x, dy, dx, ticket);
+      else
+        launch_pdl(pool_bwd_over_kernel<T, V, POOL_MAX>, dim3((unsigned)blocks), dim3(256), smem,
+                   s, g, tl, x, dy, dx, ticket);
+    } else if (mode == POOL_AVG)
+      launch_pdl(pool_bwd_gather_kernel<T, V, POOL_AVG>, dim3(grid), dim3(256), 0, s, g, x, dy,
+                 dx, ticket);
     else
-      pool_bwd_gather_kernel<T, V, POOL_MAX><<<grid, 256, 0, s>>>(g, x, dy, dx, ticket);
+      launch_pdl(pool_bwd_gather_kernel<T, V, POOL_MAX>, dim3(grid), dim3(256), 0, s, g, x, dy,
+                 dx, ticket);
     OWL_CHECK_LAUNCH("pool_bwd_gather_kernel");
   }
   return kOk;
