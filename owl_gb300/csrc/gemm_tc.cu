@@ -23,6 +23,7 @@
 
 #include "../../include/owlgpu.h"
 #include "common.cuh"
+#include "reduce.cuh"
 #include "tc_ptx.cuh"
 #include "tc_stage.cuh"
 
@@ -465,22 +466,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
   }
 }
 
-// out[m][n] = act(sum over splits z = 0, 1, ... of part[z][m][n] + bias[n]),
-// in split order.
-__global__ void gemm_reduce(const float *__restrict__ part, float *__restrict__ out,
-                            const float *__restrict__ bias, int act, long long M, long long N,
-                            int splits) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched with launch_pdl
-  const long long n_all = M * N;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_all;
-       i += (long long)gridDim.x * blockDim.x) {
-    float s = part[i];
-    for (int z = 1; z < splits; ++z) s += part[(long long)z * n_all + i];
-    if (bias) s += bias[i % N];
-    out[i] = apply_act(s, act);
-  }
-}
-
 int *gemm_status_word() {
   static int *p[64] = {nullptr};
   int dev = 0;
@@ -573,15 +558,8 @@ int gemm_run(int prec, GemmParams p, float *c, cudaStream_t s) {
   const dim3 grid((unsigned)mt, (unsigned)nt, (unsigned)p.splits);
   int rc = kind == stage::K_BF16X3 ? launch<stage::K_BF16X3>(p, smem, grid, s)
                                    : launch<stage::K_BF16>(p, smem, grid, s);
-  if (rc == kOk && p.splits > 1) {
-    const long long n_all = M * N;
-    const int blocks = (int)std::max<long long>(1, std::min<long long>((n_all + 255) / 256, 4 * 152));
-    cudaError_t e = launch_pdl(gemm_reduce, dim3(blocks), dim3(256), 0, s, (const float *)part,
-                               c, bias, act, M, N, p.splits);
-    if (e == cudaSuccess) e = cudaGetLastError();
-    note_launch();
-    if (e != cudaSuccess) rc = cuda_fail(e, "gemm_reduce");
-  }
+  if (rc == kOk && p.splits > 1)
+    rc = sum_splits<float>(part, c, M * N, p.splits, bias, N, act, s);
   if (part) scratch_free(part, s);
   return rc;
 }
