@@ -90,9 +90,7 @@ int conv_fwd(Dtype dt, int prec, const ConvGeom &g, const void *x, const void *w
     }
   }
   t_last_path = 0;
-  int rc = simt_conv_fwd(dt, g, x, w, y, s);
-  if (rc || (!bias && act == OWLGPU_ACT_NONE)) return rc;
-  return bias_act_inplace(dt, y, bias, g.y_elems(), g.Co, act, s);
+  return simt_conv_fwd(dt, g, x, w, y, s, bias, act);
 }
 
 int conv_bwd_input(Dtype dt, int prec, const ConvGeom &g, void *dx, const void *w,

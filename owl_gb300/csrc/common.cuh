@@ -180,8 +180,7 @@ void scratch_free(void *p, cudaStream_t s);
 
 // ---- compute entry points (device pointers, asynchronous) --------------
 // Forward convolution; with `bias` (per output channel, or null) and `act`
-// (OWLGPU_ACT_*), y = act(conv + bias): in the tensor-core epilogue, or by a
-// second pass after the CUDA-core kernel.
+// (OWLGPU_ACT_*), y = act(conv + bias), in the kernel's epilogue.
 int conv_fwd(Dtype dt, int prec, const ConvGeom &g, const void *x, const void *w, void *y,
              cudaStream_t s, const void *bias = nullptr, int act = 0);
 // y[i] = act(y[i] + bias[i % C]) over n elements (real kinds).
@@ -203,8 +202,9 @@ int upsample_fwd(Dtype dt, const UpGeom &g, const void *x, void *y, cudaStream_t
 int upsample_bwd(Dtype dt, const UpGeom &g, void *dx, const void *dy, cudaStream_t s);
 
 // SIMT (CUDA-core) implementations: the plain FP32 path and the FP64 path.
+// (forward: y = act(conv + bias[co]), as conv_fwd)
 int simt_conv_fwd(Dtype dt, const ConvGeom &g, const void *x, const void *w, void *y,
-                  cudaStream_t s);
+                  cudaStream_t s, const void *bias = nullptr, int act = 0);
 int simt_conv_bwd_input(Dtype dt, const ConvGeom &g, void *dx, const void *w, const void *dy,
                         cudaStream_t s);
 int simt_conv_bwd_kernel(Dtype dt, const ConvGeom &g, const void *x, void *dw, const void *dy,
@@ -213,8 +213,9 @@ int simt_conv_bwd_kernel(Dtype dt, const ConvGeom &g, const void *x, void *dw, c
 // A pass of a 1x1 geometry on the CUDA cores as a split-K GEMM (partials
 // summed in order): mode 0 forward (a = x, b = w, c = y), 1 backward_input
 // (a = dy, b = w, c = dx), 2 backward_kernel (a = x, b = dy, c = dw).
+// `bias` (per column of c, or null) and `act` are applied to the sums.
 int simt_gemm(Dtype dt, int mode, const ConvGeom &g, const void *a, const void *b, void *c,
-              cudaStream_t s);
+              cudaStream_t s, const void *bias = nullptr, int act = 0);
 
 // backward_kernel (float32, SIMT) with split-K partials in a caller-provided
 // workspace of ws_elems floats; splits are capped to fit it.

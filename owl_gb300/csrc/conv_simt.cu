@@ -14,7 +14,9 @@
 //   bwd kernel   dW[tap*Ci+ci][co] = sum_m X[gather(m, tap)][ci] * dY[m][co]
 //                reduction over output pixels, split across CTAs and summed
 //                by a second kernel in a fixed order (deterministic).
+#include "../../include/owlgpu.h"
 #include "common.cuh"
+#include "reduce.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -40,7 +42,20 @@ struct Dev {
   // receives exactly one tap)
   int64_t s2d_ci, s2d_tc, s2d_tr;
   int s2d_kr, s2d_kd;
+  // FWD: y = act(conv + bias[n]) (bias of the element type, or null; act
+  // OWLGPU_ACT_*), applied to the finished sum as a second pass would
+  const void *bias;
+  int act;
 };
+
+template <typename T>
+__device__ __forceinline__ T with_bias_act(T v, const Dev &g, int64_t n) {
+  if (g.bias) v += static_cast<const T *>(g.bias)[n];
+  if constexpr (std::is_floating_point_v<T>) {
+    if (g.act == OWLGPU_ACT_RELU) v = v > T(0) ? v : T(0);
+  }
+  return v;
+}
 
 template <typename T, int MODE, int BM, int BN, int BK, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
@@ -52,12 +67,20 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
   constexpr int B_PER = BN * BK / NT;
   static_assert(BM * BK % NT == 0 && BN * BK % NT == 0, "tile/thread mismatch");
 
+  static_assert(MODE != FWD || 256 % BK == 0, "the tap table holds whole slabs");
   __shared__ T As[2][BK][BM + 4];
   __shared__ T Bs[2][BK][BN + 4];
   // Per-row (FWD/BWDI) or per-k (BWDK) pixel decode cache.
   constexpr int PIX = (MODE == BWDK) ? BK : BM;
   __shared__ int64_t s_base[2][PIX];
   __shared__ int s_c[2][PIX], s_r[2][PIX], s_d[2][PIX];
+  // FWD: where k's tap and channel lie relative to a window's origin (element
+  // offset, and the tap's position for the bounds), for KT consecutive k: one
+  // 64-bit division per k and CTA instead of several per k slab and thread.
+  constexpr int KT = MODE == FWD ? (sizeof(T) < 16 ? 512 : 256) : 1;
+  __shared__ int64_t s_koff[KT];
+  __shared__ int s_kc[KT], s_kr[KT], s_kd[KT];
+  int64_t kt_begin = -KT;  // k of the table's first entry
 
   const int tid = threadIdx.x;
   const int64_t m0 = (int64_t)blockIdx.x * BM;
@@ -124,6 +147,14 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
       s_c[1][i] = s_c[0][i]; s_r[1][i] = s_r[0][i]; s_d[1][i] = s_d[0][i];
     }
     __syncthreads();  // rows decoded by one thread are gathered by others
+    if (MODE == FWD) {
+      // a window's origin as an element offset
+      for (int i = tid; i < BM; i += NT)
+        if (s_base[0][i] >= 0)
+          s_base[1][i] =
+              (s_base[0][i] + ((int64_t)s_c[0][i] * g.IR + s_r[0][i]) * g.ID + s_d[0][i]) * g.Ci;
+      __syncthreads();
+    }
   }
 
   T a_reg[A_PER], b_reg[B_PER];
@@ -132,26 +163,41 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
   auto load_tiles = [&](int64_t k0, int buf) {
     if (MODE == FWD) {
       // A[m][k]: thread owns a fixed k column, several rows.
+      if (k0 >= kt_begin + KT) {  // (the same for every thread; KT is whole slabs)
+        kt_begin = k0;
+        __syncthreads();
+        for (int i = tid; i < KT; i += NT) {
+          const int64_t k = k0 + i;
+          if (k >= k_end) break;
+          int64_t tap = k / g.Ci;
+          const int64_t ci = k - tap * g.Ci;
+          const int64_t kd = tap % g.KD;
+          tap /= g.KD;
+          const int64_t kr = tap % g.KR, kc = tap / g.KR;
+          s_kc[i] = (int)(kc * g.dc);
+          s_kr[i] = (int)(kr * g.dr);
+          s_kd[i] = (int)(kd * g.dd);
+          s_koff[i] = ((kc * g.dc * g.IR + kr * g.dr) * g.ID + kd * g.dd) * g.Ci + ci;
+        }
+        __syncthreads();
+      }
       const int kk = tid % BK;
-      const int64_t k = k0 + kk;
-      int kc = 0, kr = 0, kd = 0, ci = 0;
-      bool kval = k < k_end;
+      const int ki = (int)(k0 - kt_begin) + kk;
+      const bool kval = k0 + kk < k_end;
+      int64_t koff = 0;
+      int tc = 0, tr = 0, td = 0;
       if (kval) {
-        int64_t tap = k / g.Ci;
-        ci = (int)(k - tap * g.Ci);
-        kd = (int)(tap % g.KD); tap /= g.KD;
-        kr = (int)(tap % g.KR); kc = (int)(tap / g.KR);
+        koff = s_koff[ki];
+        tc = s_kc[ki]; tr = s_kr[ki]; td = s_kd[ki];
       }
 #pragma unroll
       for (int i = 0; i < A_PER; ++i) {
         int mm = tid / BK + i * (NT / BK);
         T v = T(0);
-        int64_t base = s_base[buf][mm];
-        if (kval && base >= 0) {
-          int c = s_c[buf][mm] + kc * g.dc, r = s_r[buf][mm] + kr * g.dr,
-              d = s_d[buf][mm] + kd * g.dd;
+        if (kval && s_base[0][mm] >= 0) {
+          const int c = s_c[0][mm] + tc, r = s_r[0][mm] + tr, d = s_d[0][mm] + td;
           if (c >= 0 && c < g.IC && r >= 0 && r < g.IR && d >= 0 && d < g.ID)
-            v = A0[((base + ((int64_t)c * g.IR + r) * g.ID + d) * g.Ci) + ci];
+            v = A0[s_base[1][mm] + koff];
         }
         a_reg[i] = v;
       }
@@ -324,105 +370,116 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
       int64_t n = n0 + tx * TN + j;
-      if (n < g.N) Cz[row * g.N + n] = acc[i][j];
+      if (n < g.N) Cz[row * g.N + n] = MODE == FWD ? with_bias_act(acc[i][j], g, n) : acc[i][j];
     }
   }
 }
 
-// Fixed-order sum of split-K partials: out[i] = ((p0 + p1) + p2) + ...
-template <typename T>
-__global__ void splitk_reduce_kernel(const T *__restrict__ part, T *__restrict__ out,
-                                     int64_t n, int splits) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched with launch_pdl
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (; i < n; i += stride) {
-    T s = part[i];
-    for (int z = 1; z < splits; ++z) s += part[(int64_t)z * n + i];
-    out[i] = s;
-  }
-}
-
 // ---- float32 vector path ----------------------------------------------------
-// The same GEMM views in float32 with 16-byte operand gathers: 128 x 128
-// tiles (128 x 64 when N <= 64, 256 x 32 when N <= 32), 16-deep k slabs,
-// 256 threads of 8 x 8 outputs (four 4 x 4 quadrants, rows ty*4 and
-// 64 + ty*4, columns tx*4 and 64 + tx*4, so every shared-memory fragment is
-// one 16-byte load without bank conflicts; 8 x 4 in the narrower tiles).
+// The same GEMM views in float32 with 16-byte operand gathers and packed
+// multiply-adds: BM x BN tiles, 16-deep k slabs, a thread TM x TN outputs in
+// 4 x 4 quadrants (rows ty*4 + q*BM*4/TM, columns tx*4 + q*BN*4/TN, so every
+// shared-memory fragment is one 16-byte load without bank conflicts).
 //   FWD : a slab is 16 consecutive input channels of one tap (Ci % 16 == 0);
-//         four threads read one pixel's 64 bytes, and each thread's two
-//         output pixels are decoded once per CTA.  A is stored k-major with
+//         four threads read one pixel's 64 bytes, and each thread's output
+//         pixels and the taps inside X are decoded once per CTA.  A is stored k-major with
 //         its row index XOR-swizzled by the channel quad (k / 4) * 8, so the
-//         four threads of a pixel write four different bank groups.
+//         four threads of a pixel write four different bank groups.  BT: the
+//         kernel operand is [n][k] (a dense layer's x w^T), staged like A.
 //   BWDK: a slab is 16 consecutive output pixels; a thread reads four
 //         consecutive (tap, ci) rows of one pixel (Ci % 4 == 0), a warp one
-//         pixel's 128 rows; the slab's pixels are decoded by 16 threads into
+//         pixel's rows; the slab's pixels are decoded by 16 threads into
 //         shared memory one slab ahead.
 // The k order of every output's sum is the same as the scalar kernel's
-// (ascending, one fused multiply-add per k), so a float32 forward gives the
-// same bits on either path.
-constexpr int kVBK = 16, kVNT = 256;
+// (ascending, one fused multiply-add per k), whatever the tile, so a float32
+// result has the same bits on either path.
+//
+// Bound: the FMA pipe and the latency that two or three warps a scheduler leave
+// open.  A loop of nothing but fmaf reaches 60 TFLOP/s on this chip, one of
+// fma.rn.f32x2 (two multiply-adds an instruction, each rounded as fmaf) 68, so
+// the accumulators are pairs of neighbouring rows: A's fragments are read as
+// pairs, B's values duplicated into both halves.  Blocks of 128 threads (three an
+// SM) instead of 256 (one) let one block's barrier and loads overlap another's
+// arithmetic: [32;56;56;128] x [3;3;128;128] 43 -> 48 TFLOP/s.
+constexpr int kVBK = 16;
 
 __device__ __forceinline__ float4 ldg4(const float *p) {
   return __ldg(reinterpret_cast<const float4 *>(p));
 }
 
-// Tile shapes, by the GEMM's N:
-//   CN = 2: 128 x 128, a thread 8 x 8 (rows ty*4 + {0, 64}, columns tx*4 + {0, 64})
-//   CN = 1: 128 x 64,  a thread 8 x 4 (columns tx*4)
-//   CN = 0: 256 x 32,  a thread 8 x 4 (rows ty*4 + {0, 128}, columns tx*4)
-template <int CN>
-struct F32vShape {
-  static constexpr int BM = CN == 0 ? 256 : 128;
-  static constexpr int BN = CN == 0 ? 32 : 64 * CN;
-  static constexpr int RQ = BM / 64;    // FWD: A rows per thread (a 4-channel quad each)
-  static constexpr int NJ = CN == 0 ? 1 : CN;  // column quads per thread
-  static constexpr int RSTEP = BM / 2;  // a thread's second row quad
-  static constexpr int BH = CN == 2 ? 2 : 1;  // B float4 loads per thread
-};
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ void ffma2(uint64_t &d, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
 
-template <int MODE, int CN>
-__global__ void __launch_bounds__(kVNT, 1)
+template <int MODE, int BM, int BN, int TM, int TN, bool BT>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
     conv_f32v_kernel(Dev g, const float *__restrict__ A0, const float *__restrict__ B0,
                      float *__restrict__ C, int64_t k_per_split) {
   asm volatile("griddepcontrol.wait;" ::: "memory");  // launched with launch_pdl
-  using S = F32vShape<CN>;
-  constexpr int BM = S::BM, BN = S::BN, RQ = S::RQ, NJ = S::NJ;
+  static_assert(MODE == FWD || !BT, "transposed B: FWD only");
+  constexpr int NT = (BM / TM) * (BN / TN);
+  constexpr int NI = TM / 4, NJ = TN / 4;            // row and column quads per thread
+  constexpr int RSTEP = BM / NI, CSTEP = BN / NJ;    // between them
   __shared__ __align__(16) float As[2][kVBK][BM];
   __shared__ __align__(16) float Bs[2][kVBK][BN];
-  __shared__ int64_t s_base[2][kVBK];  // BWDK: slab pixels (batch image offset, -1 past the end)
-  __shared__ int s_c[2][kVBK], s_r[2][kVBK], s_d[2][kVBK];
+  // BWDK: the slab's pixels: window origin (c, r, d; w = 0 past the end) and
+  // the origin's pixel index in X
+  __shared__ int4 s_pix[2][kVBK];
+  __shared__ int64_t s_lin[2][kVBK];
 
   const int tid = threadIdx.x;
-  // A warp's 16-byte fragment loads touch one contiguous run of A and one of
-  // B per k (one shared-memory wavefront each): 8 row groups x 4 column
-  // groups in the 128-row tiles, 4 x 8 in the 256-row one.
+  // A warp covers 8 row threads x 4 column threads: its 16-byte fragment
+  // loads touch one contiguous run of A and one of B per k (one shared-memory
+  // wavefront each).
+  constexpr int CW = BN / TN / 4;  // warps along the columns
   const int lane = tid & 31, warp = tid >> 5;
-  const int ty = CN == 0 ? warp * 4 + (lane >> 3) : (warp >> 2) * 8 + (lane >> 2);
-  const int tx = CN == 0 ? (lane & 7) : (warp & 3) * 4 + (lane & 3);
+  const int ty = (warp / CW) * 8 + (lane >> 2), tx = (warp % CW) * 4 + (lane & 3);
   const int64_t m0 = (int64_t)blockIdx.x * BM, n0 = (int64_t)blockIdx.y * BN;
   const int64_t k_begin = (int64_t)blockIdx.z * k_per_split;
   const int64_t k_end = min(g.K, k_begin + k_per_split);
   const int64_t img = g.IC * g.IR * g.ID;  // pixels per batch image of X
 
   // ---- FWD: this thread's RQ output pixels and its channel quad -----------
+  constexpr int RQ = BM * 4 / NT;
   const int aq = tid & 3;  // FWD: channel quad within the slab
+  // MASKS: a pixel's window origin in X (at this thread's channel quad) and a
+  // bit for each of 32 taps, set when the tap lies inside X, rebuilt every 32
+  // taps: a slab costs a pixel one bit test and one add.  Otherwise its image
+  // and origin coordinates, tested per slab.  The masks pay in the 128 x 32 tile
+  // ([16;57;43;96] x [3;3;96;160] 282 -> 254 us); in the 8 x 8-output tile their
+  // registers cost more than they save (617 -> 637 us on [32;56;56;128] x
+  // [3;3;128;128]), and in the small tile, for short reductions, their set-up.
+  constexpr bool MASKS = MODE == FWD && TM == 8 && TN == 4;
+  const float *arow[RQ];
+  uint32_t amask[RQ];
   int64_t abase[RQ];
   int ac[RQ], ar[RQ], ad[RQ];
-  // ---- BWDK: this thread's four (tap, ci) rows, its pixels ak + k*(256/(BM/4))
-  constexpr int MQ = BM / 4;       // row quads per k row
-  constexpr int AKS = kVNT / MQ;   // k rows per pass
+  // ---- BWDK: this thread's four (tap, ci) rows, its pixels ak + AKS*h
+  constexpr int MQ = BM / 4;   // row quads per k row
+  constexpr int AKS = NT / MQ > kVBK ? kVBK : NT / MQ;  // k rows per pass
   const int mq = (tid % MQ) * 4;
   const int ak = tid / MQ;
   bool mval = false;
   int t_dc = 0, t_dr = 0, t_dd = 0;
-  int64_t mci = 0;
-  if (MODE == FWD) {
+  const float *a_tap = A0;  // BWDK: the rows' channel at their tap from a window's origin
+  // FWD: decode this thread's pixels (MASKS: with the masks of the 32 taps from
+  // t0 on)
+  auto row_masks = [&](int t0, bool first) {
 #pragma unroll
     for (int h = 0; h < RQ; ++h) {
-      const int64_t m = m0 + (tid >> 2) + 64 * h;
+      const int64_t m = m0 + (tid >> 2) + NT / 4 * h;
+      amask[h] = 0;
       abase[h] = -1;
       ac[h] = ar[h] = ad[h] = 0;
+      if (first) arow[h] = A0;
       if (m < g.M) {
         int64_t t = m;
         const int64_t od = t % g.OD;
@@ -430,27 +487,61 @@ __global__ void __launch_bounds__(kVNT, 1)
         const int64_t orr = t % g.OR;
         t /= g.OR;
         const int64_t oc = t % g.OC, b = t / g.OC;
-        abase[h] = b * img;
-        ac[h] = (int)(oc * g.sc) - g.pc;
-        ar[h] = (int)(orr * g.sr) - g.pr;
-        ad[h] = (int)(od * g.sd) - g.pd;
+        const int c = (int)(oc * g.sc) - g.pc, r = (int)(orr * g.sr) - g.pr,
+                  d = (int)(od * g.sd) - g.pd;
+        if (!MASKS) {
+          abase[h] = b * img;
+          ac[h] = c; ar[h] = r; ad[h] = d;
+          continue;
+        }
+        if (first)
+          arow[h] = A0 + (b * img + ((int64_t)c * g.IR + r) * g.ID + d) * g.Ci + aq * 4;
+        const int krd = (int)(g.KR * g.KD);
+        int kc = t0 / krd, rem = t0 - kc * krd;
+        int kr = rem / (int)g.KD, kd = rem - kr * (int)g.KD;
+        const int n = (int)min((int64_t)32, g.KC * g.KR * g.KD - t0);
+        uint32_t mask = 0;
+        for (int q = 0; q < n; ++q) {
+          mask |= (uint32_t)((unsigned)(c + kc * g.dc) < (unsigned)g.IC &&
+                             (unsigned)(r + kr * g.dr) < (unsigned)g.IR &&
+                             (unsigned)(d + kd * g.dd) < (unsigned)g.ID)
+                  << q;
+          if (++kd == g.KD) {
+            kd = 0;
+            if (++kr == g.KR) {
+              kr = 0;
+              ++kc;
+            }
+          }
+        }
+        amask[h] = mask;
       }
     }
+  };
+  if (MODE == FWD) {
+    row_masks(0, true);
   } else {
     const int64_t m = m0 + mq;
     if (m < g.M) {
       mval = true;
       int64_t tap = m / g.Ci;
-      mci = m - tap * g.Ci;
+      const int64_t mci = m - tap * g.Ci;
       const int kd = (int)(tap % g.KD);
       tap /= g.KD;
       const int kr = (int)(tap % g.KR), kc = (int)(tap / g.KR);
       t_dc = kc * g.dc;
       t_dr = kr * g.dr;
       t_dd = kd * g.dd;
+      a_tap = A0 + (((int64_t)t_dc * g.IR + t_dr) * g.ID + t_dd) * g.Ci + mci;
     }
   }
   // BWDK: decode pixel p into slot `slot` of buffer `buf` (-1 past k_end)
+  auto put_pixel = [&](int64_t b, int64_t oc, int64_t orr, int64_t od, int slot, int buf) {
+    const int c = (int)(oc * g.sc) - g.pc, r = (int)(orr * g.sr) - g.pr,
+              d = (int)(od * g.sd) - g.pd;
+    s_pix[buf][slot] = make_int4(c, r, d, 1);
+    s_lin[buf][slot] = b * img + ((int64_t)c * g.IR + r) * g.ID + d;
+  };
   auto decode = [&](int64_t p, int slot, int buf) {
     if (p < k_end) {
       int64_t t = p;
@@ -458,13 +549,9 @@ __global__ void __launch_bounds__(kVNT, 1)
       t /= g.OD;
       const int64_t orr = t % g.OR;
       t /= g.OR;
-      const int64_t oc = t % g.OC, b = t / g.OC;
-      s_base[buf][slot] = b * img;
-      s_c[buf][slot] = (int)(oc * g.sc) - g.pc;
-      s_r[buf][slot] = (int)(orr * g.sr) - g.pr;
-      s_d[buf][slot] = (int)(od * g.sd) - g.pd;
+      put_pixel(t / g.OC, t % g.OC, orr, od, slot, buf);
     } else {
-      s_base[buf][slot] = -1;
+      s_pix[buf][slot] = make_int4(0, 0, 0, 0);
     }
   };
 
@@ -484,12 +571,9 @@ __global__ void __launch_bounds__(kVNT, 1)
   auto decode_next = [&](int slot, int buf) {
     if (dp < k_end) {
       const int64_t orr = g.OD == 1 ? dq : dq / g.OD, od = dq - orr * g.OD;
-      s_base[buf][slot] = db * img;
-      s_c[buf][slot] = (int)(doc * g.sc) - g.pc;
-      s_r[buf][slot] = (int)(orr * g.sr) - g.pr;
-      s_d[buf][slot] = (int)(od * g.sd) - g.pd;
+      put_pixel(db, doc, orr, od, slot, buf);
     } else {
-      s_base[buf][slot] = -1;
+      s_pix[buf][slot] = make_int4(0, 0, 0, 0);
     }
     dp += kVBK;
     dq += kVBK;
@@ -502,82 +586,112 @@ __global__ void __launch_bounds__(kVNT, 1)
     }
   };
 
-  // FWD slab position: tap (kc, kr, kd) and first channel ci0 of slab k0
-  int kc = 0, kr = 0, kd = 0;
-  int64_t ci0 = 0;
+  // FWD slab position: tap (kc, kr, kd) = number `tap`, first channel ci0 of
+  // slab k0, and their offset soff from a window's origin
+  int kc = 0, kr = 0, kd = 0, tap = 0;
+  int64_t ci0 = 0, soff = 0;
+  auto tap_offset = [&]() {
+    soff = (((int64_t)kc * g.dc * g.IR + (int64_t)kr * g.dr) * g.ID + (int64_t)kd * g.dd) * g.Ci;
+  };
   if (MODE == FWD) {
-    int64_t tap = k_begin / g.Ci;
-    ci0 = k_begin - tap * g.Ci;
-    kd = (int)(tap % g.KD);
-    tap /= g.KD;
-    kr = (int)(tap % g.KR);
-    kc = (int)(tap / g.KR);
+    int64_t t = k_begin / g.Ci;
+    ci0 = k_begin - t * g.Ci;
+    tap = (int)t;
+    kd = (int)(t % g.KD);
+    t /= g.KD;
+    kr = (int)(t % g.KR);
+    kc = (int)(t / g.KR);
+    tap_offset();
+    soff += ci0;
+    if (MASKS && tap >= 32) row_masks(tap & ~31, false);
   }
 
-  // A: FWD RQ float4 (pixels), BWDK 16/AKS float4 (k rows); B: BH float4
+  // A: FWD RQ float4 (pixels), BWDK 16/AKS float4 (k rows)
   constexpr int AH = MODE == FWD ? RQ : kVBK / AKS;
-  float4 va[AH], vb[S::BH];
-  // B: float4 column bcol of k rows bk (+ 8)
+  // B: float4 column bcol of k rows bk + BKS*h, or (BT) k quad aq of rows n
   constexpr int BQ = BN / 4;  // float4 per k row of B
+  constexpr int BKS = NT / BQ > kVBK ? kVBK : NT / BQ;
+  constexpr int BH = BT ? (BN * 4 + NT - 1) / NT : kVBK / BKS;
   const int bcol = (tid % BQ) * 4;
   const int bk = tid / BQ;
-  const bool bval = bk < kVBK && n0 + bcol < g.N;  // (256x32: threads past 128 load no B)
+  const bool bval = bk < BKS && n0 + bcol < g.N;
+  float4 va[AH], vb[BH];
 
   // global -> registers for slab k0 (FWD: at tap kc/kr/kd, channels ci0..)
   auto load = [&](int64_t k0, int buf) {
     if (MODE == FWD) {
 #pragma unroll
       for (int h = 0; h < AH; ++h) {
-        const int c = ac[h] + kc * g.dc, r = ar[h] + kr * g.dr, d = ad[h] + kd * g.dd;
         va[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (abase[h] >= 0 && (unsigned)c < (unsigned)g.IC && (unsigned)r < (unsigned)g.IR &&
-            (unsigned)d < (unsigned)g.ID)
-          va[h] = ldg4(A0 + (abase[h] + ((int64_t)c * g.IR + r) * g.ID + d) * g.Ci + ci0 + aq * 4);
+        if (MASKS) {
+          if ((amask[h] >> (tap & 31)) & 1u) va[h] = ldg4(arow[h] + soff);
+        } else {
+          const int c = ac[h] + kc * g.dc, r = ar[h] + kr * g.dr, d = ad[h] + kd * g.dd;
+          if (abase[h] >= 0 && (unsigned)c < (unsigned)g.IC && (unsigned)r < (unsigned)g.IR &&
+              (unsigned)d < (unsigned)g.ID)
+            va[h] = ldg4(A0 + (abase[h] + ((int64_t)c * g.IR + r) * g.ID + d) * g.Ci + ci0 + aq * 4);
+        }
       }
     } else {
 #pragma unroll
       for (int h = 0; h < AH; ++h) {
-        const int kl = ak + AKS * h;
-        const int64_t base = s_base[buf][kl];
         va[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (mval && base >= 0) {
-          const int c = s_c[buf][kl] + t_dc, r = s_r[buf][kl] + t_dr, d = s_d[buf][kl] + t_dd;
-          if ((unsigned)c < (unsigned)g.IC && (unsigned)r < (unsigned)g.IR &&
-              (unsigned)d < (unsigned)g.ID)
-            va[h] = ldg4(A0 + (base + ((int64_t)c * g.IR + r) * g.ID + d) * g.Ci + mci);
+        if (mval && ak < AKS) {
+          const int kl = ak + AKS * h;
+          const int4 px = s_pix[buf][kl];
+          if (px.w && (unsigned)(px.x + t_dc) < (unsigned)g.IC &&
+              (unsigned)(px.y + t_dr) < (unsigned)g.IR && (unsigned)(px.z + t_dd) < (unsigned)g.ID)
+            va[h] = ldg4(a_tap + s_lin[buf][kl] * g.Ci);
         }
       }
     }
 #pragma unroll
-    for (int h = 0; h < S::BH; ++h) {
-      const int64_t kq = k0 + bk + 8 * h;
-      vb[h] = (bval && kq < k_end) ? ldg4(B0 + kq * g.N + n0 + bcol)
-                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int h = 0; h < BH; ++h) {
+      vb[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (BT) {
+        const int n = (tid >> 2) + NT / 4 * h;
+        if (n < BN && n0 + n < g.N) vb[h] = ldg4(B0 + (n0 + n) * g.K + k0 + aq * 4);
+      } else {
+        const int64_t kq = k0 + bk + BKS * h;
+        if (bval && kq < k_end) vb[h] = ldg4(B0 + kq * g.N + n0 + bcol);
+      }
     }
   };
   auto store = [&](int buf) {
     if (MODE == FWD) {
 #pragma unroll
       for (int h = 0; h < AH; ++h) {
-        const int row = ((tid >> 2) + 64 * h) ^ (aq << 3);
+        const int row = ((tid >> 2) + NT / 4 * h) ^ (aq << 3);
         As[buf][aq * 4 + 0][row] = va[h].x;
         As[buf][aq * 4 + 1][row] = va[h].y;
         As[buf][aq * 4 + 2][row] = va[h].z;
         As[buf][aq * 4 + 3][row] = va[h].w;
       }
-    } else {
+    } else if (ak < AKS) {
 #pragma unroll
       for (int h = 0; h < AH; ++h)
         *reinterpret_cast<float4 *>(&As[buf][ak + AKS * h][mq]) = va[h];
     }
-    if (bk < kVBK) {
+    if (BT) {
 #pragma unroll
-      for (int h = 0; h < S::BH; ++h)
-        *reinterpret_cast<float4 *>(&Bs[buf][bk + 8 * h][bcol]) = vb[h];
+      for (int h = 0; h < BH; ++h) {
+        const int n = (tid >> 2) + NT / 4 * h, col = n ^ (aq << 3);
+        if (n < BN) {
+          Bs[buf][aq * 4 + 0][col] = vb[h].x;
+          Bs[buf][aq * 4 + 1][col] = vb[h].y;
+          Bs[buf][aq * 4 + 2][col] = vb[h].z;
+          Bs[buf][aq * 4 + 3][col] = vb[h].w;
+        }
+      }
+    } else if (bk < BKS) {
+#pragma unroll
+      for (int h = 0; h < BH; ++h)
+        *reinterpret_cast<float4 *>(&Bs[buf][bk + BKS * h][bcol]) = vb[h];
     }
   };
   auto next_tap = [&]() {
     ci0 += kVBK;
+    soff += kVBK;
     if (ci0 == g.Ci) {
       ci0 = 0;
       if (++kd == g.KD) {
@@ -587,14 +701,16 @@ __global__ void __launch_bounds__(kVNT, 1)
           ++kc;
         }
       }
+      tap_offset();
+      if (MASKS && (++tap & 31) == 0) row_masks(tap, false);
     }
   };
 
-  float acc[8][4 * NJ];
+  uint64_t acc[TM / 2][TN];  // rows 2i, 2i + 1 of the thread's TM
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < TM / 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 4 * NJ; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0;
 
   if (k_begin < k_end) {
     if (MODE == BWDK) {
@@ -615,24 +731,26 @@ __global__ void __launch_bounds__(kVNT, 1)
       if (MODE == BWDK && tid < kVBK) decode_next(tid, buf);  // pixel kn + 16 + tid
 #pragma unroll
       for (int k = 0; k < kVBK; ++k) {
-        const int sw = MODE == FWD ? ((k >> 2) << 3) : 0;
-        float a[8];
+        const int sw = MODE == FWD ? ((k >> 2) << 3) : 0, swb = BT ? ((k >> 2) << 3) : 0;
+        uint64_t a[TM / 2];
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const float4 f =
-              *reinterpret_cast<const float4 *>(&As[buf][k][(S::RSTEP * q + ty * 4) ^ sw]);
-          a[4 * q] = f.x; a[4 * q + 1] = f.y; a[4 * q + 2] = f.z; a[4 * q + 3] = f.w;
+        for (int q = 0; q < NI; ++q) {
+          const ulonglong2 f =
+              *reinterpret_cast<const ulonglong2 *>(&As[buf][k][(RSTEP * q + ty * 4) ^ sw]);
+          a[2 * q] = f.x;
+          a[2 * q + 1] = f.y;
         }
-        float b[4 * NJ];
 #pragma unroll
         for (int q = 0; q < NJ; ++q) {
-          const float4 f = *reinterpret_cast<const float4 *>(&Bs[buf][k][64 * q + tx * 4]);
-          b[4 * q] = f.x; b[4 * q + 1] = f.y; b[4 * q + 2] = f.z; b[4 * q + 3] = f.w;
+          const float4 f =
+              *reinterpret_cast<const float4 *>(&Bs[buf][k][(CSTEP * q + tx * 4) ^ swb]);
+          const uint64_t b[4] = {pack2(f.x, f.x), pack2(f.y, f.y), pack2(f.z, f.z),
+                                 pack2(f.w, f.w)};
+#pragma unroll
+          for (int i = 0; i < TM / 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) ffma2(acc[i][4 * q + j], a[i], b[j]);
         }
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 4 * NJ; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
       }
       if (more) {
         store(buf ^ 1);
@@ -645,8 +763,8 @@ __global__ void __launch_bounds__(kVNT, 1)
 
   float *Cz = C + (int64_t)blockIdx.z * g.M * g.N;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int64_t m = m0 + S::RSTEP * (i >> 2) + ty * 4 + (i & 3);
+  for (int i = 0; i < TM; ++i) {
+    const int64_t m = m0 + RSTEP * (i >> 2) + ty * 4 + (i & 3);
     if (m >= g.M) continue;
     int64_t row = m;
     if (MODE == FWD && g.ystrided) {
@@ -660,26 +778,32 @@ __global__ void __launch_bounds__(kVNT, 1)
     }
 #pragma unroll
     for (int q = 0; q < NJ; ++q) {
-      const int64_t n = n0 + q * 64 + tx * 4;
+      const int64_t n = n0 + q * CSTEP + tx * 4;
       if (n >= g.N) continue;
-      const float4 v =
-          make_float4(acc[i][4 * q], acc[i][4 * q + 1], acc[i][4 * q + 2], acc[i][4 * q + 3]);
+      float v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float lo, hi;
+        unpack2(acc[i >> 1][4 * q + j], lo, hi);
+        v[j] = (i & 1) ? hi : lo;
+        if (MODE == FWD) v[j] = with_bias_act(v[j], g, n + j);
+      }
+      float *dst = Cz + row * g.N + n;
       if (MODE == FWD && g.ystrided == 2) {
         const int64_t t = n / g.s2d_ci, ci = n - t * g.s2d_ci;
         const int64_t tc = t / (g.s2d_kr * g.s2d_kd), tr = (t / g.s2d_kd) % g.s2d_kr,
                       td = t % g.s2d_kd;
-        *reinterpret_cast<float4 *>(
-            Cz + (row + tc * g.s2d_tc + tr * g.s2d_tr + td) * g.s2d_ci + ci) = v;
-      } else {
-        *reinterpret_cast<float4 *>(Cz + row * g.N + n) = v;
+        dst = Cz + (row + tc * g.s2d_tc + tr * g.s2d_tr + td) * g.s2d_ci + ci;
       }
+      *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
     }
   }
 }
 
 // Whether the float32 vector path takes a launch: 16-byte aligned operands,
-// N a multiple of 4 (128-, 64- or 32-wide tiles), FWD slabs inside one tap
-// (Ci % 16, whole slabs per split), BWDK rows in quads of one tap (Ci % 4).
+// N a multiple of 4, FWD slabs inside one tap (Ci % 16, whole slabs per
+// split), BWDK rows in quads of one tap (Ci % 4); BWDI only as the product
+// x w^T of a 1x1 geometry (simt_gemm), with whole slabs of K = Co.
 bool f32v_ok(int mode, const Dev &d, const void *A, const void *B, const void *C,
              int64_t kps) {
   auto al = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
@@ -687,22 +811,53 @@ bool f32v_ok(int mode, const Dev &d, const void *A, const void *B, const void *C
   if (d.IC >= (1 << 30) || d.IR >= (1 << 30) || d.ID >= (1 << 30)) return false;
   if (mode == FWD) return d.Ci % kVBK == 0 && kps % kVBK == 0;
   if (mode == BWDK) return d.Ci % 4 == 0;
-  return false;
+  return d.KC * d.KR * d.KD == 1 && d.sc == 1 && d.sr == 1 && d.sd == 1 && d.pc == 0 &&
+         d.pr == 0 && d.pd == 0 && d.IC == d.OC && d.IR == d.OR && d.ID == d.OD &&
+         d.Co % kVBK == 0 && kps % kVBK == 0;
 }
 
-template <int MODE>
+template <int MODE, int BM, int BN, int TM, int TN, bool BT>
+cudaError_t launch_f32v_tile(const Dev &d, const float *A, const float *B, float *C, int splits,
+                             int64_t kps, cudaStream_t s) {
+  dim3 grid((unsigned)ceil_div(d.M, BM), (unsigned)ceil_div(d.N, BN), (unsigned)splits);
+  return launch_pdl(conv_f32v_kernel<MODE, BM, BN, TM, TN, BT>, grid,
+                    dim3((BM / TM) * (BN / TN)), 0, s, d, A, B, C, kps);
+}
+
+// The tile of a launch: the one whose busiest SM takes the least time: n * BM *
+// BN outputs (n whole tiles while they are resident together, else the average
+// plus half a tile of tail), at the tile's cost per output with the GPU full
+// (measured on [32;56;56;128] x [3;3;128;128]: 617, 699 and 790 us), over the
+// share of the FMA pipe that the resident tiles keep busy, about w / (w + 3) for
+// w warps (by registers 3 blocks of 128 x 64 fit, 4 of 128 x 32, 6 of 64 x 32).
+// Measured against each tile forced: it takes the fastest on wide, ragged (N =
+// 160, 96), 5x5x32x64, 3-D and [8;32;32;16] x [3;3;16;32] layers in all three passes,
+// or one within 3 %.
+int pick_f32v(const Dev &d, int splits) {
+  static const struct { int bm, bn, most; double cost; } t[] = {
+      {128, 64, 3, 1.0}, {128, 32, 4, 1.13}, {64, 32, 6, 1.33}};
+  int best = 0;
+  double least = 0;
+  for (int i = 0; i < 3; ++i) {
+    const int64_t tiles = ceil_div(d.M, t[i].bm) * ceil_div(d.N, t[i].bn) * splits;
+    const int64_t whole = ceil_div(tiles, 152);
+    const double n = whole <= t[i].most ? (double)whole : (double)tiles / 152 + 0.5;
+    const double w = 4.0 * std::min<double>(n, t[i].most);
+    const double c = n * t[i].bm * t[i].bn * t[i].cost * (w + 3) / w;
+    if (i == 0 || c < least) { least = c; best = i; }
+  }
+  return best;
+}
+
+template <int MODE, bool BT = false>
 int launch_f32v(const Dev &d, const float *A, const float *B, float *C, int splits, int64_t kps,
                 cudaStream_t s) {
-  const int cn = d.N > 64 ? 2 : (d.N > 32 ? 1 : 0);
-  const int bm = cn == 0 ? 256 : 128, bn = cn == 0 ? 32 : 64 * cn;
-  dim3 grid((unsigned)ceil_div(d.M, bm), (unsigned)ceil_div(d.N, bn), (unsigned)splits);
   cudaError_t e;
-  if (cn == 2)
-    e = launch_pdl(conv_f32v_kernel<MODE, 2>, grid, dim3(kVNT), 0, s, d, A, B, C, kps);
-  else if (cn == 1)
-    e = launch_pdl(conv_f32v_kernel<MODE, 1>, grid, dim3(kVNT), 0, s, d, A, B, C, kps);
-  else
-    e = launch_pdl(conv_f32v_kernel<MODE, 0>, grid, dim3(kVNT), 0, s, d, A, B, C, kps);
+  switch (pick_f32v(d, splits)) {
+    case 0: e = launch_f32v_tile<MODE, 128, 64, 8, 8, BT>(d, A, B, C, splits, kps, s); break;
+    case 1: e = launch_f32v_tile<MODE, 128, 32, 8, 4, BT>(d, A, B, C, splits, kps, s); break;
+    default: e = launch_f32v_tile<MODE, 64, 32, 4, 4, BT>(d, A, B, C, splits, kps, s);
+  }
   if (e == cudaSuccess) e = cudaGetLastError();
   note_launch();
   return e == cudaSuccess ? kOk : cuda_fail(e, "conv_f32v_kernel");
@@ -737,25 +892,48 @@ int launch_cfg(const Dev &d, const T *A, const T *B, T *C, int splits, int64_t k
   return e == cudaSuccess ? kOk : cuda_fail(e, "conv_simt_kernel");
 }
 
-// Tile choice by the GEMM's N (output channels for FWD, input channels for
-// BWDI, Co for BWDK).
+// The scalar kernel's tile.  4-byte elements: by the GEMM's N (output channels
+// for FWD, input channels for BWDI, Co for BWDK), and 32 rows for a
+// backward_kernel of at most 32 (tap, channel) rows (a one-channel image),
+// with slabs of 32 pixels: each slab costs a pixel decode and two barriers.
+// 8- and 16-byte elements: the FP64 pipe is slow enough that any tile feeds
+// it, so the smallest busiest SM wins, ceil(tiles / SMs) tiles of BM x BN, the
+// larger tile on a tie ([8;28;28;32] x [5;5;32;64]: 98 tiles of 64 x 64 leave a
+// third of the SMs idle, 883 us; 392 of 32 x 32, 625 us).
 template <typename T, int MODE>
 int launch_any(const Dev &d, const T *A, const T *B, T *C, int splits, int64_t kps,
                cudaStream_t s) {
   if constexpr (std::is_same_v<T, float>) {
-    if ((MODE == FWD || MODE == BWDK) && f32v_ok(MODE, d, A, B, C, kps))
-      return launch_f32v<MODE == BWDK ? BWDK : FWD>(d, A, B, C, splits, kps, s);
+    if (f32v_ok(MODE, d, A, B, C, kps)) {
+      if (MODE != BWDI) return launch_f32v<MODE == BWDK ? BWDK : FWD>(d, A, B, C, splits, kps, s);
+      // dX = dY w^T of a 1x1 geometry: a forward product with w read as [n][k]
+      Dev f = d;
+      f.Ci = d.Co;
+      f.Co = d.Ci;
+      return launch_f32v<FWD, true>(f, A, B, C, splits, kps, s);
+    }
   }
   if constexpr (sizeof(T) == 4) {
+    if constexpr (MODE == BWDK) {
+      if (d.M <= 32) return launch_cfg<T, MODE, 32, 32, 32, 2, 2>(d, A, B, C, splits, kps, s);
+    }
     if (d.N > 64) return launch_cfg<T, MODE, 128, 128, 8, 8, 8>(d, A, B, C, splits, kps, s);
     if (d.N > 32) return launch_cfg<T, MODE, 128, 64, 8, 8, 4>(d, A, B, C, splits, kps, s);
     return launch_cfg<T, MODE, 128, 32, 8, 4, 4>(d, A, B, C, splits, kps, s);
   } else {
+    auto busiest = [&](int bm, int bn) {
+      return ceil_div(ceil_div(d.M, bm) * ceil_div(d.N, bn) * splits, 152) * bm * bn;
+    };
+    const int64_t big = d.N > 32 ? busiest(64, 64) : busiest(64, 32), mid = busiest(32, 32);
+    if (busiest(16, 32) < std::min(big, mid))
+      return launch_cfg<T, MODE, 16, 32, 16, 1, 2>(d, A, B, C, splits, kps, s);
+    if (mid < big) return launch_cfg<T, MODE, 32, 32, 8, 2, 2>(d, A, B, C, splits, kps, s);
     if (d.N > 32) return launch_cfg<T, MODE, 64, 64, 8, 4, 4>(d, A, B, C, splits, kps, s);
     return launch_cfg<T, MODE, 64, 32, 8, 4, 2>(d, A, B, C, splits, kps, s);
   }
 }
 
+// The tile that the split count of a reduction is planned for.
 template <typename T>
 int tile_m(const Dev &d) { return sizeof(T) == 4 ? (d.N <= 32 ? 256 : 128) : 64; }
 template <typename T>
@@ -765,8 +943,11 @@ int tile_n(const Dev &d) {
 }
 
 template <typename T>
-int fwd_t(const ConvGeom &g, const T *x, const T *w, T *y, cudaStream_t s) {
+int fwd_t(const ConvGeom &g, const T *x, const T *w, T *y, cudaStream_t s, const void *bias,
+          int act) {
   Dev d = make_dev(g, FWD);
+  d.bias = bias;
+  d.act = act;
   if (d.M == 0 || d.N == 0) return kOk;
   if (d.K == 0) {
     OWL_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * d.M * d.N, s));
@@ -955,8 +1136,10 @@ int bwdi_t(const ConvGeom &g, T *dx, const T *w, const T *dy, cudaStream_t s) {
 // The GEMM view of one pass with its reduction split across CTAs: each
 // split writes a partial, summed in split order by a second kernel
 // (deterministic).  A/B are the pass's operands in launch_any's order.
+// A bias (per column) and activation, if any, are applied to the finished sums.
 template <typename T, int MODE>
-int splitk_t(const ConvGeom &g, const T *A, const T *B, T *C, cudaStream_t s) {
+int splitk_t(Dtype dt, const ConvGeom &g, const T *A, const T *B, T *C, cudaStream_t s,
+             const void *bias = nullptr, int act = 0) {
   Dev d = make_dev(g, MODE);
   if (d.M == 0 || d.N == 0) return kOk;
   if (d.K == 0) {
@@ -971,28 +1154,30 @@ int splitk_t(const ConvGeom &g, const T *A, const T *B, T *C, cudaStream_t s) {
   int splits = (int)std::max<int64_t>(1, std::min<int64_t>(want, std::min<int64_t>(max_by_k, 256)));
   int64_t kps = ceil_div(ceil_div(d.K, splits), 16) * 16;
   splits = (int)ceil_div(d.K, kps);
-  if (splits == 1) return launch_any<T, MODE>(d, A, B, C, 1, kps, s);
+  if (splits == 1) {
+    if (MODE == FWD) {
+      d.bias = bias;
+      d.act = act;
+    }
+    int rc = launch_any<T, MODE>(d, A, B, C, 1, kps, s);
+    if (rc || MODE == FWD || (!bias && act == OWLGPU_ACT_NONE)) return rc;
+    return bias_act_inplace(dt, C, bias, d.M * d.N, d.N, act, s);
+  }
   void *ws = nullptr;
   size_t bytes = sizeof(T) * (size_t)splits * d.M * d.N;
   int rc = scratch_alloc(&ws, bytes, s);
   if (rc) return rc;
   rc = launch_any<T, MODE>(d, A, B, (T *)ws, splits, kps, s);
   if (rc == kOk) {
-    int64_t n = d.M * d.N;
-    int blocks = (int)std::min<int64_t>(ceil_div(n, 256), 4 * 152);
-    cudaError_t e = launch_pdl(splitk_reduce_kernel<T>, dim3(blocks), dim3(256), 0, s,
-                               (const T *)ws, C, (int64_t)n, splits);
-    if (e == cudaSuccess) e = cudaGetLastError();
-    note_launch();
-    if (e != cudaSuccess) rc = cuda_fail(e, "splitk_reduce_kernel");
+    rc = sum_splits<T>((const T *)ws, C, d.M * d.N, splits, (const T *)bias, d.N, act, s);
   }
   scratch_free(ws, s);
   return rc;
 }
 
 template <typename T>
-int bwdk_t(const ConvGeom &g, const T *x, T *dw, const T *dy, cudaStream_t s) {
-  return splitk_t<T, BWDK>(g, x, dy, dw, s);
+int bwdk_t(Dtype dt, const ConvGeom &g, const T *x, T *dw, const T *dy, cudaStream_t s) {
+  return splitk_t<T, BWDK>(dt, g, x, dy, dw, s);
 }
 
 // backward_kernel, float32, with the split-K partials written into a
@@ -1019,13 +1204,7 @@ int bwdk_f32_into(const ConvGeom &g, const float *x, float *dw, const float *dy,
   if (splits == 1) return launch_any<float, BWDK>(d, x, dy, dw, 1, kps, s);
   int rc = launch_any<float, BWDK>(d, x, dy, ws, splits, kps, s);
   if (rc != kOk) return rc;
-  int64_t n = d.M * d.N;
-  int blocks = (int)std::min<int64_t>(ceil_div(n, 256), 4 * 152);
-  cudaError_t e = launch_pdl(splitk_reduce_kernel<float>, dim3(blocks), dim3(256), 0, s,
-                             (const float *)ws, dw, (int64_t)n, splits);
-  if (e == cudaSuccess) e = cudaGetLastError();
-  note_launch();
-  return e == cudaSuccess ? kOk : cuda_fail(e, "splitk_reduce_kernel");
+  return sum_splits<float>(ws, dw, d.M * d.N, splits, nullptr, d.N, 0, s);
 }
 
 }  // namespace
@@ -1051,10 +1230,14 @@ static int by_dtype(Dtype dt, F f) {
 }
 
 int simt_conv_fwd(Dtype dt, const ConvGeom &g, const void *x, const void *w, void *y,
-                  cudaStream_t s) {
+                  cudaStream_t s, const void *bias, int act) {
+  if (g.taps() * g.Ci == 0 && g.y_elems() > 0 && (bias || act != OWLGPU_ACT_NONE)) {
+    const int rc = simt_conv_fwd(dt, g, x, w, y, s, nullptr, OWLGPU_ACT_NONE);
+    return rc ? rc : bias_act_inplace(dt, y, bias, g.y_elems(), g.Co, act, s);
+  }
   return by_dtype(dt, [&](auto *tag) {
     using T = std::remove_pointer_t<decltype(tag)>;
-    return fwd_t<T>(g, (const T *)x, (const T *)w, (T *)y, s);
+    return fwd_t<T>(g, (const T *)x, (const T *)w, (T *)y, s, bias, act);
   });
 }
 
@@ -1069,17 +1252,20 @@ int simt_conv_bwd_input(Dtype dt, const ConvGeom &g, void *dx, const void *w, co
 // A pass of a 1x1 geometry as a split-K GEMM (the dense layer's products on
 // the CUDA cores): mode 0 forward (a = x, b = w, c = y), 1 backward_input
 // (a = dy, b = w, c = dx), 2 backward_kernel (a = x, b = dy, c = dw).
+// `bias` (per column of c, or null) and `act` are applied to the product.
 int simt_gemm(Dtype dt, int mode, const ConvGeom &g, const void *a, const void *b, void *c,
-              cudaStream_t s) {
+              cudaStream_t s, const void *bias, int act) {
   if (dt != F32 && dt != F64) {
     set_error("simt_gemm: real element kinds only");
     return kErrInvalid;
   }
   return by_dtype(dt, [&](auto *tag) {
     using T = std::remove_pointer_t<decltype(tag)>;
-    if (mode == FWD) return splitk_t<T, FWD>(g, (const T *)a, (const T *)b, (T *)c, s);
-    if (mode == BWDI) return splitk_t<T, BWDI>(g, (const T *)a, (const T *)b, (T *)c, s);
-    return splitk_t<T, BWDK>(g, (const T *)a, (const T *)b, (T *)c, s);
+    if (mode == FWD)
+      return splitk_t<T, FWD>(dt, g, (const T *)a, (const T *)b, (T *)c, s, bias, act);
+    if (mode == BWDI)
+      return splitk_t<T, BWDI>(dt, g, (const T *)a, (const T *)b, (T *)c, s, bias, act);
+    return splitk_t<T, BWDK>(dt, g, (const T *)a, (const T *)b, (T *)c, s, bias, act);
   });
 }
 
@@ -1087,7 +1273,7 @@ int simt_conv_bwd_kernel(Dtype dt, const ConvGeom &g, const void *x, void *dw, c
                          cudaStream_t s) {
   return by_dtype(dt, [&](auto *tag) {
     using T = std::remove_pointer_t<decltype(tag)>;
-    return bwdk_t<T>(g, (const T *)x, (T *)dw, (const T *)dy, s);
+    return bwdk_t<T>(dt, g, (const T *)x, (T *)dw, (const T *)dy, s);
   });
 }
 

@@ -44,35 +44,60 @@ __global__ void bias_act_kernel(T *__restrict__ y, const T *__restrict__ bias, l
 
 // dz = dy * act'(from y); partial[chunk][c] = sum of dz over the chunk's
 // pixels, in pixel order within each of the 8 row groups, the groups summed
-// in order.  Block (32, 8): x = channel within a 32-channel tile, y = row
-// group.
-constexpr int kBiasRows = 8;
-template <typename T>
+// in order.  Block (32 / V, 8): x = V channels of a 32-channel tile (16-byte
+// vectors when the channels allow), y = row group.  HBM-bound: dy, y and dz once;
+// kBiasAhead rows' loads are issued before any of them is used.
+constexpr int kBiasRows = 8, kBiasAhead = 8;
+template <typename T, int V>
 __global__ void bias_act_bwd_kernel(const T *__restrict__ y, const T *__restrict__ dy,
                                     T *__restrict__ dz, T *__restrict__ partial, long long P,
                                     long long C, long long rows_per_chunk, int act) {
   asm volatile("griddepcontrol.wait;" ::: "memory");  // launched with launch_pdl
   __shared__ T red[kBiasRows][33];
-  const long long c = (long long)blockIdx.x * 32 + threadIdx.x;
+  struct alignas(sizeof(T) * V) Vec { T e[V]; };
+  const long long c = (long long)blockIdx.x * 32 + threadIdx.x * V;
   const long long p0 = (long long)blockIdx.y * rows_per_chunk;
   const long long p1 = min(P, p0 + rows_per_chunk);
-  T acc = T(0);
-  if (c < C) {
-    for (long long p = p0 + threadIdx.y; p < p1; p += kBiasRows) {
-      const long long i = p * C + c;
-      T g = dy[i];
-      if (act == OWLGPU_ACT_RELU && !(y[i] > T(0))) g = T(0);
-      if (dz) dz[i] = g;
-      acc += g;
+  T acc[V];
+#pragma unroll
+  for (int e = 0; e < V; ++e) acc[e] = T(0);
+  auto one = [&](long long q, Vec g, const Vec &a) {
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      if (act == OWLGPU_ACT_RELU && !(a.e[e] > T(0))) g.e[e] = T(0);
+      acc[e] += g.e[e];
     }
+    if (dz) *reinterpret_cast<Vec *>(dz + q * C + c) = g;
+  };
+  auto outputs = [&](long long q) {  // y is read only where the mask needs it
+    return act == OWLGPU_ACT_RELU ? *reinterpret_cast<const Vec *>(y + q * C + c) : Vec{};
+  };
+  if (c < C) {
+    long long p = p0 + threadIdx.y;
+    for (; p + (kBiasAhead - 1) * kBiasRows < p1; p += kBiasRows * kBiasAhead) {
+      Vec g[kBiasAhead], a[kBiasAhead];
+#pragma unroll
+      for (int u = 0; u < kBiasAhead; ++u) {
+        g[u] = *reinterpret_cast<const Vec *>(dy + (p + u * kBiasRows) * C + c);
+        a[u] = outputs(p + u * kBiasRows);
+      }
+#pragma unroll
+      for (int u = 0; u < kBiasAhead; ++u) one(p + u * kBiasRows, g[u], a[u]);
+    }
+    for (; p < p1; p += kBiasRows)
+      one(p, *reinterpret_cast<const Vec *>(dy + p * C + c), outputs(p));
   }
-  red[threadIdx.y][threadIdx.x] = acc;
+#pragma unroll
+  for (int e = 0; e < V; ++e) red[threadIdx.y][threadIdx.x * V + e] = acc[e];
   __syncthreads();
   if (threadIdx.y == 0 && c < C && partial) {
-    T s = red[0][threadIdx.x];
 #pragma unroll
-    for (int r = 1; r < kBiasRows; ++r) s += red[r][threadIdx.x];
-    partial[(long long)blockIdx.y * C + c] = s;
+    for (int e = 0; e < V; ++e) {
+      T s = red[0][threadIdx.x * V + e];
+#pragma unroll
+      for (int r = 1; r < kBiasRows; ++r) s += red[r][threadIdx.x * V + e];
+      partial[(long long)blockIdx.y * C + c + e] = s;
+    }
   }
 }
 
@@ -88,6 +113,7 @@ __global__ void sum_chunks_kernel(const T *__restrict__ partial, T *__restrict__
   const long long c = (long long)blockIdx.x * 32 + threadIdx.x;
   T s = T(0);
   if (c < C)
+#pragma unroll 8
     for (int k = threadIdx.y; k < chunks; k += 32) s += partial[(long long)k * C + c];
   red[threadIdx.y][threadIdx.x] = s;
   __syncthreads();
@@ -202,7 +228,7 @@ int bias_act(T *y, const T *bias, long long n, long long C, int act, cudaStream_
 // read as [N][K]), TN a backward_kernel (X = A over K pixels, dY = B).
 template <typename T>
 int simt_dot(Dtype dt, bool ta, bool tb, long long M, long long N, long long K, const T *a,
-             const T *b, T *c, cudaStream_t s) {
+             const T *b, T *c, const T *bias, int act, cudaStream_t s) {
   ConvGeom g{};
   g.B = 1; g.IC = 1; g.ID = 1; g.OC = 1; g.OD = 1;
   g.KC = g.KR = g.KD = 1;
@@ -210,14 +236,14 @@ int simt_dot(Dtype dt, bool ta, bool tb, long long M, long long N, long long K, 
   g.pc = g.pr = g.pd = 0;
   if (!ta && !tb) {
     g.IR = g.OR = M; g.Ci = K; g.Co = N;
-    return simt_gemm(dt, 0, g, a, b, c, s);
+    return simt_gemm(dt, 0, g, a, b, c, s, bias, act);
   }
   if (!ta && tb) {
     g.IR = g.OR = M; g.Ci = N; g.Co = K;
-    return simt_gemm(dt, 1, g, a, b, c, s);
+    return simt_gemm(dt, 1, g, a, b, c, s, bias, act);
   }
   g.IR = g.OR = K; g.Ci = M; g.Co = N;
-  return simt_gemm(dt, 2, g, a, b, c, s);
+  return simt_gemm(dt, 2, g, a, b, c, s, bias, act);
 }
 
 template <typename T>
@@ -240,9 +266,7 @@ int dot_t(Dtype dt, const char *fn, const T *a, const T *b, T *c, long m, long n
       if (rc != kErrUnsupported) return rc;
     }
   }
-  int rc = simt_dot<T>(dt, trans_a != 0, trans_b != 0, m, n, k, a, b, c, s);
-  if (rc) return rc;
-  return bias_act<T>(c, bias, (long long)m * n, n, act, s);
+  return simt_dot<T>(dt, trans_a != 0, trans_b != 0, m, n, k, a, b, c, bias, act, s);
 }
 
 template <typename T>
@@ -257,9 +281,10 @@ int bias_act_bwd_t(const char *fn, const T *y, const T *dy, T *dz, T *db, long P
     return kOk;
   }
   if (!db && !dz) return kOk;
-  // pixel chunks: about four blocks per SM over all channel tiles
+  // pixel chunks: about sixteen blocks (of 64 threads with 16-byte vectors) per
+  // SM over all channel tiles, at least 64 pixels each
   const long long ctiles = (C + 31) / 32;
-  long long chunks = std::max<long long>(1, std::min<long long>(4 * 152 / ctiles + 1, P / 64));
+  long long chunks = std::max<long long>(1, std::min<long long>(16 * 152 / ctiles + 1, P / 64));
   chunks = std::min<long long>(chunks, 4096);
   const long long rows = (P + chunks - 1) / chunks;
   chunks = (P + rows - 1) / rows;
@@ -268,8 +293,15 @@ int bias_act_bwd_t(const char *fn, const T *y, const T *dy, T *dz, T *db, long P
     int rc = scratch_alloc((void **)&part, sizeof(T) * (size_t)(chunks * C), s);
     if (rc) return rc;
   }
-  cudaError_t e = launch_pdl(bias_act_bwd_kernel<T>, dim3((unsigned)ctiles, (unsigned)chunks),
-                             dim3(32, kBiasRows), 0, s, y, dy, dz, part, P, C, rows, act);
+  // 16-byte vectors of channels where every pixel's channels start aligned
+  constexpr int V = 16 / (int)sizeof(T);
+  const bool vec = C % V == 0 && (uintptr_t)dy % 16 == 0 && (uintptr_t)dz % 16 == 0 &&
+                   (act != OWLGPU_ACT_RELU || (uintptr_t)y % 16 == 0);
+  const dim3 grid((unsigned)ctiles, (unsigned)chunks);
+  cudaError_t e = vec ? launch_pdl(bias_act_bwd_kernel<T, V>, grid, dim3(32 / V, kBiasRows), 0, s,
+                                   y, dy, dz, part, P, C, rows, act)
+                      : launch_pdl(bias_act_bwd_kernel<T, 1>, grid, dim3(32, kBiasRows), 0, s, y,
+                                   dy, dz, part, P, C, rows, act);
   if (e == cudaSuccess) e = cudaGetLastError();
   note_launch();
   int rc = e == cudaSuccess ? kOk : cuda_fail(e, "bias_act_bwd_kernel");
