@@ -342,8 +342,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
       if (sl < na) slot_plan(A, sl, k_begin, sp.base[q], sp.off[q]);
       else if (sl < total) slot_plan(B, sl - na, k_begin, sp.base[q], sp.off[q]);
     }
-    // plain strided operands whose rows start 16-byte aligned (the fast path)
-    const bool aligned = !p.s2d.on && ((uintptr_t)p.a & 15) == 0 && ((uintptr_t)p.b & 15) == 0 &&
+    // plain strided operands whose rows start 16-byte aligned and, MN-major,
+    // fill whole 8-row chunks (the fast path: its slots load whole chunks)
+    const bool aligned = !p.s2d.on && (p.a_kmaj || p.M % 8 == 0) && (p.b_kmaj || p.N % 8 == 0) && ((uintptr_t)p.a & 15) == 0 && ((uintptr_t)p.b & 15) == 0 &&
                          (p.a_kmaj ? p.a_sm % 4 == 0 : p.a_sk % 4 == 0) &&
                          (p.b_kmaj ? p.b_sn % 4 == 0 : p.b_sk % 4 == 0);
     // ... and 32-byte aligned: one 32-byte load per slot
