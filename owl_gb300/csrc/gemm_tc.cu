@@ -344,7 +344,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     }
     // plain strided operands whose rows start 16-byte aligned and, MN-major,
     // fill whole 8-row chunks (the fast path: its slots load whole chunks)
-    const bool aligned = !p.s2d.on && (p.a_kmaj || p.M % 8 == 0) && (p.b_kmaj || p.N % 8 == 0) && ((uintptr_t)p.a & 15) == 0 && ((uintptr_t)p.b & 15) == 0 &&
+    const bool aligned = !p.s2d.on && (p.a_kmaj || p.M % 8 == 0) &&
+                         (p.b_kmaj || p.N % 8 == 0) && ((uintptr_t)p.a & 15) == 0 &&
+                         ((uintptr_t)p.b & 15) == 0 &&
                          (p.a_kmaj ? p.a_sm % 4 == 0 : p.a_sk % 4 == 0) &&
                          (p.b_kmaj ? p.b_sn % 4 == 0 : p.b_sk % 4 == 0);
     // ... and 32-byte aligned: one 32-byte load per slot
@@ -510,6 +512,47 @@ int *tc_gemm_status_word() { return gemm_status_word(); }
 
 namespace {
 
+// Tile width and reduction split: the pair with the least estimated time, in
+// us.  A CTA takes kStart + its k blocks' staging, (128 + BN) x 64 floats at
+// the rate an SM stages them (8192^3 in BF16: 1.4 us a block of BN = 256), or
+// the four dependent MMAs of a block where that is longer (three times as
+// many in split BF16), + its store; CTAs run one an SM, in whole waves; a
+// split adds the ordered sum's launch and its traffic.  Wide tiles stage the
+// least, narrow ones and splits fill the GPU, and a split writes M x N floats
+// per piece, so small outputs split and large ones narrow.  Before, the tile was
+// always 256 wide and the split covered two waves: 256x1024x3136 (x w^T) took
+// 31.5 us in 208 CTAs of two k blocks each, 17.8 now; 3136x256x1024 31.6 and
+// 12.3, 256x3136x1024 17.8 and 15.8.
+struct Plan {
+  int bn;
+  long long kbs;  // k blocks per split
+};
+
+Plan plan(long long M, long long N, long long nkb, long long mt, int parts) {
+  constexpr double kStart = 3.0, kStage = 70e3, kStore = 60e3, kSum = 2.0, kSumRate = 5e6;
+  const double mma = (parts == 2 ? 3 : 1) * 4 * 0.085;
+  const int sms = num_sms();
+  const int n16 = (int)std::min<long long>(256, std::max<long long>(16, (N + 15) / 16 * 16));
+  Plan best{n16, nkb};
+  double least = -1;
+  for (int bn = n16; bn >= 16; bn = bn > 32 ? (bn - 1) / 32 * 32 : 0) {
+    const long long tiles = mt * ((N + bn - 1) / bn);
+    const double kb = std::max(mma, (kBM + bn) * (double)kBK * 4 / kStage);
+    for (long long splits = 1; splits <= std::min<long long>(nkb, 64); ++splits) {
+      const long long kbs = (nkb + splits - 1) / splits, used = (nkb + kbs - 1) / kbs;
+      if (used != splits) continue;
+      const long long waves = (tiles * splits + sms - 1) / sms;
+      double t = waves * (kStart + kbs * kb + kBM * (double)bn * 4 / kStore);
+      if (splits > 1) t += kSum + (splits + 1) * (double)M * N * 4 / kSumRate;
+      if (least < 0 || t < least) {
+        least = t;
+        best = {bn, kbs};
+      }
+    }
+  }
+  return best;
+}
+
 // Tiles, pipeline depth and split of a GEMM whose operands `p` describes
 // (a, b, strides, majorness, M, N, K, bias, act, s2d), then the launch and
 // the fixed-order sum of the splits into c.
@@ -519,23 +562,18 @@ int gemm_run(int prec, GemmParams p, float *c, cudaStream_t s) {
   const int act = p.act;
   const int kind = prec == OWLGPU_PREC_BF16X3 ? stage::K_BF16X3 : stage::K_BF16;
   const int parts = kind == stage::K_BF16X3 ? 2 : 1;
-  p.BN = N >= 256 ? 256 : (int)std::max<long long>(16, (N + 15) / 16 * 16);
   // one padded plane per k chunk (K-major) or per row chunk (MN-major)
   p.a_bytes = (unsigned)(p.a_kmaj ? 8 * (kBM + 1) * 16 : (kBM / 8) * (kBK + 1) * 16);
+  const long long nkb = (K + kBK - 1) / kBK, mt = (M + kBM - 1) / kBM;
+  const Plan pl = plan(M, N, nkb, mt, parts);
+  p.BN = pl.bn;
   p.b_bytes = (unsigned)(p.b_kmaj ? 8 * (p.BN + 1) * 16 : (p.BN / 8) * (kBK + 1) * 16);
   const size_t stage_bytes = (size_t)parts * (p.a_bytes + p.b_bytes);
   p.NS = (int)std::min<size_t>(4, (kSmemMax - 256) / stage_bytes);
   if (p.NS < 2) return kErrUnsupported;
-  const long long mt = (M + kBM - 1) / kBM, nt = (N + p.BN - 1) / p.BN;
-  const long long nkb = (K + kBK - 1) / kBK;
-  // split the reduction so that about two waves of CTAs cover the GPU, each
-  // split at least two k blocks deep
-  long long splits = std::max<long long>(1, (2LL * num_sms() + mt * nt - 1) / (mt * nt));
-  splits = std::min<long long>(splits, std::max<long long>(1, nkb / 2));
-  splits = std::min<long long>(splits, 64);
-  const long long kbs = (nkb + splits - 1) / splits;
-  p.kps = kbs * kBK;
-  p.splits = (int)((nkb + kbs - 1) / kbs);
+  const long long nt = (N + p.BN - 1) / p.BN;
+  p.kps = pl.kbs * kBK;
+  p.splits = (int)((nkb + pl.kbs - 1) / pl.kbs);
   p.small_off = (unsigned)p.BN;
   p.tmem_cols = 32;
   while (p.tmem_cols < (unsigned)(parts * p.BN)) p.tmem_cols <<= 1;
