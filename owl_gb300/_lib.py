@@ -97,14 +97,24 @@ def last_error() -> str:
 _entry: dict = {}  # name -> bound entry point (lib() and getattr once per name)
 
 
-def call(name: str, *args) -> None:
-    """Call an `int`-returning entry point and raise on a negative status."""
+def entry(name: str):
+    """The bound entry point `name`."""
     f = _entry.get(name)
     if f is None:
         f = _entry[name] = getattr(lib(), name)
-    rc = f(*args)
+    return f
+
+
+def failure(name: str, status: int) -> OwlGpuError:
+    """The error for a negative status of `name` (with the library's text)."""
+    return OwlGpuError(name, status, last_error())
+
+
+def call(name: str, *args) -> None:
+    """Call an `int`-returning entry point and raise on a negative status."""
+    rc = (_entry.get(name) or entry(name))(*args)
     if rc != 0:
-        raise OwlGpuError(name, rc, last_error())
+        raise failure(name, rc)
 
 
 def launch_count() -> int:

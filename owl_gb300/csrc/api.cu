@@ -34,13 +34,68 @@ int cuda_fail(cudaError_t e, const char *where) {
   return e == cudaErrorMemoryAllocation ? kErrNoMem : kErrCuda;
 }
 
+// Scratch comes from a stream-ordered pool of the library's own, one per
+// device, that keeps up to kScratchKeep bytes across synchronisations: the default
+// pool gives everything back at each one, and a call after it then took 250-400
+// us longer to map its workspace again.  The bound covers the workspaces of the
+// measured layers (at most 40 MB each) on several streams at once; what is above
+// it goes back at the next synchronisation, and all of it when an allocation
+// fails.
+constexpr uint64_t kScratchKeep = 256ull << 20;
+
+static cudaMemPool_t scratch_pool() {
+  static cudaMemPool_t pools[64] = {};
+  static std::mutex mu;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lk(mu);
+  if (!pools[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    uint64_t keep = kScratchKeep;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;  // the device's default pool serves
+    }
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    pools[dev] = pool;
+  }
+  return pools[dev];
+}
+
 int scratch_alloc(void **p, size_t bytes, cudaStream_t s) {
+  *p = nullptr;
+  if (bytes == 0) return kOk;
+  cudaMemPool_t pool = scratch_pool();
+  auto get = [&] {
+    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+  };
+  cudaError_t e = get();
+  if (e == cudaErrorMemoryAllocation && pool) {
+    cudaGetLastError();
+    cudaMemPoolTrimTo(pool, 0);
+    e = get();
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    *p = nullptr;
+    return cuda_fail(e, "cudaMallocAsync(scratch)");
+  }
+  return kOk;
+}
+
+// Memory that callers hold or that a host drop-in call stages its arrays in:
+// from the device's default pool (which the drop-in path keeps whole).
+static int device_alloc(void **p, size_t bytes, cudaStream_t s) {
   *p = nullptr;
   if (bytes == 0) return kOk;
   cudaError_t e = cudaMallocAsync(p, bytes, s);
   if (e != cudaSuccess) {
     cudaGetLastError();
-    return cuda_fail(e, "cudaMallocAsync(scratch)");
+    return cuda_fail(e, "cudaMallocAsync");
   }
   return kOk;
 }
@@ -349,7 +404,7 @@ static int host_call(std::vector<Buf> bufs, int64_t batch, int chunks, F body,
   cudaStream_t cin = one ? hs->s : hs->cin, cout = one ? hs->s : hs->cout;
   for (auto &b : bufs) {
     if (b.bytes == 0) continue;
-    rc = scratch_alloc(&b.dev, b.bytes, cin);
+    rc = device_alloc(&b.dev, b.bytes, cin);
     if (rc) break;
     if (b.in && !b.batched) {
       cudaError_t e = cudaMemcpyAsync(b.dev, b.host, b.bytes, cudaMemcpyHostToDevice, cin);
@@ -488,7 +543,7 @@ static int conv_host(ConvOp op, const ConvGeom &g, const void *a, const void *b,
         void *w = p[1];
         if (split) {
           if (ci == 0) {
-            const int r = scratch_alloc((void **)&part, sizeof(float) * (size_t)welems * chunks, s);
+            const int r = device_alloc((void **)&part, sizeof(float) * (size_t)welems * chunks, s);
             if (r) return r;
           }
           w = part + (size_t)welems * ci++;
@@ -662,7 +717,7 @@ int owlgpu_device_alloc(void **ptr, uint64_t bytes, void *stream) {
   }
   *ptr = nullptr;
   OWL_CUDA(cudaSetDevice(g_device.load()));
-  return scratch_alloc(ptr, (size_t)bytes, (cudaStream_t)stream);
+  return device_alloc(ptr, (size_t)bytes, (cudaStream_t)stream);
 }
 int owlgpu_device_free(void *ptr, void *stream) {
   if (ptr) OWL_CUDA(cudaFreeAsync(ptr, (cudaStream_t)stream));

@@ -29,10 +29,14 @@ from __future__ import annotations
 
 import numpy as np
 
-from .dense import NN, GpuBackend, InvalidArgument
+from .dense import (NN, GpuBackend, InvalidArgument, _pad_typ, _torch,
+                    calc_conv2d_output_shape, current_stream)
 
 ACT_NONE = 0
 ACT_RELU = 1
+
+
+_KINDS: dict = {}  # element type -> kind name, filled as types are met
 
 
 def _is_torch(a) -> bool:
@@ -40,12 +44,14 @@ def _is_torch(a) -> bool:
 
 
 def _kind(a) -> str:
-    dt = str(a.dtype)
-    if "float32" in dt:
-        return "float32"
-    if "float64" in dt:
-        return "float64"
-    raise InvalidArgument(f"{dt}: the layer kernels take float32 or float64 arrays")
+    k = _KINDS.get(a.dtype)
+    if k is None:
+        dt = str(a.dtype)
+        k = "float32" if "float32" in dt else ("float64" if "float64" in dt else None)
+        if k is None:
+            raise InvalidArgument(f"{dt}: the layer kernels take float32 or float64 arrays")
+        _KINDS[a.dtype] = k
+    return k
 
 
 class Layers:
@@ -65,10 +71,11 @@ class Layers:
         """True when the GPU kernels run: GPU backend and CUDA tensors."""
         if not self.gpu:
             return False
+        tensor = _torch().Tensor
         for a in arrays:
             if a is None:
                 continue
-            if not (_is_torch(a) and a.is_cuda and a.is_contiguous()):
+            if not ((type(a) is tensor or _is_torch(a)) and a.is_cuda and a.is_contiguous()):
                 raise InvalidArgument("the layer kernels take contiguous CUDA tensors")
         return True
 
@@ -76,16 +83,10 @@ class Layers:
     def _p(a) -> int | None:
         return None if a is None else a.data_ptr()
 
-    @staticmethod
-    def _stream():
-        import torch
-
-        return torch.cuda.current_stream().cuda_stream
+    _stream = staticmethod(current_stream)
 
     def _empty(self, like, shape):
-        import torch
-
-        return torch.empty(tuple(shape), dtype=like.dtype, device=like.device)
+        return _torch().empty(shape, dtype=like.dtype, device=like.device)
 
     # -- convolution + bias + activation
     def conv2d_bias_act(self, x, w, b, stride, padding="SAME", act=ACT_RELU):
@@ -96,8 +97,6 @@ class Layers:
             if b is not None:
                 y = y + b
             return np.maximum(y, 0) if act == ACT_RELU else y
-        from .dense import _pad_typ, calc_conv2d_output_shape
-
         B, IC, IR, Ci = x.shape
         KC, KR, kci, Co = w.shape
         if Ci != kci or len(stride) != 2:
