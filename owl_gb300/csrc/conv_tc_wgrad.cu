@@ -102,7 +102,9 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
   }
 }
 
-template <int KIND>
+// LANES: the operands are staged as whole 32-byte chunks (both arrays 32-byte
+// aligned, their channels multiples of 8), else element by element where needed.
+template <int KIND, bool LANES>
 __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_constant__ WgParams p) {
   constexpr int EB = (KIND == K_TF32) ? 4 : 2;
   constexpr int EPC = 16 / EB;
@@ -196,16 +198,46 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
   if (warp != kMmaWarp) {
     // ===================== producers: X halo + dY tile =====================
     bool staged = true;
-    long long k = 0;
-    for (long long t = t_begin; t < t_end; ++t, ++k) {
-      long long q = t;
-      const int v0 = (int)(q % p.v_tiles) * 8; q /= p.v_tiles;
-      const int u0 = (int)(q % p.u_tiles) * p.TU; q /= p.u_tiles;
-      const int ow = (int)(q % p.OW);
-      const int b = (int)(q / p.OW);
-      const int st = (int)(k % p.NS);
-      if (!wait_bar(smem_u32(&empty[st]), (uint32_t)(((k / p.NS) & 1) ^ 1), abort_flag,
-                    p.status, p.spin_limit)) {
+    // The tile's position and the ring's stage advance by counting: every warp
+    // decodes every tile, and the 64-bit divisions there took 14 of 128 us on
+    // [64;56;56;128] x [3;3;128;128].
+    int v0, u0, ow, b;
+    {
+      long long q = t_begin;
+      v0 = (int)(q % p.v_tiles) * 8; q /= p.v_tiles;
+      u0 = (int)(q % p.u_tiles) * p.TU; q /= p.u_tiles;
+      ow = (int)(q % p.OW);
+      b = (int)(q / p.OW);
+    }
+    const int v_end = p.v_tiles * 8, u_end = p.u_tiles * p.TU;
+    auto next_tile = [&]() {
+      if ((v0 += 8) == v_end) {
+        v0 = 0;
+        if ((u0 += p.TU) == u_end) {
+          u0 = 0;
+          if (++ow == p.OW) {
+            ow = 0;
+            ++b;
+          }
+        }
+      }
+    };
+    int st = 0;
+    uint32_t ph = 1;
+    // LANES: the chunks that exist are staged (the planes past the channels stay
+    // as they are: they only reach accumulator rows and columns that are not
+    // stored), QX and QY pixels of a row per lane and round
+    constexpr int QX = 5, QY = 4;
+    const stage::Lane lx(min(XPL, (p.Ci - mb * 128 + 7) / 8), lane);
+    const stage::Lane ly(min(YPL, (p.Co - nb * p.BN + 7) / 8), lane);
+    const int nx = lx.on ? (HVR - lx.i0 + lx.di - 1) / lx.di : 0;  // the lane's pixels of a row
+    const int ny = ly.on ? (8 - ly.i0 + ly.di - 1) / ly.di : 0;
+    const uint32_t lane_x = (uint32_t)lx.j * (uint32_t)p.PS * 16u + (uint32_t)lx.i0 * 16u,
+                   lane_y = (uint32_t)ly.j * (uint32_t)p.YPS * 16u + (uint32_t)ly.i0 * 16u;
+    const long long pix_x = (long long)p.sv * p.xsv * p.Ci, pix_y = p.ysv * (long long)p.Co;
+    const int steps_x = (HVR + lx.di - 1) / lx.di, steps_y = (8 + ly.di - 1) / ly.di;
+    for (long long t = t_begin; t < t_end; ++t, next_tile()) {
+      if (!wait_bar(smem_u32(&empty[st]), ph, abort_flag, p.status, p.spin_limit)) {
         staged = false;
         break;
       }
@@ -214,6 +246,45 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
       // X halo: rows (w, u) of HVR pixels x 128 channels of ci block mb;
       // dY tile: TU rows (u) of 8 output pixels x BN channels of co block nb.
       const int xcb = mb * 128, ycb = nb * p.BN;
+      if constexpr (LANES) {
+        const int ivs = v0 * p.sv - p.pv + minv;
+        const float *xt = p.x +
+                          ((long long)b * p.xsb + (long long)(ivs + lx.i0 * p.sv) * p.xsv) * p.Ci +
+                          xcb + lx.j * 8;
+        const float *yt = p.dy +
+                          ((long long)b * p.ysb + (long long)ow * p.ysw +
+                           (long long)(v0 + ly.i0) * p.ysv) * p.Co + ycb + ly.j * 8;
+        const int iw0 = ow * p.sw - p.pw + minw, iu0 = u0 * p.su - p.pu + minu;
+        int hw = 0, hu = pidx;
+        while (hu >= HU) { hu -= HU; ++hw; }
+        for (int r = pidx; r < xrows || r < p.TU; r += kProducerWarps) {
+          const int iw = iw0 + hw * p.sw, iu = iu0 + hu * p.su;
+          const bool xok = r < xrows && (unsigned)iw < (unsigned)p.IW &&
+                           (unsigned)iu < (unsigned)p.IU && lx.on;
+          const bool yok = r < p.TU && u0 + r < p.OU && ly.on;
+          const float *xs_ = xt + ((long long)iw * p.xsw + (long long)iu * p.xsu) * p.Ci;
+          const float *ys_ = yt + (long long)(u0 + r) * p.ysu * p.Co;
+          uint8_t *xdst = xd + lane_x + (uint32_t)(r * HVR) * 16u;
+          uint8_t *ydst = yd + lane_y + (uint32_t)r * 128u;
+          const int mx = r < xrows ? nx : 0, my = r < p.TU ? ny : 0;
+          const int sx = r < xrows ? steps_x : 0, sy = r < p.TU ? steps_y : 0;
+          for (int k = 0; k * QX < sx || k * QY < sy; ++k) {
+            float vx[QX][8], vy[QY][8];
+            stage::lane_load<QX>(xs_ + (long long)k * QX * lx.di * pix_x, lx.di * pix_x,
+                                 ivs + (lx.i0 + k * QX * lx.di) * p.sv, lx.di * p.sv,
+                                 xok ? (unsigned)p.IV : 0u, sx - k * QX, vx);
+            stage::lane_load<QY>(ys_ + (long long)k * QY * ly.di * pix_y, ly.di * pix_y,
+                                 v0 + ly.i0 + k * QY * ly.di, ly.di, yok ? (unsigned)p.OV : 0u,
+                                 sy - k * QY, vy);
+            stage::lane_store<KIND, QX>(xdst + (uint32_t)(k * QX * lx.di) * 16u,
+                                        (uint32_t)lx.di * 16u, p.x_bytes, mx - k * QX, vx);
+            stage::lane_store<KIND, QY>(ydst + (uint32_t)(k * QY * ly.di) * 16u,
+                                        (uint32_t)ly.di * 16u, p.y_bytes, my - k * QY, vy);
+          }
+          hu += kProducerWarps;
+          while (hu >= HU) { hu -= HU; ++hw; }
+        }
+      } else {
       auto xrow = [&](int r) {
         const int hu = r % HU, hw = r / HU;
         const int iw = ow * p.sw - p.pw + minw + hw * p.sw;
@@ -255,8 +326,10 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
                                         p.Co - ycb, p.vec_y, pidx, kProducerWarps, lane,
                                         yrow);
       }
+      }
       fence_proxy_async();
       mbar_arrive(smem_u32(&full[st]));
+      if (++st == p.NS) { st = 0; ph ^= 1; }
     }
     if (staged && warp >= kEpiWarp0) {
       // ===================== epilogue: TMEM -> partial dW =====================
@@ -406,17 +479,18 @@ int *status_word() {
   return p[dev];
 }
 
-template <int KIND>
+template <int KIND, bool LANES>
 int launch(const WgParams &p, size_t smem, int grid, cudaStream_t s) {
   static bool attr[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr[dev]) {
-    OWL_CUDA(cudaFuncSetAttribute(wgrad_tc_kernel<KIND>,
+    OWL_CUDA(cudaFuncSetAttribute(wgrad_tc_kernel<KIND, LANES>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
     attr[dev] = true;
   }
-  cudaError_t e = launch_pdl(wgrad_tc_kernel<KIND>, dim3(grid), dim3(kThreads), smem, s, p);
+  cudaError_t e = launch_pdl(wgrad_tc_kernel<KIND, LANES>, dim3(grid), dim3(kThreads), smem, s,
+                             p);
   if (e == cudaSuccess) e = cudaGetLastError();
   note_launch();
   note_tc_launch();
@@ -631,8 +705,11 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
       (size_t)p.NS * parts * (p.x_bytes + p.y_bytes) + (2 * p.NS + 2) * 8 + 16 + 4 * (size_t)p.TG;
   const int grid = (int)(units * p.R);
   int rc;
-  if (kind == K_BF16X3) rc = launch<K_BF16X3>(p, smem, grid, s);
-  else rc = launch<K_BF16>(p, smem, grid, s);
+  const bool lanes = p.vec_x == 2 && p.vec_y == 2;
+  if (kind == K_BF16X3)
+    rc = lanes ? launch<K_BF16X3, true>(p, smem, grid, s) : launch<K_BF16X3, false>(p, smem, grid, s);
+  else
+    rc = lanes ? launch<K_BF16, true>(p, smem, grid, s) : launch<K_BF16, false>(p, smem, grid, s);
   if (rc == kOk && p.R > 1) rc = sum_partials_f32(part, dw, welems, p.R, s);
   if (part) scratch_free(part, s);
   return rc;
