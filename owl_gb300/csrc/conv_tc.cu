@@ -104,8 +104,14 @@ struct TcParams {
   // column stride of the accumulators of a tile's co tiles and buffers).
   int TU, TN, TNA;
   int T;  // plan: taps of the longest segment
+  int n_table;  // taps of all segments
   int sw, su, sv;          // strides along w, u, v
   int HW, HU, HV, HVR, HP, PS;  // halo rows along w, u; pixels per u-row (= sv * HVR)
+  // Halo rows that some tap reads, for the row table: NHU u rows of the n_ures
+  // residues mod su in ures, n_vres residue rows mod sv in vres (a 1x1 kernel of
+  // stride 2 reads a quarter of its footprint); nrows in all.
+  int n_ures, n_vres, NHU, nrows;
+  unsigned char ures[8], vres[8];
   int n_tiles;
   int NCT, n_groups;  // output-channel tiles per CTA tile (1 or 2), and tile groups
   long long total_tiles;
@@ -174,15 +180,15 @@ __device__ __forceinline__ Tile decode_tile(const TcParams &p, long long t, int 
   Tile r;
   const Seg &sg = p.seg[c];
   r.c = c;
-  t -= sg.tile0;
-  r.nt = (int)(t % p.n_groups);  // co-tile group: tiles nt*NCT .. nt*NCT+NCT-1
-  t /= p.n_groups;
-  r.v0 = (int)(t % sg.v_tiles) * 8;
-  t /= sg.v_tiles;
-  r.u0 = (int)(t % sg.u_tiles) * p.TU;
-  t /= sg.u_tiles;
-  r.ow = (int)(t % sg.OW);
-  r.b = (int)(t / sg.OW);
+  unsigned q = (unsigned)(t - sg.tile0);  // (fewer than 2^31 tiles)
+  r.nt = (int)(q % (unsigned)p.n_groups);  // co-tile group: tiles nt*NCT .. nt*NCT+NCT-1
+  q /= (unsigned)p.n_groups;
+  r.v0 = (int)(q % (unsigned)sg.v_tiles) * 8;
+  q /= (unsigned)sg.v_tiles;
+  r.u0 = (int)(q % (unsigned)sg.u_tiles) * p.TU;
+  q /= (unsigned)sg.u_tiles;
+  r.ow = (int)(q % (unsigned)sg.OW);
+  r.b = (int)(q / (unsigned)sg.OW);
   return r;
 }
 
@@ -199,9 +205,52 @@ __device__ __forceinline__ uint32_t to_tf32(float a) {
   return r;
 }
 
+// One producer warp's staging of a channel block in whole 32-byte chunks: the
+// rows of the row table from `first` on, every kProducerWarps * ROWS, ROWS rows
+// of STEPS loads per lane a round (ROWS * STEPS <= 6 loads in flight).  What a
+// slot needs is constant for the lane or advances by an add.  `ready` waits for
+// the stage, after the first round's loads are issued.
+template <int KIND, int STEPS, int ROWS, class Ready>
+__device__ __forceinline__ bool stage_lanes(const TcParams &p, const int4 *rows, int first,
+                                            const stage::Lane &L, int steps, int n_lane,
+                                            const float *xt, int iw0, int iu0, int iv0,
+                                            uint8_t *dst, Ready ready) {
+  const long long pix = (long long)p.sv * p.xsv * p.Cin;  // floats between row pixels
+  bool waited = false;
+  for (int r0 = first * ROWS; r0 < p.nrows; r0 += kProducerWarps * ROWS) {
+    // (steps > STEPS only in the one-row form: a row in several rounds)
+    for (int k = 0; k < steps; k += STEPS) {
+      float v[ROWS][STEPS][8];
+#pragma unroll
+      for (int a = 0; a < ROWS; ++a) {
+        const int4 e = rows[min(r0 + a, p.nrows - 1)];
+        const int hw = e.z & 0xffff, hu = e.z >> 16;
+        const bool ok = r0 + a < p.nrows && (unsigned)(iw0 + hw) < (unsigned)p.IW &&
+                        (unsigned)(iu0 + hu) < (unsigned)p.IU && L.on;
+        stage::lane_load<STEPS>(xt + (long long)e.x * p.Cin + (long long)k * L.di * pix,
+                                L.di * pix, iv0 + e.w + (L.i0 + k * L.di) * p.sv, L.di * p.sv,
+                                ok ? (unsigned)p.IV : 0u, steps - k, v[a]);
+      }
+      if (!waited) {
+        if (!ready()) return false;
+        waited = true;
+      }
+#pragma unroll
+      for (int a = 0; a < ROWS; ++a) {
+        const int row = rows[min(r0 + a, p.nrows - 1)].y;
+        stage::lane_store<KIND, STEPS>(dst + (uint32_t)(row + k * L.di) * 16u,
+                                       (uint32_t)L.di * 16u, p.halo_bytes,
+                                       r0 + a < p.nrows ? n_lane - k : 0, v[a]);
+      }
+    }
+  }
+  return waited || ready();
+}
+
 // MULTI: the launch has several segments (else segment 0 only, read at a
-// constant offset of the parameters).
-template <int KIND, bool MULTI>
+// constant offset of the parameters).  LANES: the input is staged as whole
+// 32-byte chunks (32-byte aligned, channels a multiple of 8).
+template <int KIND, bool MULTI, bool LANES>
 __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_constant__ TcParams p) {
   if (p.wait_all) asm volatile("griddepcontrol.wait;" ::: "memory");
   constexpr int EPC = (KIND == K_TF32) ? 4 : 8;  // channels per 16-byte chunk
@@ -229,6 +278,19 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   uint32_t *tap_off = tmem_slot + 2;  // per-tap start pixel in the halo (16-byte units)
+  // LANES, the rows to stage: {pixel offset from the tile's first input pixel,
+  // first pixel in the stage, hw | hu << 16, hr}
+  int4 *rows = reinterpret_cast<int4 *>((reinterpret_cast<uintptr_t>(tap_off + p.n_table) + 15) &
+                                        ~(uintptr_t)15);
+  if (LANES) {
+    for (int i = threadIdx.x; i < p.nrows; i += blockDim.x) {
+      const int q = i / p.n_vres, hr = p.vres[i - q * p.n_vres];
+      const int hw = q / p.NHU, hi = q - hw * p.NHU;
+      const int uq = hi / p.n_ures, hu = uq * p.su + p.ures[hi - uq * p.n_ures];
+      rows[i] = make_int4((int)(hw * p.xsw + hu * p.xsu + hr * p.xsv),
+                          ((hw * p.HU + hu) * p.sv + hr) * p.HVR, hw | hu << 16, hr);
+    }
+  }
 
   // tap offsets of every segment, segment c's at tap_off[seg[c].toff ..]
   for (int c = 0; c < (MULTI ? p.nseg : 1); ++c) {
@@ -267,7 +329,53 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
   const uint32_t tmem_base = *tmem_slot;
 
   const int pidx = producer_index(warp);
-  if (pidx >= 0) {
+  if (LANES && pidx >= 0) {
+    // ===================== halo producers, whole chunks =====================
+    if constexpr (LANES) {
+      const stage::Lane L(p.NCH, lane);
+      const int steps = (p.HVR + L.di - 1) / L.di;
+      const int n_lane = L.on ? (p.HVR - L.i0 + L.di - 1) / L.di : 0;  // the lane's pixels
+      const uint32_t lane_off = (uint32_t)L.j * (uint32_t)p.PS * 16u + (uint32_t)L.i0 * 16u;
+      int hs = 0, sc = 0;
+      uint32_t hph = 1;
+      bool ok = true;
+      for (long long t = blockIdx.x; ok && t < p.total_tiles; t += gridDim.x) {
+        sc = MULTI ? seg_of(p, t, sc) : 0;
+        const Tile tl = decode_tile(p, t, sc);
+        const int iw0 = tl.ow * p.sw - p.seg[sc].pw, iu0 = tl.u0 * p.su - p.seg[sc].pu,
+                  iv0 = tl.v0 * p.sv - p.seg[sc].pv;
+        const float *xt = p.x + ((long long)tl.b * p.xsb + (long long)iw0 * p.xsw +
+                                 (long long)iu0 * p.xsu +
+                                 (long long)(iv0 + L.i0 * p.sv) * p.xsv) * p.Cin + L.j * EPC;
+        for (int cb = 0; cb < p.NCB; ++cb, xt += p.CPB) {
+          // chunks past the channels (a ragged last block) are zeros
+          stage::Lane Lb = L;
+          const bool real = (cb * p.CPB + L.j * EPC) < p.Cin;
+          auto ready = [&] {
+            return wait_bar(smem_u32(&halo_empty[hs]), hph, abort_flag, p.status, p.spin_limit);
+          };
+          Lb.on = L.on && real;
+          uint8_t *dst = halo + (size_t)hs * PARTS * p.halo_bytes + lane_off;
+          if (steps == 1)
+            ok = stage_lanes<KIND, 1, 6>(p, rows, pidx, Lb, steps, n_lane, xt, iw0, iu0, iv0, dst,
+                                         ready);
+          else if (steps == 2)
+            ok = stage_lanes<KIND, 2, 3>(p, rows, pidx, Lb, steps, n_lane, xt, iw0, iu0, iv0, dst,
+                                         ready);
+          else if (steps == 3)
+            ok = stage_lanes<KIND, 3, 2>(p, rows, pidx, Lb, steps, n_lane, xt, iw0, iu0, iv0, dst,
+                                         ready);
+          else
+            ok = stage_lanes<KIND, 6, 1>(p, rows, pidx, Lb, steps, n_lane, xt, iw0, iu0, iv0, dst,
+                                         ready);
+          if (!ok) break;
+          fence_proxy_async();
+          mbar_arrive(smem_u32(&halo_full[hs]));
+          if (++hs == p.NH) { hs = 0; hph ^= 1; }
+        }
+      }
+    }
+  } else if (!LANES && pidx >= 0) {
     // ===================== halo producers =====================
     // Each warp stages whole halo rows: a row is one (w, u, residue) line of
     // HVR pixels whose global addresses advance by a fixed step, so the row
@@ -972,10 +1080,14 @@ bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table) {
       q.HVR = 8 + ((v.KV - 1) * v.dv) / v.sv;
       q.HV = v.sv * q.HVR;
       q.HP = q.HW * q.HU * q.HV;
+      q.NHU = q.HU / v.su * q.n_ures;
+      for (int i = 0; i < q.n_ures; ++i) q.NHU += q.ures[i] < q.HU % v.su;
+      q.nrows = q.HW * q.NHU * q.n_vres;
       q.PS = q.HP + (((1 - q.HP) % 8) + 8) % 8;  // plane stride = 1 (mod 8) pixels
       if (q.PS >= 16384 || q.HV >= 16384) continue;
       q.halo_bytes = (unsigned)q.PS * 16u * (unsigned)q.NCH;
-      const long long fixed = (long long)q.NH * parts * q.halo_bytes + 512 + 4LL * t_table;
+      const long long fixed =
+          (long long)q.NH * parts * q.halo_bytes + 512 + 4LL * t_table + 16LL * q.nrows + 16;
       const long long room = kSmemMax - fixed;
       if (room <= 0) continue;
       // at least two weight slots
@@ -1073,13 +1185,13 @@ int drop_images(int dev, const void *w, bool all) {
   return kOk;
 }
 
-template <int KIND, bool MULTI>
+template <int KIND, bool MULTI, bool LANES>
 int launch(const TcParams &p, size_t smem, cudaStream_t s, bool after_prep) {
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    OWL_CUDA(cudaFuncSetAttribute(conv_tc_kernel<KIND, MULTI>,
+    OWL_CUDA(cudaFuncSetAttribute(conv_tc_kernel<KIND, MULTI, LANES>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
     attr_set[dev] = true;
   }
@@ -1099,7 +1211,7 @@ int launch(const TcParams &p, size_t smem, cudaStream_t s, bool after_prep) {
   // then every thread waits for the earlier work (wait_all)
   TcParams q = p;
   q.wait_all = after_prep ? 0 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, conv_tc_kernel<KIND, MULTI>, q);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, conv_tc_kernel<KIND, MULTI, LANES>, q);
   note_launch();
   note_tc_launch();
   if (e != cudaSuccess) return cuda_fail(e, "conv_tc_kernel");
@@ -1158,7 +1270,20 @@ int run_segs(int prec, int nseg_in, const SegSpec *sp, bool bwd_input, int Ci, i
   pv.KW = spw + 1; pv.KU = spu + 1; pv.KV = spv + 1;
   pv.dw = pv.du = pv.dv = 1;
   TcParams p{};
-  if (pv.Cin == 0 || !plan(p, pv, kind, t_slot, t_table)) return kErrUnsupported;
+  // the residues mod the stride that the taps read (several segments: stride 1)
+  {
+    const View &v = sp[idx[0]].v;
+    bool ru[8] = {false}, rv[8] = {false};
+    for (int t = 0; t < v.KU; ++t) ru[t * v.du % v.su] = true;
+    for (int t = 0; t < v.KV; ++t) rv[t * v.dv % v.sv] = true;
+    for (int r = 0; r < v.su; ++r)
+      if (ru[r]) p.ures[p.n_ures++] = (unsigned char)r;
+    for (int r = 0; r < v.sv; ++r)
+      if (rv[r]) p.vres[p.n_vres++] = (unsigned char)r;
+  }
+  if (pv.Cin == 0 || p.n_ures == 0 || p.n_vres == 0 || !plan(p, pv, kind, t_slot, t_table))
+    return kErrUnsupported;
+  p.n_table = t_table;
   p.x = x; p.y = y;
   p.B = pv.B; p.IW = pv.IW; p.IU = pv.IU; p.IV = pv.IV;
   p.sw = pv.sw; p.su = pv.su; p.sv = pv.sv;
@@ -1193,6 +1318,7 @@ int run_segs(int prec, int nseg_in, const SegSpec *sp, bool bwd_input, int Ci, i
     toff += g.T;
     woff += (size_t)p.n_tiles * p.NCB * g.T * p.tile_bytes;
   }
+  if (tiles >= (1LL << 31)) return kErrUnsupported;
   p.total_tiles = tiles;
   p.idesc = instr_desc(kind == K_TF32 ? 2u : 1u, (uint32_t)p.TN);
   // 1: 16-byte vector loads; 2: 32-byte aligned chunks (one load per chunk)
@@ -1308,14 +1434,25 @@ int run_segs(int prec, int nseg_in, const SegSpec *sp, bool bwd_input, int Ci, i
     }
   }
   const size_t smem = (size_t)p.NH * parts * p.halo_bytes + (size_t)p.NB * parts * p.b_bytes +
-                      (2 * p.NH + 2 * p.NB + 5) * 8 + 16 + 4 * (size_t)t_table;
+                      (2 * p.NH + 2 * p.NB + 5) * 8 + 16 + 4 * (size_t)t_table + 16 +
+                      16 * (size_t)p.nrows;
   const bool multi = p.nseg > 1;
   const bool pdl = prep && !build_cached;
+  // (the row table's pixel offsets are 32-bit)
+  const bool lanes = p.vec_in == 2 && p.HW * p.xsw + p.HU * p.xsu + p.HV * p.xsv < (1LL << 31);
   if (kind == K_TF32)
-    rc = multi ? launch<K_TF32, true>(p, smem, s, pdl) : launch<K_TF32, false>(p, smem, s, pdl);
+    rc = multi ? launch<K_TF32, true, false>(p, smem, s, pdl)
+               : launch<K_TF32, false, false>(p, smem, s, pdl);
   else if (kind == K_BF16X3)
-    rc = multi ? launch<K_BF16X3, true>(p, smem, s, pdl) : launch<K_BF16X3, false>(p, smem, s, pdl);
-  else rc = multi ? launch<K_BF16, true>(p, smem, s, pdl) : launch<K_BF16, false>(p, smem, s, pdl);
+    rc = lanes ? (multi ? launch<K_BF16X3, true, true>(p, smem, s, pdl)
+                        : launch<K_BF16X3, false, true>(p, smem, s, pdl))
+               : (multi ? launch<K_BF16X3, true, false>(p, smem, s, pdl)
+                        : launch<K_BF16X3, false, false>(p, smem, s, pdl));
+  else
+    rc = lanes ? (multi ? launch<K_BF16, true, true>(p, smem, s, pdl)
+                        : launch<K_BF16, false, true>(p, smem, s, pdl))
+               : (multi ? launch<K_BF16, true, false>(p, smem, s, pdl)
+                        : launch<K_BF16, false, false>(p, smem, s, pdl));
   if (!cached) scratch_free(wt, s);
   return rc;
 }
