@@ -102,6 +102,22 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
   }
 }
 
+// The MMA warp's: polled by the whole warp.
+__device__ __forceinline__ bool poll_bar(uint32_t bar, uint32_t parity, volatile int *abort_flag,
+                                         int *status, long long limit) {
+  if (mbar_test_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!mbar_test_wait(bar, parity)) {
+    if (*abort_flag) return false;
+    if (clock64() - t0 > limit) {
+      *abort_flag = 1;
+      atomicExch(status, 1);
+      return false;
+    }
+  }
+  return true;
+}
+
 // LANES: the operands are staged as whole 32-byte chunks (both arrays 32-byte
 // aligned, their channels multiples of 8), else element by element where needed.
 template <int KIND, bool LANES>
@@ -375,7 +391,8 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
     }
   } else {
     // ===================== MMA issuer =====================
-    if (lane == 0) {
+    {
+      const uint32_t lead = elect_one();
       const uint32_t x0 = smem_u32(xs), y0 = smem_u32(ys);
       const uint32_t a_lbo = (uint32_t)HVR * 16, a_sbo = (uint32_t)p.PS * 16;
       const uint32_t b_lbo = 128, b_sbo = (uint32_t)p.YPS * 16;
@@ -397,7 +414,7 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
       uint32_t acc = 0;
       bool ok = true;
       for (long long t = t_begin; t < t_end; ++t) {
-        if (!wait_bar(smem_u32(&full[st]), ph, abort_flag, p.status, p.spin_limit)) {
+        if (!poll_bar(smem_u32(&full[st]), ph, abort_flag, p.status, p.spin_limit)) {
           ok = false;
           break;
         }
@@ -405,6 +422,7 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
         // descriptors advance by adds of 16-byte units (start-address field)
         const uint64_t xd_st = smem_desc(x0 + (uint32_t)st * PARTS * p.x_bytes, a_lbo, a_sbo);
         const uint64_t yd_st = smem_desc(y0 + (uint32_t)st * PARTS * p.y_bytes, b_lbo, b_sbo);
+#pragma unroll 2
         for (int s = 0; s < nks; ++s) {
           const uint64_t bd = yd_st + (uint64_t)(s * KSTEP_PIX);
           const uint64_t xs_ = xd_st + (uint64_t)(s * xk16);
@@ -414,12 +432,12 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
               if (i < ntap) {
                 const uint64_t ad = xs_ + (uint64_t)to[i];
                 if (KIND == K_TF32) {
-                  mma_tf32(dc[i], ad, bd, p.idesc, acc);
+                  mma_tf32(lead, dc[i], ad, bd, p.idesc, acc);
                 } else {
-                  mma_bf16(dc[i], ad, bd, p.idesc, acc);
+                  mma_bf16(lead, dc[i], ad, bd, p.idesc, acc);
                   if (KIND == K_BF16X3) {
-                    mma_bf16(dc[i] + p.small_off, ad, bd + (uint64_t)ylo16, p.idesc, acc);
-                    mma_bf16(dc[i] + p.small_off, ad + (uint64_t)xlo16, bd, p.idesc, 1);
+                    mma_bf16(lead, dc[i] + p.small_off, ad, bd + (uint64_t)ylo16, p.idesc, acc);
+                    mma_bf16(lead, dc[i] + p.small_off, ad + (uint64_t)xlo16, bd, p.idesc, 1);
                   }
                 }
               }
@@ -429,23 +447,23 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
               const uint64_t ad = xs_ + (uint64_t)tap_off[i];
               const uint32_t d = tmem_base + (uint32_t)(i * p.BN);
               if (KIND == K_TF32) {
-                mma_tf32(d, ad, bd, p.idesc, acc);
+                mma_tf32(lead, d, ad, bd, p.idesc, acc);
               } else {
-                mma_bf16(d, ad, bd, p.idesc, acc);
+                mma_bf16(lead, d, ad, bd, p.idesc, acc);
                 if (KIND == K_BF16X3) {
-                  mma_bf16(d + p.small_off, ad, bd + (uint64_t)ylo16, p.idesc, acc);
-                  mma_bf16(d + p.small_off, ad + (uint64_t)xlo16, bd, p.idesc, 1);
+                  mma_bf16(lead, d + p.small_off, ad, bd + (uint64_t)ylo16, p.idesc, acc);
+                  mma_bf16(lead, d + p.small_off, ad + (uint64_t)xlo16, bd, p.idesc, 1);
                 }
               }
             }
           }
           acc = 1;
         }
-        mma_commit(smem_u32(&empty[st]));
+        mma_commit(lead, smem_u32(&empty[st]));
         if (++st == p.NS) { st = 0; ph ^= 1; }
       }
-      if (ok) mma_commit(smem_u32(acc_full));
-      mma_commit(smem_u32(drain));
+      if (ok) mma_commit(lead, smem_u32(acc_full));
+      mma_commit(lead, smem_u32(drain));
       long long t0 = clock64();
       while (!mbar_try_wait(smem_u32(drain), 0) && clock64() - t0 < kSpinLimit) {
       }

@@ -107,6 +107,22 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
   }
 }
 
+// The MMA warp's: polled by the whole warp.
+__device__ __forceinline__ bool poll_bar(uint32_t bar, uint32_t parity, volatile int *abort_flag,
+                                         int *status, long long limit) {
+  if (mbar_test_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!mbar_test_wait(bar, parity)) {
+    if (*abort_flag) return false;
+    if (clock64() - t0 > limit) {
+      *abort_flag = 1;
+      atomicExch(status, 1);
+      return false;
+    }
+  }
+  return true;
+}
+
 __device__ __forceinline__ float apply_act(float v, int act) {
   return act == OWLGPU_ACT_RELU ? (v > 0.f ? v : 0.f) : v;
 }
@@ -417,8 +433,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         tc_fence_before();
       }
     }
-  } else if (lane == 0) {
+  } else {
     // ===================== MMA issuer =====================
+    const uint32_t lead = elect_one();
     const uint32_t s0 = smem_u32(smem);
     // K-major: core matrices along k are (R+1)*16 bytes apart, along rows
     // 128; MN-major: along k 128 bytes apart, along rows (kBK+1)*16.  One
@@ -435,7 +452,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     bool ok = true;
     for (int i = 0; i < nkb; ++i) {
       const int st = i % p.NS;
-      if (!wait_bar(smem_u32(&full[st]), (uint32_t)((i / p.NS) & 1), abort_flag, p.status,
+      if (!poll_bar(smem_u32(&full[st]), (uint32_t)((i / p.NS) & 1), abort_flag, p.status,
                     p.spin_limit)) {
         ok = false;
         break;
@@ -446,17 +463,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
 #pragma unroll
       for (int s = 0; s < kBK / 16; ++s) {
         const uint64_t ad = ad0 + (uint64_t)(s * a_step), bd = bd0 + (uint64_t)(s * b_step);
-        mma_bf16(d, ad, bd, p.idesc, acc);
+        mma_bf16(lead, d, ad, bd, p.idesc, acc);
         if (SEP) {
-          mma_bf16(ds, ad + (uint64_t)alo, bd, p.idesc, acc);
-          mma_bf16(ds, ad, bd + (uint64_t)blo, p.idesc, 1);
+          mma_bf16(lead, ds, ad + (uint64_t)alo, bd, p.idesc, acc);
+          mma_bf16(lead, ds, ad, bd + (uint64_t)blo, p.idesc, 1);
         }
         acc = 1;
       }
-      mma_commit(smem_u32(&empty[st]));
+      mma_commit(lead, smem_u32(&empty[st]));
     }
-    if (ok) mma_commit(smem_u32(acc_full));
-    mma_commit(smem_u32(drain));
+    if (ok) mma_commit(lead, smem_u32(acc_full));
+    mma_commit(lead, smem_u32(drain));
     long long t0 = clock64();
     while (!mbar_try_wait(smem_u32(drain), 0) && clock64() - t0 < kSpinLimit) {
     }
