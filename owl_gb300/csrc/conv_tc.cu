@@ -74,6 +74,7 @@ __device__ __forceinline__ int producer_index(int warp) {
   return (warp & 3) != 0 && warp < 12 ? (warp >> 2) * 3 + (warp & 3) - 1 : -1;
 }
 constexpr int kSmemMax = 232448;  // 227 KB opt-in dynamic shared memory
+constexpr int kSmemLean = 195 * 1024;  // the carve-out step below it, less the block's 1 KB
 constexpr long long kSpinLimit = 4000000000LL;  // cycles (~2 s) before a wait gives up
 
 enum Kind { K_BF16 = 0, K_TF32 = 1, K_BF16X3 = 2 };
@@ -1054,96 +1055,177 @@ int *status_ptr() {
   return p[dev];
 }
 
+// Output extents and taps of a launch segment, as the plan needs them.
+struct PlanSeg {
+  int OW, OU, OV, T;
+};
+
+// What a plan's time is made of, in us (measured on GB300; the choice needs
+// their ratios only): an MMA with one and with two accumulators in turn, and per
+// column of N; a round of the producers' loads; weight bytes and output bytes
+// per us and SM; the hand-off of a weight slot.
+constexpr double kMma1 = 0.056, kMma2 = 0.0485, kMmaCol = 0.00027;
+constexpr double kRound = 1.15, kWeightRate = 100e3, kStoreRate = 45e3, kSlot = 0.2;
+
 // Choose tile and pipeline sizes; false if no configuration fits.
-// Priorities: the fewest halo stagings, tiles along u times co-tile groups
-// (an MMA costs the same whatever its N, so a tile's MMA count does not
-// depend on its height, and a tile of up to 128 pixels stages its halo once
-// for two co tiles); then the widest
-// channel block (fewer, fuller halo stages for the producers: a whole
-// 128-channel pixel per stage when two stages fit); then the most taps per
-// weight slot (fewer barrier polls between MMAs); then the lowest tile (the
-// least halo).  Tile heights are even (N = 8*TU a multiple of 16) up to 32.
+//
+// The channel block CB sets the order of the sums, so it comes from the layer
+// alone (an entry's result does not depend on what else is in its batch): all
+// channels, up to 224 bytes a pixel, else blocks of 128, 64 or 32 bytes, the
+// least padded (a padded 32 bytes costs a full MMA per tap), then the widest.
+// Two stages of 128 bytes overlap where one of 256 is waited for:
+// [64;56;56;128]x[3;3;128;128] took 61.5 us with 256, 57.8 with 128.
+//
+// The tile, TU positions by 8 and one or two co tiles (staged once, their MMAs
+// alternating accumulators), has the least estimated time for this batch: a CTA
+// works through ceil(tiles / SMs) tiles, each as slow as the slowest of its
+// MMAs, its producers, its weight stream and its stores, and overlaps neither
+// its first stage nor its last stores.  An MMA costs little less for a small N,
+// so layers with many tiles take tall ones (the least halo and the fewest MMAs),
+// and those with few take low ones that fill the SMs: [16;28;28;128] to 256
+// channels at stride 2 took 25 us with the tallest tile and two co tiles (32
+// CTAs), 14.5 with TU = 8 and one (128 CTAs).  TU is even (N = 8*TU a multiple
+// of 16) and at most 32.
 // `v` holds the largest halo extents of the launch's segments; t_slot is the
 // most taps of one segment (weight slots), t_table the taps of all segments
 // (the shared-memory tap table).
-bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table) {
+bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const PlanSeg *segs,
+          int nseg) {
   const int EB = (kind == K_TF32) ? 4 : 2;
   const int parts = (kind == K_BF16X3) ? 2 : 1;
+  const int sms = num_sms();
   p.BN = 128;  // output channels per tile = the MMA's M
   p.n_tiles = (v.Cout + p.BN - 1) / p.BN;
   p.T = t_slot;
-  const int cb0 = std::min(256, (int)((v.Cin * EB + 31) / 32 * 32));
-  bool found = false;
-  TcParams best = p;
-  long long best_score = 0;
-  // two halo stages (staging overlaps the MMAs); one only when two do not
-  // fit shared memory (wide strided halos in split-BF16)
-  for (int nh = 2; nh >= 1 && !found; --nh)
-  for (int tu = 32; tu >= 2; tu -= 2) {
-    const long long u_tiles = (v.OU + tu - 1) / tu;
-    for (int cb = cb0; cb >= 32; cb -= 32) {
-      // cb0 (all channels, up to 256 bytes), then 128, 64, 32: blocks that
-      // divide the channels evenly (a ragged last block costs full MMAs)
-      if (cb != cb0 && cb != 128 && cb != 64 && cb != 32) continue;
-      TcParams q = p;
-      q.NH = nh;
-      q.TU = tu;
-      q.TN = 8 * tu;
-      q.TNA = (q.TN + 31) / 32 * 32;
-      // tiles of up to 128 pixels take two co tiles when there are two: the
-      // halo is staged once for both and their MMAs alternate accumulators
-      q.NCT = (q.TN <= 128 && p.n_tiles >= 2) ? 2 : 1;
-      q.n_groups = (p.n_tiles + q.NCT - 1) / q.NCT;
-      q.CB = cb;
-      q.CPB = q.CB / EB;
-      q.NCH = q.CB / 16;
-      q.NCB = (v.Cin + q.CPB - 1) / q.CPB;
-      q.tile_bytes = (unsigned)(q.BN * q.CB);
-      q.HW = (v.KW - 1) * v.dw + 1;
-      q.HU = (tu - 1) * v.su + (v.KU - 1) * v.du + 1;
-      q.HVR = 8 + ((v.KV - 1) * v.dv) / v.sv;
-      q.HV = v.sv * q.HVR;
-      q.HP = q.HW * q.HU * q.HV;
-      q.NHU = q.HU / v.su * q.n_ures;
-      for (int i = 0; i < q.n_ures; ++i) q.NHU += q.ures[i] < q.HU % v.su;
-      q.nrows = q.HW * q.NHU * q.n_vres;
-      q.PS = q.HP + (((1 - q.HP) % 8) + 8) % 8;  // plane stride = 1 (mod 8) pixels
-      if (q.PS >= 16384 || q.HV >= 16384) continue;
-      q.halo_bytes = (unsigned)q.PS * 16u * (unsigned)q.NCH;
-      const long long fixed =
-          (long long)q.NH * parts * q.halo_bytes + 512 + 4LL * t_table + 16LL * q.nrows + 16;
-      const long long room = kSmemMax - fixed;
-      if (room <= 0) continue;
-      // at least two weight slots
-      const long long tps =
-          std::min<long long>(q.T, room / (2LL * parts * q.NCT * q.tile_bytes));
-      if (tps < 1) continue;
-      q.TPS = (int)tps;
-      q.NSL = (q.T + q.TPS - 1) / q.TPS;
-      q.TPS = (q.T + q.NSL - 1) / q.NSL;  // balance the slots
-      q.b_bytes = (unsigned)(q.NCT * q.TPS) * q.tile_bytes;
-      q.NB = (int)std::min<long long>(4, room / ((long long)parts * q.b_bytes));
-      if (q.NB < 2) continue;
-      // accumulator sets: double-buffered when they fit TMEM (the epilogue
-      // of one tile overlaps the next tile's MMAs), else one set
-      q.small_off = (unsigned)(q.NCT * q.TNA);
-      q.acc_cols = q.small_off * (unsigned)parts;
-      q.nbuf = q.acc_cols * 2 <= 512 ? 2 : 1;
-      if (q.acc_cols > 512) continue;
-      q.tmem_cols = 32;
-      while (q.tmem_cols < q.acc_cols * (unsigned)q.nbuf) q.tmem_cols <<= 1;
-      // halo stagings per output: tiles along u times co-tile groups
-      const long long stagings = u_tiles * q.n_groups;
-      const long long score = -stagings * 1000000000000LL + (long long)q.CB * 1000000LL +
-                              (long long)q.TPS * (q.NCH / 2) * 1000LL - tu;
-      if (!found || score > best_score) {
-        best_score = score;
-        best = q;
-        found = true;
+  int max_ou = 2;
+  for (int c = 0; c < nseg; ++c) max_ou = std::max(max_ou, (segs[c].OU + 1) / 2 * 2);
+  const int max_tu = std::min(32, max_ou);
+
+  // q: the sizes of one configuration; false when it does not fit
+  auto fit = [&](TcParams &q, int nh, int tu, int cb, int nct) {
+    q = p;
+    q.NH = nh;
+    q.TU = tu;
+    q.TN = 8 * tu;
+    q.TNA = (q.TN + 31) / 32 * 32;
+    q.NCT = nct;
+    q.n_groups = (p.n_tiles + q.NCT - 1) / q.NCT;
+    q.CB = cb;
+    q.CPB = q.CB / EB;
+    q.NCH = q.CB / 16;
+    q.NCB = (v.Cin + q.CPB - 1) / q.CPB;
+    q.tile_bytes = (unsigned)(q.BN * q.CB);
+    q.HW = (v.KW - 1) * v.dw + 1;
+    q.HU = (tu - 1) * v.su + (v.KU - 1) * v.du + 1;
+    q.HVR = 8 + ((v.KV - 1) * v.dv) / v.sv;
+    q.HV = v.sv * q.HVR;
+    q.HP = q.HW * q.HU * q.HV;
+    q.NHU = q.HU / v.su * q.n_ures;
+    for (int i = 0; i < q.n_ures; ++i) q.NHU += q.ures[i] < q.HU % v.su;
+    q.nrows = q.HW * q.NHU * q.n_vres;
+    q.PS = q.HP + (((1 - q.HP) % 8) + 8) % 8;  // plane stride = 1 (mod 8) pixels
+    if (q.PS >= 16384 || q.HV >= 16384) return false;
+    q.halo_bytes = (unsigned)q.PS * 16u * (unsigned)q.NCH;
+    const long long fixed =
+        (long long)q.NH * parts * q.halo_bytes + 512 + 4LL * t_table + 16LL * q.nrows + 16;
+    // Shared memory up to the step that leaves 60 KB of the SM's 256 for the L1
+    // cache where three taps per weight slot fit in that: the producers' loads in
+    // flight (up to 55 KB) wait for lines of a smaller one (57.3 us against 53.2
+    // for [64;56;56;128]x[3;3;128;128]).
+    const long long slot = (long long)parts * q.NCT * q.tile_bytes;
+    long long room = kSmemLean - fixed;
+    if (room < 2 * slot * std::min(3, q.T)) room = kSmemMax - fixed;
+    if (room <= 0) return false;
+    // the most taps per weight slot (fewer barrier polls between MMAs) that
+    // leaves at least two slots
+    const long long tps = std::min<long long>(q.T, room / (2 * slot));
+    if (tps < 1) return false;
+    q.TPS = (int)tps;
+    q.NSL = (q.T + q.TPS - 1) / q.TPS;
+    q.TPS = (q.T + q.NSL - 1) / q.NSL;  // balance the slots
+    q.b_bytes = (unsigned)(q.NCT * q.TPS) * q.tile_bytes;
+    q.NB = (int)std::min<long long>(4, room / ((long long)parts * q.b_bytes));
+    if (q.NB < 2) return false;
+    // accumulator sets: double-buffered when they fit TMEM (the epilogue
+    // of one tile overlaps the next tile's MMAs), else one set
+    q.small_off = (unsigned)(q.NCT * q.TNA);
+    q.acc_cols = q.small_off * (unsigned)parts;
+    q.nbuf = q.acc_cols * 2 <= 512 ? 2 : 1;
+    if (q.acc_cols > 512) return false;
+    q.tmem_cols = 32;
+    while (q.tmem_cols < q.acc_cols * (unsigned)q.nbuf) q.tmem_cols <<= 1;
+    return true;
+  };
+  // estimated time of a configuration (the start that all share left out)
+  auto estimate = [&](const TcParams &q) {
+    long long tiles = 0, taps_sum = 0;
+    for (int c = 0; c < nseg; ++c) {
+      const long long n = (long long)segs[c].OW * ((segs[c].OU + q.TU - 1) / q.TU) *
+                          ((segs[c].OV + 7) / 8);
+      tiles += n;
+      taps_sum += n * segs[c].T;
+    }
+    const double taps = (double)taps_sum / (double)std::max(tiles, 1LL);  // a tile's, on average
+    tiles *= (long long)v.B * q.n_groups;
+    const double rounds = (double)((tiles + sms - 1) / sms);
+    const double mmas = taps * q.NCB * (q.NCH / 2) * q.NCT * (parts == 2 ? 3 : 1);
+    const double mma = mmas * std::max(q.NCT * parts == 1 ? kMma1 : kMma2, kMmaCol * q.TN) +
+                       q.NCB * std::max(1.0, taps / q.TPS) * kSlot;
+    // a row of the halo in 32-lane loads, six loads a lane and round
+    int chunks = 1;
+    while (chunks < q.NCH) chunks *= 2;
+    const int steps = (q.HVR * chunks + 31) / 32;
+    const int per_round = kProducerWarps * std::max(1, 6 / steps);
+    const double stage = kRound * ((q.nrows + per_round - 1) / per_round) * ((steps + 5) / 6) *
+                         (parts == 2 ? 1.3 : 1.0);
+    const double weights = taps * q.NCB * q.tile_bytes * (parts * q.NCT) / kWeightRate;
+    const double store = (double)q.TN * std::min(v.Cout, q.BN * q.NCT) * 4 / kStoreRate;
+    const double fill = q.NCB * stage;
+    const double work = std::max(weights, q.NH >= 2 ? std::max(mma, fill) : mma + fill);
+    return q.nbuf == 2 ? stage + rounds * std::max(work, store) + store
+                       : stage + rounds * (work + store);
+  };
+
+  // channel blocks, the least padded first (a block's own cost counts as half a
+  // step of 32 bytes)
+  const int all = (int)std::min<long long>(256, ((long long)v.Cin * EB + 31) / 32 * 32);
+  int cbs[4], ncb = 0;
+  if (all <= 224) cbs[ncb++] = all;
+  for (int cb = 128; cb >= 32; cb /= 2)
+    if (cb < all) cbs[ncb++] = cb;
+  auto padded = [&](int cb) {
+    const long long n = ((long long)v.Cin * EB + cb - 1) / cb;
+    return n * (cb + 16);
+  };
+  std::stable_sort(cbs, cbs + ncb, [&](int a, int b) { return padded(a) < padded(b); });
+  // the first of them that fits with two halo stages (staging overlaps the MMAs)
+  // and the tallest tile, 32-byte ones with one half as tall: a tall tile's fewer
+  // MMAs outweigh a wide block ([64;56;56;128]x[3;3;128;128] at rate 2 in split
+  // BF16 takes 155 us with 128 bytes and TU <= 20, 122 with 64 and TU = 28).
+  // Else the first that fits with the lowest tile, then with one stage.
+  TcParams q;
+  int nh = 0, cb = 0;
+  for (int form = 0; form < 4 && !cb; ++form)
+    for (int i = 0; i < ncb && !cb; ++i) {
+      const int tall = form == 0 ? max_tu : (form == 1 ? std::min(16, max_tu) : 2);
+      if (form == 0 && cbs[i] == 32 && all > 32) continue;
+      if (fit(q, form < 3 ? 2 : 1, tall, cbs[i], 1)) {
+        nh = form < 3 ? 2 : 1;
+        cb = cbs[i];
       }
     }
-  }
-  if (!found) return false;
+  if (!cb) return false;
+  double least = -1;
+  TcParams best = p;
+  for (int tu = max_tu; tu >= 2; tu -= 2)
+    for (int nct = std::min(2, p.n_tiles); nct >= 1; --nct) {
+      if (!fit(q, nh, tu, cb, nct)) continue;
+      const double t = estimate(q);
+      if (least < 0 || t < least) {
+        least = t;
+        best = q;
+      }
+    }
   p = best;
   return true;
 }
@@ -1305,7 +1387,13 @@ int run_segs(int prec, int nseg_in, const SegSpec *sp, bool bwd_input, int Ci, i
     for (int r = 0; r < v.sv; ++r)
       if (rv[r]) p.vres[p.n_vres++] = (unsigned char)r;
   }
-  if (pv.Cin == 0 || p.n_ures == 0 || p.n_vres == 0 || !plan(p, pv, kind, t_slot, t_table))
+  PlanSeg psegs[kMaxSeg];
+  for (int k = 0; k < nseg; ++k) {
+    const View &v = sp[idx[k]].v;
+    psegs[k] = {v.OW, v.OU, v.OV, v.KW * v.KU * v.KV};
+  }
+  if (pv.Cin == 0 || p.n_ures == 0 || p.n_vres == 0 ||
+      !plan(p, pv, kind, t_slot, t_table, psegs, nseg))
     return kErrUnsupported;
   p.n_table = t_table;
   p.x = x; p.y = y;
