@@ -68,7 +68,6 @@ constexpr int kMmaWarp = 0;
 constexpr int kLoadWarp = 4;
 constexpr int kEpiWarp0 = 12;
 constexpr int kProducerWarps = 9;
-constexpr int kProducerThreads = kProducerWarps * 32;
 // producer index of a warp (warps 1-3, 5-7, 9-11), or -1
 __device__ __forceinline__ int producer_index(int warp) {
   return (warp & 3) != 0 && warp < 12 ? (warp >> 2) * 3 + (warp & 3) - 1 : -1;
@@ -168,6 +167,13 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
   }
 }
 
+// A producer warp's: the same answer for all its lanes (they arrive together).
+__device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity,
+                                              volatile int *abort_flag, int *status,
+                                              long long limit) {
+  return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag, status, limit));
+}
+
 // The MMA warp's: polled by the whole warp.
 __device__ __forceinline__ bool poll_bar(uint32_t bar, uint32_t parity, volatile int *abort_flag,
                                          int *status, long long limit) {
@@ -211,18 +217,9 @@ __device__ __forceinline__ Tile decode_tile(const TcParams &p, long long t, int 
   return r;
 }
 
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t *>(&h);
-}
-__device__ __forceinline__ float bf16_round(float a) {
-  return __bfloat162float(__float2bfloat16_rn(a));
-}
-__device__ __forceinline__ uint32_t to_tf32(float a) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(a));
-  return r;
-}
+using stage::pack_bf16;
+using stage::pack_rest;
+using stage::to_tf32;
 
 // One producer warp's staging of a channel block in whole 32-byte chunks: the
 // rows of the row table from `first` on, every kProducerWarps * ROWS, ROWS rows
@@ -323,7 +320,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
   }
   if (threadIdx.x == 0) {
     for (int i = 0; i < p.NH; ++i) {
-      mbar_init(smem_u32(&halo_full[i]), kProducerThreads);
+      mbar_init(smem_u32(&halo_full[i]), kProducerWarps);
       mbar_init(smem_u32(&halo_empty[i]), 1);
     }
     for (int i = 0; i < p.NB; ++i) {
@@ -371,7 +368,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
           stage::Lane Lb = L;
           const bool real = (cb * p.CPB + L.j * EPC) < p.Cin;
           auto ready = [&] {
-            return wait_bar(smem_u32(&halo_empty[hs]), hph, abort_flag, p.status, p.spin_limit);
+            return wait_bar_warp(smem_u32(&halo_empty[hs]), hph, abort_flag, p.status, p.spin_limit);
           };
           Lb.on = L.on && real;
           uint8_t *dst = halo + (size_t)hs * PARTS * p.halo_bytes + lane_off;
@@ -389,7 +386,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
                                          ready);
           if (!ok) break;
           fence_proxy_async();
-          mbar_arrive(smem_u32(&halo_full[hs]));
+          mbar_arrive_warp(smem_u32(&halo_full[hs]), lane);
           if (++hs == p.NH) { hs = 0; hph ^= 1; }
         }
       }
@@ -416,7 +413,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
       for (int cb = 0; cb < p.NCB; ++cb, ++k) {
         const int hs = (int)(k % p.NH);
         const uint32_t ph = (uint32_t)((k / p.NH) & 1);
-        if (!wait_bar(smem_u32(&halo_empty[hs]), ph ^ 1, abort_flag, p.status, p.spin_limit)) goto done;
+        if (!wait_bar_warp(smem_u32(&halo_empty[hs]), ph ^ 1, abort_flag, p.status, p.spin_limit)) goto done;
         uint8_t *dst = halo + (size_t)hs * PARTS * p.halo_bytes;
         const int cbase = cb * p.CPB;
         for (int r0 = pidx * rpp; r0 < nrows; r0 += rpp * kProducerWarps) {
@@ -482,12 +479,9 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
             }
             *reinterpret_cast<uint4 *>(dst + off[q]) = hi;
             if (KIND == K_BF16X3) {
-              float rs[8];
-#pragma unroll
-              for (int e = 0; e < 8; ++e) rs[e] = v[q][e] - bf16_round(v[q][e]);
-              uint4 lo = make_uint4(pack_bf16(rs[0], rs[1]), pack_bf16(rs[2], rs[3]),
-                                    pack_bf16(rs[4], rs[5]), pack_bf16(rs[6], rs[7]));
-              *reinterpret_cast<uint4 *>(dst + p.halo_bytes + off[q]) = lo;
+              *reinterpret_cast<uint4 *>(dst + p.halo_bytes + off[q]) =
+                  make_uint4(pack_rest(hi.x, v[q][0], v[q][1]), pack_rest(hi.y, v[q][2], v[q][3]),
+                             pack_rest(hi.z, v[q][4], v[q][5]), pack_rest(hi.w, v[q][6], v[q][7]));
             }
           }
           // rows wider than 32*kSlots chunk slots (one row per pass then):
@@ -524,18 +518,15 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
               }
               *reinterpret_cast<uint4 *>(dst + o) = hi;
               if (KIND == K_BF16X3) {
-                float rs[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) rs[e] = w8[e] - bf16_round(w8[e]);
                 *reinterpret_cast<uint4 *>(dst + p.halo_bytes + o) =
-                    make_uint4(pack_bf16(rs[0], rs[1]), pack_bf16(rs[2], rs[3]),
-                               pack_bf16(rs[4], rs[5]), pack_bf16(rs[6], rs[7]));
+                    make_uint4(pack_rest(hi.x, w8[0], w8[1]), pack_rest(hi.y, w8[2], w8[3]),
+                               pack_rest(hi.z, w8[4], w8[5]), pack_rest(hi.w, w8[6], w8[7]));
               }
             }
           }
         }
         fence_proxy_async();
-        mbar_arrive(smem_u32(&halo_full[hs]));
+        mbar_arrive_warp(smem_u32(&halo_full[hs]), lane);
       }
     }
   } else if (warp == kMmaWarp) {
@@ -891,13 +882,9 @@ __global__ void prep_weights(const float *__restrict__ w, uint8_t *__restrict__ 
     } else {
       h4 = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]),
                       pack_bf16(v[6], v[7]));
-      if (KIND == K_BF16X3) {
-        float rr[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) rr[e] = v[e] - bf16_round(v[e]);
-        l4 = make_uint4(pack_bf16(rr[0], rr[1]), pack_bf16(rr[2], rr[3]), pack_bf16(rr[4], rr[5]),
-                        pack_bf16(rr[6], rr[7]));
-      }
+      if (KIND == K_BF16X3)
+        l4 = make_uint4(pack_rest(h4.x, v[0], v[1]), pack_rest(h4.y, v[2], v[3]),
+                        pack_rest(h4.z, v[4], v[5]), pack_rest(h4.w, v[6], v[7]));
     }
     // byte offset of (nt, cb, tap) tile, then chunk j, row n
     const long long tile = ((long long)nt * NCB + cb) * T + tap;
@@ -964,17 +951,13 @@ __global__ void prep_weights_v4(const float *__restrict__ w, uint8_t *__restrict
     const long long off = tile * (long long)NCH * BN * 16 + ((long long)j * BN + n0) * 16;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      *reinterpret_cast<uint4 *>(hi + off + q * 16) =
-          make_uint4(pack_bf16(v[q][0], v[q][1]), pack_bf16(v[q][2], v[q][3]),
-                     pack_bf16(v[q][4], v[q][5]), pack_bf16(v[q][6], v[q][7]));
-      if (KIND == K_BF16X3) {
-        float rr[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) rr[e] = v[q][e] - bf16_round(v[q][e]);
+      const uint4 h4 = make_uint4(pack_bf16(v[q][0], v[q][1]), pack_bf16(v[q][2], v[q][3]),
+                                  pack_bf16(v[q][4], v[q][5]), pack_bf16(v[q][6], v[q][7]));
+      *reinterpret_cast<uint4 *>(hi + off + q * 16) = h4;
+      if (KIND == K_BF16X3)
         *reinterpret_cast<uint4 *>(lo + off + q * 16) =
-            make_uint4(pack_bf16(rr[0], rr[1]), pack_bf16(rr[2], rr[3]), pack_bf16(rr[4], rr[5]),
-                       pack_bf16(rr[6], rr[7]));
-      }
+            make_uint4(pack_rest(h4.x, v[q][0], v[q][1]), pack_rest(h4.y, v[q][2], v[q][3]),
+                       pack_rest(h4.z, v[q][4], v[q][5]), pack_rest(h4.w, v[q][6], v[q][7]));
     }
   }
 }

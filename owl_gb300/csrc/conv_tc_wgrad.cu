@@ -24,6 +24,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "../../include/owlgpu.h"
 #include "common.cuh"
@@ -38,15 +39,15 @@ using namespace ptx;
 
 // Warp roles.  The accumulator is drained once per CTA, after the last
 // pixel tile, so every warp but the MMA issuer (warp 0) stages operands;
-// warps 12-15, one per TMEM lane quadrant, then drain the accumulator.
+// warps 4-15, three per TMEM lane quadrant, then drain the accumulator (8.7 us
+// of [64;56;56;128]x[3;3;128;128] with one per quadrant).
 // (Measured on GB300: 15 producer warps beat 9 or 12 here even though three
 // of them share the MMA warp's scheduler.)
 constexpr int kWarps = 16;
 constexpr int kThreads = kWarps * 32;
 constexpr int kMmaWarp = 0;
-constexpr int kEpiWarp0 = 12;
+constexpr int kEpiWarp0 = 4, kEpiParts = (kWarps - kEpiWarp0) / 4;
 constexpr int kProducerWarps = kWarps - 1;
-constexpr int kProducerThreads = kProducerWarps * 32;
 __device__ __forceinline__ int producer_index(int warp) { return warp - 1; }
 constexpr int kSmemMax = 232448;
 // Taps are grouped through a table in the launch parameters when the
@@ -68,12 +69,16 @@ struct WgParams {
                           // of one pixel fall in different shared-memory banks
   int u_tiles, v_tiles;
   long long total_tiles, tiles_per_range;
+  int n_tab;              // pixels of the largest X halo and the dY tile (the LANES tables)
   int PS;                 // X halo plane stride in pixels (max over groups)
   unsigned x_bytes, y_bytes;  // per stage, per precision part
   int NS;
   unsigned idesc, tmem_cols;
   unsigned small_off;  // BF16X3: TMEM column of the cross-term accumulators (TG * BN)
   int vec_x, vec_y;
+  // LANES: floats from a tile's first pixel to the next tile's along v; from there
+  // to the next row of tiles; and so on along w and b
+  long long x_dv, x_du, x_dw, x_db, y_dv, y_du, y_dw, y_db;
   // Tap groups.  ordered: group g holds taps tap_order[gstart[g] ..
   // gstart[g+1]); else group g holds taps g*TG .. min(T, (g+1)*TG) - 1.
   // Every group is phase-uniform: all its taps have the same k*d mod s in
@@ -100,6 +105,13 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
       return false;
     }
   }
+}
+
+// A producer warp's: the same answer for all its lanes (they arrive together).
+__device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity,
+                                              volatile int *abort_flag, int *status,
+                                              long long limit) {
+  return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag, status, limit));
 }
 
 // The MMA warp's: polled by the whole warp.
@@ -141,11 +153,11 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
   const int YPL = p.BN * EB / 16;
 
   // ---- work unit of this CTA ----
-  long long u = blockIdx.x;
-  const int tg = (int)(u % p.n_tg); u /= p.n_tg;
-  const int nb = (int)(u % p.n_nb); u /= p.n_nb;
-  const int mb = (int)(u % p.n_mb);
-  const int r = (int)(u / p.n_mb);
+  unsigned u = blockIdx.x;
+  const int tg = (int)(u % (unsigned)p.n_tg); u /= (unsigned)p.n_tg;
+  const int nb = (int)(u % (unsigned)p.n_nb); u /= (unsigned)p.n_nb;
+  const int mb = (int)(u % (unsigned)p.n_mb);
+  const int r = (int)(u / (unsigned)p.n_mb);
   const long long t_begin = (long long)r * p.tiles_per_range;
   const long long t_end = min(p.total_tiles, t_begin + p.tiles_per_range);
   const int gbeg = p.ordered ? (int)p.gstart[tg] : tg * p.TG;
@@ -191,9 +203,29 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
                             (kv * p.dv - minv) / p.sv);
   }
 
+  // LANES: where the tile's pixels lie, X's then dY's: {offset in floats from the
+  // tile's first pixel, position}, and one past the end that is outside any bounds
+  int2 *xtab = reinterpret_cast<int2 *>((reinterpret_cast<uintptr_t>(tap_off + p.TG) + 7) &
+                                        ~(uintptr_t)7);
+  int2 *ytab = xtab + xrows * HVR + 1;
+  if (LANES) {
+    const int n = xrows * HVR, out = (int)(stage::position(stage::kMaxV + 1, 0, 0) | stage::kGuard);
+    for (int i = threadIdx.x; i <= n; i += blockDim.x) {
+      const int hv = i % HVR, hu = (i / HVR) % HU, hw = i / (HVR * HU);
+      xtab[i] =
+          i < n ? make_int2((int)((hw * p.sw * p.xsw + hu * p.su * p.xsu + hv * p.sv * p.xsv) * p.Ci),
+                            (int)(stage::position(hv * p.sv, hu * p.su, hw * p.sw) | stage::kGuard))
+                : make_int2(0, out);
+    }
+    for (int i = threadIdx.x; i <= p.TP; i += blockDim.x)
+      ytab[i] = i < p.TP ? make_int2((int)((i / 8 * p.ysu + i % 8 * p.ysv) * p.Co),
+                                     (int)(stage::position(i % 8, i / 8, 0) | stage::kGuard))
+                         : make_int2(0, out);
+  }
+
   if (threadIdx.x == 0) {
     for (int i = 0; i < p.NS; ++i) {
-      mbar_init(smem_u32(&full[i]), kProducerThreads);
+      mbar_init(smem_u32(&full[i]), kProducerWarps);
       mbar_init(smem_u32(&empty[i]), 1);
     }
     mbar_init(smem_u32(acc_full), 1);
@@ -240,116 +272,182 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
     };
     int st = 0;
     uint32_t ph = 1;
-    // LANES: the chunks that exist are staged (the planes past the channels stay
-    // as they are: they only reach accumulator rows and columns that are not
-    // stored), QX and QY pixels of a row per lane and round
-    constexpr int QX = 5, QY = 4;
-    const stage::Lane lx(min(XPL, (p.Ci - mb * 128 + 7) / 8), lane);
-    const stage::Lane ly(min(YPL, (p.Co - nb * p.BN + 7) / 8), lane);
-    const int nx = lx.on ? (HVR - lx.i0 + lx.di - 1) / lx.di : 0;  // the lane's pixels of a row
-    const int ny = ly.on ? (8 - ly.i0 + ly.di - 1) / ly.di : 0;
-    const uint32_t lane_x = (uint32_t)lx.j * (uint32_t)p.PS * 16u + (uint32_t)lx.i0 * 16u,
-                   lane_y = (uint32_t)ly.j * (uint32_t)p.YPS * 16u + (uint32_t)ly.i0 * 16u;
-    const long long pix_x = (long long)p.sv * p.xsv * p.Ci, pix_y = p.ysv * (long long)p.Co;
-    const int steps_x = (HVR + lx.di - 1) / lx.di, steps_y = (8 + ly.di - 1) / ly.di;
-    for (long long t = t_begin; t < t_end; ++t, next_tile()) {
-      if (!wait_bar(smem_u32(&empty[st]), ph, abort_flag, p.status, p.spin_limit)) {
-        staged = false;
-        break;
-      }
-      uint8_t *xd = xs + (size_t)st * PARTS * p.x_bytes;
-      uint8_t *yd = ys + (size_t)st * PARTS * p.y_bytes;
-      // X halo: rows (w, u) of HVR pixels x 128 channels of ci block mb;
-      // dY tile: TU rows (u) of 8 output pixels x BN channels of co block nb.
-      const int xcb = mb * 128, ycb = nb * p.BN;
-      if constexpr (LANES) {
-        const int ivs = v0 * p.sv - p.pv + minv;
-        const float *xt = p.x +
-                          ((long long)b * p.xsb + (long long)(ivs + lx.i0 * p.sv) * p.xsv) * p.Ci +
-                          xcb + lx.j * 8;
-        const float *yt = p.dy +
-                          ((long long)b * p.ysb + (long long)ow * p.ysw +
-                           (long long)(v0 + ly.i0) * p.ysv) * p.Co + ycb + ly.j * 8;
-        const int iw0 = ow * p.sw - p.pw + minw, iu0 = u0 * p.su - p.pu + minu;
-        int hw = 0, hu = pidx;
-        while (hu >= HU) { hu -= HU; ++hw; }
-        for (int r = pidx; r < xrows || r < p.TU; r += kProducerWarps) {
-          const int iw = iw0 + hw * p.sw, iu = iu0 + hu * p.su;
-          const bool xok = r < xrows && (unsigned)iw < (unsigned)p.IW &&
-                           (unsigned)iu < (unsigned)p.IU && lx.on;
-          const bool yok = r < p.TU && u0 + r < p.OU && ly.on;
-          const float *xs_ = xt + ((long long)iw * p.xsw + (long long)iu * p.xsu) * p.Ci;
-          const float *ys_ = yt + (long long)(u0 + r) * p.ysu * p.Co;
-          uint8_t *xdst = xd + lane_x + (uint32_t)(r * HVR) * 16u;
-          uint8_t *ydst = yd + lane_y + (uint32_t)r * 128u;
-          const int mx = r < xrows ? nx : 0, my = r < p.TU ? ny : 0;
-          const int sx = r < xrows ? steps_x : 0, sy = r < p.TU ? steps_y : 0;
-          for (int k = 0; k * QX < sx || k * QY < sy; ++k) {
-            float vx[QX][8], vy[QY][8];
-            stage::lane_load<QX>(xs_ + (long long)k * QX * lx.di * pix_x, lx.di * pix_x,
-                                 ivs + (lx.i0 + k * QX * lx.di) * p.sv, lx.di * p.sv,
-                                 xok ? (unsigned)p.IV : 0u, sx - k * QX, vx);
-            stage::lane_load<QY>(ys_ + (long long)k * QY * ly.di * pix_y, ly.di * pix_y,
-                                 v0 + ly.i0 + k * QY * ly.di, ly.di, yok ? (unsigned)p.OV : 0u,
-                                 sy - k * QY, vy);
-            stage::lane_store<KIND, QX>(xdst + (uint32_t)(k * QX * lx.di) * 16u,
-                                        (uint32_t)lx.di * 16u, p.x_bytes, mx - k * QX, vx);
-            stage::lane_store<KIND, QY>(ydst + (uint32_t)(k * QY * ly.di) * 16u,
-                                        (uint32_t)ly.di * 16u, p.y_bytes, my - k * QY, vy);
+    if constexpr (LANES) {
+      // The chunks that exist are staged (the planes past the channels stay as they
+      // are: they only reach accumulator rows and columns that are not stored): a
+      // lane keeps one chunk of each operand and takes every lanes/chunks-th pixel of
+      // the tile, QX of X and QY of dY a round (one round for most tiles).  Where a
+      // pixel lies relative to its tile comes from a table, the tile's pointers
+      // advance by constant steps and only tiles at the array's edge test their
+      // pixels: with row and pixel arithmetic in the loop it took 610 instructions a
+      // warp and tile (54% of the issue slots), with conversion and stores some 80 of
+      // them.  The loads of one operand are in flight while the other is converted
+      // and stored, the next round's (or tile's) X while this one's dY: issued
+      // together and then waited for they cost a round trip, in all warps at once.
+      const int id = pidx * 32 + lane;
+      const int nchx = min(XPL, (p.Ci - mb * 128 + 7) / 8), nchy = min(YPL, (p.Co - nb * p.BN + 7) / 8);
+      const int lgx = 32 - __clz(nchx - 1), lgy = 32 - __clz(nchy - 1);  // (clz(0) = 32)
+      const int jx = id & ((1 << lgx) - 1), jy = id & ((1 << lgy) - 1);
+      const int px = id >> lgx, dpx = (kProducerWarps * 32) >> lgx, npx = xrows * HVR;
+      const int py = id >> lgy, dpy = (kProducerWarps * 32) >> lgy, npy = p.TP;
+      const bool onx = jx < nchx, ony = jy < nchy;  // (others load chunk 0 and store nothing)
+      const int rounds_x = (npx + dpx - 1) / dpx, rounds_y = (npy + dpy - 1) / dpy;
+      const uint32_t lane_x = (uint32_t)(jx * p.PS + px) * 16u, lane_y = (uint32_t)(jy * p.YPS + py) * 16u;
+      int iw0 = ow * p.sw - p.pw + minw, iu0 = u0 * p.su - p.pu + minu, iv0 = v0 * p.sv - p.pv + minv;
+      const float *xt = p.x + ((long long)b * p.xsb + (long long)iw0 * p.xsw + (long long)iu0 * p.xsu +
+                               (long long)iv0 * p.xsv) * p.Ci + mb * 128 + (onx ? jx * 8 : 0);
+      const float *yt = p.dy + ((long long)b * p.ysb + (long long)ow * p.ysw + (long long)u0 * p.ysu +
+                                (long long)v0 * p.ysv) * p.Co + nb * p.BN + (ony ? jy * 8 : 0);
+      // the parts of the tile that lie inside the arrays: along u and w, then along v too
+      unsigned x_lo, x_hi, y_lo, y_hi;
+      auto rows_in = [&] {
+        unsigned l, h;
+        stage::field(iu0, p.IU, stage::kMaxU, l, h);
+        x_lo = l << 11;
+        x_hi = h << 11;
+        stage::field(iw0, p.IW, stage::kMaxW, l, h);
+        x_lo |= l << 22;
+        x_hi |= h << 22;
+        stage::field(u0, p.OU, stage::kMaxU, l, h);
+        y_lo = l << 11;
+        y_hi = h << 11;
+      };
+      rows_in();
+      auto stage_tiles = [&](auto qx, auto qy) {
+        constexpr int QX = qx.value, QY = qy.value;
+        float vx[QX][8], vy[QY][8];
+        long long left = t_end - t_begin;
+        int k = 0;
+        auto load_x = [&] {
+          unsigned l, h;
+          stage::field(iv0, left > 0 ? p.IV : -p.IV, stage::kMaxV, l, h);
+          stage::table_load<QX>(xtab, px + k * dpx * QX, dpx, npx, xt, x_lo | l, x_hi | h, vx);
+        };
+        load_x();
+        while (left > 0) {
+          {
+            unsigned l, h;
+            stage::field(v0, p.OV, stage::kMaxV, l, h);
+            stage::table_load<QY>(ytab, py + k * dpy * QY, dpy, npy, yt, y_lo | l, y_hi | h, vy);
           }
-          hu += kProducerWarps;
-          while (hu >= HU) { hu -= HU; ++hw; }
+          if (k == 0 &&
+              !wait_bar_warp(smem_u32(&empty[st]), ph, abort_flag, p.status, p.spin_limit)) {
+            staged = false;
+            break;
+          }
+          const int kx = k * dpx * QX, ky = k * dpy * QY;
+          uint8_t *yd = ys + (uint32_t)st * PARTS * p.y_bytes + lane_y + (uint32_t)ky * 16u;
+          const int ny = ony ? npy - py - ky : 0;
+          stage::table_store<KIND, QX>(xs + (uint32_t)st * PARTS * p.x_bytes + lane_x + (uint32_t)kx * 16u,
+                                       dpx, p.x_bytes, onx ? npx - px - kx : 0, vx);
+          ++k;
+          const bool last = k * QX >= rounds_x && k * QY >= rounds_y;  // the tile's last round
+          if (last) {
+            k = 0;
+            --left;
+            v0 += 8;
+            iv0 += 8 * p.sv;
+            xt += p.x_dv;
+            yt += p.y_dv;
+            if (v0 == v_end) {
+              v0 = 0;
+              u0 += p.TU;
+              xt += p.x_du;
+              yt += p.y_du;
+              if (u0 == u_end) {
+                u0 = 0;
+                xt += p.x_dw;
+                yt += p.y_dw;
+                if (++ow == p.OW) {
+                  ow = 0;
+                  xt += p.x_db;
+                  yt += p.y_db;
+                }
+              }
+              iw0 = ow * p.sw - p.pw + minw;
+              iu0 = u0 * p.su - p.pu + minu;
+              iv0 = minv - p.pv;
+              rows_in();
+            }
+          }
+          load_x();
+          stage::table_store<KIND, QY>(yd, dpy, p.y_bytes, ny, vy);
+          if (last) {
+            fence_proxy_async();
+            mbar_arrive_warp(smem_u32(&full[st]), lane);
+            if (++st == p.NS) { st = 0; ph ^= 1; }
+          }
         }
-      } else {
-      auto xrow = [&](int r) {
-        const int hu = r % HU, hw = r / HU;
-        const int iw = ow * p.sw - p.pw + minw + hw * p.sw;
-        const int iu = u0 * p.su - p.pu + minu + hu * p.su;
-        const int ivs = v0 * p.sv - p.pv + minv;
-        stage::Row row;
-        row.ok = iw >= 0 && iw < p.IW && iu >= 0 && iu < p.IU;
-        row.rowp = p.x + ((long long)b * p.xsb + (long long)iw * p.xsw + (long long)iu * p.xsu +
-                          (long long)ivs * p.xsv) * p.Ci + xcb;
-        row.pstep = (long long)p.sv * p.xsv * p.Ci;
-        row.vfirst = ivs;
-        row.vstride = p.sv;
-        row.vlim = p.IV;
-        return row;
       };
-      auto yrow = [&](int r) {
-        const int ou = u0 + r;
-        stage::Row row;
-        row.ok = ou < p.OU;
-        row.rowp = p.dy + ((long long)b * p.ysb + (long long)ow * p.ysw + (long long)ou * p.ysu +
-                           (long long)v0 * p.ysv) * p.Co + ycb;
-        row.pstep = p.ysv * p.Co;
-        row.vfirst = v0;
-        row.vstride = 1;
-        row.vlim = p.OV;
-        return row;
-      };
-      if (paired) {
-        // at most one row of each per warp: both rows in one pass
-        stage::RowSet sx{xd, p.x_bytes, (uint32_t)p.PS * 16, xrows, HVR, XPL, p.Ci - xcb};
-        stage::RowSet sy{yd, p.y_bytes, (uint32_t)p.YPS * 16, p.TU, 8, YPL, p.Co - ycb};
-        stage::stage_rows2<KIND, EPC, 5, 4>(sx, xrow, sy, yrow, min(p.vec_x, p.vec_y),
-                                            pidx, kProducerWarps, lane);
-      } else {
-        stage::stage_rows<KIND, EPC, 6>(xd, p.x_bytes, (uint32_t)p.PS * 16, xrows, HVR, XPL,
-                                        p.Ci - xcb, p.vec_x, pidx, kProducerWarps, lane,
-                                        xrow);
-        stage::stage_rows<KIND, EPC, 4>(yd, p.y_bytes, (uint32_t)p.YPS * 16, p.TU, 8, YPL,
-                                        p.Co - ycb, p.vec_y, pidx, kProducerWarps, lane,
-                                        yrow);
+      // tiles of few pixels (or channels): fewer slots, each of which costs its
+      // instructions whether the tile has a pixel for it or not
+      if (rounds_x <= 3 && rounds_y <= 3)
+        stage_tiles(std::integral_constant<int, 3>{}, std::integral_constant<int, 3>{});
+      else
+        stage_tiles(std::integral_constant<int, 5>{}, std::integral_constant<int, 4>{});
+    } else {
+      for (long long t = t_begin; t < t_end; ++t, next_tile()) {
+        if (!wait_bar_warp(smem_u32(&empty[st]), ph, abort_flag, p.status, p.spin_limit)) {
+          staged = false;
+          break;
+        }
+        uint8_t *xd = xs + (size_t)st * PARTS * p.x_bytes;
+        uint8_t *yd = ys + (size_t)st * PARTS * p.y_bytes;
+        // X halo: rows (w, u) of HVR pixels x 128 channels of ci block mb;
+        // dY tile: TU rows (u) of 8 output pixels x BN channels of co block nb.
+        const int xcb = mb * 128, ycb = nb * p.BN;
+        auto xrow = [&](int r) {
+          const int hu = r % HU, hw = r / HU;
+          const int iw = ow * p.sw - p.pw + minw + hw * p.sw;
+          const int iu = u0 * p.su - p.pu + minu + hu * p.su;
+          const int ivs = v0 * p.sv - p.pv + minv;
+          stage::Row row;
+          row.ok = iw >= 0 && iw < p.IW && iu >= 0 && iu < p.IU;
+          row.rowp = p.x + ((long long)b * p.xsb + (long long)iw * p.xsw + (long long)iu * p.xsu +
+                            (long long)ivs * p.xsv) * p.Ci + xcb;
+          row.pstep = (long long)p.sv * p.xsv * p.Ci;
+          row.vfirst = ivs;
+          row.vstride = p.sv;
+          row.vlim = p.IV;
+          return row;
+        };
+        auto yrow = [&](int r) {
+          const int ou = u0 + r;
+          stage::Row row;
+          row.ok = ou < p.OU;
+          row.rowp = p.dy + ((long long)b * p.ysb + (long long)ow * p.ysw + (long long)ou * p.ysu +
+                             (long long)v0 * p.ysv) * p.Co + ycb;
+          row.pstep = p.ysv * p.Co;
+          row.vfirst = v0;
+          row.vstride = 1;
+          row.vlim = p.OV;
+          return row;
+        };
+        if (paired) {
+          // at most one row of each per warp: both rows in one pass
+          stage::RowSet sx{xd, p.x_bytes, (uint32_t)p.PS * 16, xrows, HVR, XPL, p.Ci - xcb};
+          stage::RowSet sy{yd, p.y_bytes, (uint32_t)p.YPS * 16, p.TU, 8, YPL, p.Co - ycb};
+          stage::stage_rows2<KIND, EPC, 5, 4>(sx, xrow, sy, yrow, min(p.vec_x, p.vec_y),
+                                              pidx, kProducerWarps, lane);
+        } else {
+          stage::stage_rows<KIND, EPC, 6>(xd, p.x_bytes, (uint32_t)p.PS * 16, xrows, HVR, XPL,
+                                          p.Ci - xcb, p.vec_x, pidx, kProducerWarps, lane,
+                                          xrow);
+          stage::stage_rows<KIND, EPC, 4>(yd, p.y_bytes, (uint32_t)p.YPS * 16, p.TU, 8, YPL,
+                                          p.Co - ycb, p.vec_y, pidx, kProducerWarps, lane,
+                                          yrow);
+        }
+        fence_proxy_async();
+        mbar_arrive_warp(smem_u32(&full[st]), lane);
+        if (++st == p.NS) { st = 0; ph ^= 1; }
       }
-      }
-      fence_proxy_async();
-      mbar_arrive(smem_u32(&full[st]));
-      if (++st == p.NS) { st = 0; ph ^= 1; }
     }
     if (staged && warp >= kEpiWarp0) {
       // ===================== epilogue: TMEM -> partial dW =====================
+      // (a warp reaches the TMEM lanes of its quadrant, warp % 4; the quadrant's
+      // warps take every kEpiParts-th 16 columns)
       const int q = warp & 3;
+      int mine = (warp - kEpiWarp0) >> 2;
       const int ci = mb * 128 + q * 32 + lane;
       if (wait_bar(smem_u32(acc_full), 0, abort_flag, p.status, p.spin_limit)) {
         tc_fence_after();
@@ -358,6 +456,11 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
           float *out = p.out + (((long long)r * p.T + tt) * p.Ci + ci) * p.Co + nb * p.BN;
           const uint32_t tcol = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(i * p.BN);
           for (int c0 = 0; c0 < p.BN; c0 += 16) {
+            if (mine != 0) {
+              --mine;
+              continue;
+            }
+            mine = kEpiParts - 1;
             uint32_t rr[16];
             tmem_ld16(tcol + (uint32_t)c0, rr);
             if (SEP) {
@@ -372,7 +475,10 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
             }
             if (ci < p.Ci) {
               const int n0 = nb * p.BN + c0;
-              if (p.vec_y && n0 + 16 <= p.Co && ((uintptr_t)(out + c0) % 16 == 0)) {
+              if (p.vec_y == 2 && n0 + 16 <= p.Co && ((uintptr_t)(out + c0) % 32 == 0)) {
+                stage::st8(out + c0, rr);
+                stage::st8(out + c0 + 8, rr + 8);
+              } else if (p.vec_y && n0 + 16 <= p.Co && ((uintptr_t)(out + c0) % 16 == 0)) {
 #pragma unroll
                 for (int e = 0; e < 16; e += 4)
                   *reinterpret_cast<float4 *>(out + c0 + e) =
@@ -475,6 +581,31 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
     tc_fence_after();
     tmem_dealloc(tmem_base, p.tmem_cols);
   }
+}
+
+// Estimated time of a plan in cycles, from a fit to 950 plans of twelve layers on
+// GB300 (3% off on average; the choice needs the ratios only).  A tile costs its
+// rounds of staging slots, its bytes and its MMAs, which overlap little; each wave
+// of CTAs an epilogue; the partial sums their writing and reading.
+double estimate(const WgParams &p, int halo_pixels, int parts, long long ctas, int sms) {
+  auto pow2 = [](int n) {
+    int q = 1;
+    while (q < n) q *= 2;
+    return q;
+  };
+  const int nx = std::min(16, (p.Ci + 7) / 8), ny = std::min(p.BN / 8, (p.Co + 7) / 8);
+  const int lanes = kProducerWarps * 32;
+  const int rx = (halo_pixels * pow2(nx) + lanes - 1) / lanes,
+            ry = (p.TP * pow2(ny) + lanes - 1) / lanes;
+  const bool few = rx <= 3 && ry <= 3;
+  const int rounds = few ? 1 : std::max((rx + 4) / 5, (ry + 3) / 4);
+  const double mma = p.TG <= 4 ? 23 : 45;
+  const double tile = rounds * (390 + (few ? 6 : 9) * (parts == 2 ? 135 : 132)) +
+                      (halo_pixels * nx + p.TP * ny) * 32 / 115.0 +
+                      p.TP / 16 * p.TG * (parts == 2 ? 3 : 1) * std::max(mma, 0.26 * p.BN);
+  const double waves = (double)((ctas + sms - 1) / sms);
+  const double sums = p.R > 1 ? 1.3e-3 * p.T * p.Ci * (double)p.Co * p.R : 0.0;
+  return waves * ((double)p.tiles_per_range * tile + 25.0 * p.TG * p.BN * parts) + sums;
 }
 
 int sm_count() {
@@ -604,10 +735,38 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
     p.TG = widest;
     return n;
   };
-  // Halo pixels of the largest group for tile height tu.
-  auto max_halo = [&](int tu) {
-    int maxHP = 0;
-    for (int gi = 0; gi < p.n_tg; ++gi) {
+  // Plan: BN output channels and TG taps per CTA (TG*BN <= 512 TMEM columns, or
+  // 2*TG*BN with split-BF16's separate cross-term accumulators) and tiles of TU (even,
+  // so that TU*8 pixels fill whole 16-pixel K steps) rows, two stages of which fit
+  // shared memory: those with the least estimated time.  Fewer, wider groups stage
+  // the activations less often, smaller ones fill the SMs with longer pixel ranges
+  // and leave fewer partial sums: with the widest block and the tallest tile first
+  // [16;14;14;256]x[3;3;256;256] took 27.6 us where 128 channels a CTA take 22, 64 x
+  // 7x7x512 72 where they take 46, and [64;56;56;128]x[3;3;128;128] at rate 2 in
+  // split BF16, one tap per CTA, 250 where TU = 8 and two taps take 194.
+  const int sms = sm_count();
+  int tus[8], ntu = 0;  // the heights that leave the fewest rows past the output
+  for (int tiles = 1, tu = 17; ntu < 5 && tu > 2; ++tiles) {
+    const int t = std::max(2, (p.OU + tiles - 1) / tiles + 1) / 2 * 2;
+    if (t > 16 || t >= tu) continue;
+    tus[ntu++] = tu = t;
+  }
+  struct Halo {
+    int w, u, v;
+  };
+  constexpr int kMaxHalos = 32;
+  Halo halo[kMaxHalos];
+  const long long rows = (long long)p.B * p.OW;
+  double least = -1;
+  int best_tg = 0, last_n = -1;
+  WgParams best = p;
+  for (int tg = std::min(p.T, 16); tg >= 1; --tg) {
+    const int n = p.n_tg = make_groups(tg);
+    if (n == last_n) continue;
+    last_n = n;
+    // the groups' halos beyond a tile, those that lie within another left out
+    int nh = 0;
+    for (int gi = 0; gi < n; ++gi) {
       const int b0 = p.ordered ? p.gstart[gi] : gi * p.TG;
       const int b1 = p.ordered ? p.gstart[gi + 1] : std::min(p.T, b0 + p.TG);
       int mnw = 1 << 30, mnu = 1 << 30, mnv = 1 << 30, mxw = -1, mxu = -1, mxv = -1;
@@ -618,82 +777,67 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
         mnu = std::min(mnu, ku * p.du); mxu = std::max(mxu, ku * p.du);
         mnv = std::min(mnv, kv * p.dv); mxv = std::max(mxv, kv * p.dv);
       }
-      maxHP = std::max(maxHP, ((mxw - mnw) / p.sw + 1) * (tu + (mxu - mnu) / p.su) *
-                                  (8 + (mxv - mnv) / p.sv));
+      const Halo h{(mxw - mnw) / p.sw + 1, (mxu - mnu) / p.su, (mxv - mnv) / p.sv};
+      bool seen = false;
+      for (int i = 0; i < nh && !seen; ++i)
+        seen = halo[i].w >= h.w && halo[i].u >= h.u && halo[i].v >= h.v;
+      if (seen) continue;
+      if (nh < kMaxHalos) {
+        halo[nh++] = h;
+      } else {  // one that holds both
+        Halo &l = halo[nh - 1];
+        l = {std::max(l.w, h.w), std::max(l.u, h.u), std::max(l.v, h.v)};
+      }
     }
-    return maxHP;
-  };
-
-  // Plan: BN (co block), TG (taps per CTA, TG*BN <= 512 TMEM columns, or
-  // 2*TG*BN with split-BF16's separate cross-term accumulators), NS = 2.
-  // Tile height TU (even, so that TU*8 pixels fill whole 16-pixel K steps),
-  // tried in order of estimated cost: rows staged including padding plus a
-  // fixed per-tile cost of about four rows; a tile taller than the number of
-  // producer warps needs a second staging pass and ranks last.
-  int tus[8], ntu = 0;
-  {
-    int cand[8] = {14, 12, 10, 16, 8, 6, 4, 2}, waste[8];
-    for (int i = 0; i < 8; ++i) {
-      waste[i] = (p.OU + cand[i] - 1) / cand[i] * (cand[i] + 4);
-      if (cand[i] > kProducerWarps) waste[i] += 1 << 20;
-    }
-    bool used[8] = {false};
-    for (int k = 0; k < 8; ++k) {
-      int best = -1;
-      for (int i = 0; i < 8; ++i)
-        if (!used[i] && (best < 0 || waste[i] < waste[best] ||
-                         (waste[i] == waste[best] && cand[i] > cand[best])))
-          best = i;
-      used[best] = true;
-      tus[ntu++] = cand[best];
-    }
-  }
-  // Widest output-channel block first (it is the MMA's N: narrow blocks waste
-  // the tensor core), then the cheapest tile height, then the fewest tap
-  // groups whose two stages of X halo + dY tile fit shared memory.
-  bool planned = false;
-  for (int bn : {256, 128, 64, 32, 16}) {
-    if (planned) break;
-    p.BN = std::min(bn, (p.Co + 15) / 16 * 16);
-    const int tg_max = std::min(p.T, std::min(16, 512 / (parts * p.BN)));
-    if (tg_max < 1) continue;
-    for (int ti = 0; ti < ntu && !planned; ++ti) {
-      const int tu = tus[ti];
-      p.TU = tu;
-      p.TP = tu * 8;
-      p.YPS = p.TP + 1;
-      int last_n = -1;
-      for (int tg = tg_max; tg >= 1 && !planned; --tg) {
-        p.n_tg = make_groups(tg);
-        if (p.n_tg == last_n) continue;
-        last_n = p.n_tg;
-        const int maxHP = max_halo(tu);
-        p.PS = maxHP + (((1 - maxHP) % 8) + 8) % 8;
+    int last_bn = 0;
+    for (int bn : {256, 128, 64, 32, 16}) {
+      p.BN = std::min(bn, (p.Co + 15) / 16 * 16);
+      if (p.BN == last_bn || parts * p.TG * p.BN > 512) continue;
+      if (bn < 64 && least >= 0) continue;  // (narrow blocks waste the tensor core)
+      last_bn = p.BN;
+      for (int ti = 0; ti < ntu; ++ti) {
+        const int tu = tus[ti];
+        int HP = 0;
+        for (int i = 0; i < nh; ++i)
+          HP = std::max(HP, halo[i].w * (tu + halo[i].u) * (8 + halo[i].v));
+        p.TU = tu;
+        p.TP = tu * 8;
+        p.YPS = p.TP + 1;
+        p.PS = HP + (((1 - HP) % 8) + 8) % 8;
         if (p.PS >= 16384) continue;
         p.x_bytes = (unsigned)(128 * EB / 16) * (unsigned)p.PS * 16u;
         p.y_bytes = (unsigned)(p.BN * EB / 16) * (unsigned)p.YPS * 16u;
         p.NS = 2;
-        const size_t need = (size_t)p.NS * parts * (p.x_bytes + p.y_bytes) + 256;
-        if (need <= (size_t)kSmemMax) planned = true;
+        p.n_tab = HP + p.TP;
+        const size_t need = (size_t)p.NS * parts * (p.x_bytes + p.y_bytes) + 256 +
+                            8 * (size_t)(p.n_tab + 3);
+        if (need > (size_t)kSmemMax) continue;
+        p.u_tiles = (p.OU + tu - 1) / tu;
+        p.v_tiles = (p.OV + 7) / 8;
+        p.total_tiles = rows * p.u_tiles * p.v_tiles;
+        p.n_nb = (p.Co + p.BN - 1) / p.BN;
+        // pixel ranges: enough CTAs to fill the GPU once
+        const long long units = (long long)n * p.n_nb * p.n_mb;
+        long long R = std::min(std::max<long long>(1, sms / units), p.total_tiles);
+        p.tiles_per_range = (p.total_tiles + R - 1) / R;
+        R = (p.total_tiles + p.tiles_per_range - 1) / p.tiles_per_range;
+        p.R = (int)R;
+        const double t = estimate(p, HP, parts, units * R, sms);
+        if (least < 0 || t < least) {
+          least = t;
+          best = p;
+          best_tg = tg;
+        }
       }
     }
   }
-  if (!planned) return kErrUnsupported;
-  p.u_tiles = (p.OU + p.TU - 1) / p.TU;
-  p.v_tiles = (p.OV + 7) / 8;
-  p.total_tiles = (long long)p.B * p.OW * p.u_tiles * p.v_tiles;
-  p.n_nb = (p.Co + p.BN - 1) / p.BN;
+  if (least < 0) return kErrUnsupported;
+  p = best;
+  p.n_tg = make_groups(best_tg);
   p.small_off = (unsigned)(p.TG * p.BN);
   p.tmem_cols = 32;
   while (p.tmem_cols < (unsigned)(parts * p.TG * p.BN)) p.tmem_cols <<= 1;
-  // pixel ranges: enough CTAs to fill the GPU once
   const long long units = (long long)p.n_tg * p.n_nb * p.n_mb;
-  const int sms = sm_count();
-  long long R = std::max<long long>(1, sms / std::max<long long>(1, units));
-  R = std::min<long long>(R, p.total_tiles);
-  p.tiles_per_range = (p.total_tiles + R - 1) / R;
-  R = (p.total_tiles + p.tiles_per_range - 1) / p.tiles_per_range;
-  p.R = (int)R;
   uint32_t idesc = instr_desc(kind == K_TF32 ? 2u : 1u, (uint32_t)p.BN);
   idesc |= (1u << 15) | (1u << 16);  // A and B MN-major
   p.idesc = idesc;
@@ -720,10 +864,26 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
     p.out = dw;
   }
   const size_t smem =
-      (size_t)p.NS * parts * (p.x_bytes + p.y_bytes) + (2 * p.NS + 2) * 8 + 16 + 4 * (size_t)p.TG;
+      (size_t)p.NS * parts * (p.x_bytes + p.y_bytes) + (2 * p.NS + 2) * 8 + 16 + 4 * (size_t)p.TG +
+      8 * (size_t)(p.n_tab + 3);
   const int grid = (int)(units * p.R);
   int rc;
-  const bool lanes = p.vec_x == 2 && p.vec_y == 2;
+  // (the tables' offsets are 32-bit, their positions' fields 10, 10 and 9 bits)
+  const long long fw = (long long)p.KW * p.dw + p.sw,
+                  fu = (long long)p.TU * p.su + (long long)p.KU * p.du,
+                  fv = 8LL * p.sv + (long long)p.KV * p.dv;
+  const bool lanes = p.vec_x == 2 && p.vec_y == 2 && fw <= stage::kMaxW && fu <= stage::kMaxU &&
+                     fv <= stage::kMaxV &&
+                     (fw * p.xsw + fu * p.xsu + fv * p.xsv) * p.Ci < (1LL << 31) &&
+                     (p.TU * p.ysu + 8 * p.ysv) * p.Co < (1LL << 31);
+  p.x_dv = 8LL * p.sv * p.xsv * p.Ci;
+  p.x_du = (long long)p.TU * p.su * p.xsu * p.Ci - p.v_tiles * p.x_dv;
+  p.x_dw = p.sw * p.xsw * p.Ci - (long long)p.u_tiles * p.TU * p.su * p.xsu * p.Ci;
+  p.x_db = p.xsb * p.Ci - (long long)p.OW * p.sw * p.xsw * p.Ci;
+  p.y_dv = 8LL * p.ysv * p.Co;
+  p.y_du = (long long)p.TU * p.ysu * p.Co - p.v_tiles * p.y_dv;
+  p.y_dw = p.ysw * p.Co - (long long)p.u_tiles * p.TU * p.ysu * p.Co;
+  p.y_db = p.ysb * p.Co - (long long)p.OW * p.ysw * p.Co;
   if (kind == K_BF16X3)
     rc = lanes ? launch<K_BF16X3, true>(p, smem, grid, s) : launch<K_BF16X3, false>(p, smem, grid, s);
   else

@@ -107,6 +107,13 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
   }
 }
 
+// A producer warp's: the same answer for all its lanes (they arrive together).
+__device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity,
+                                              volatile int *abort_flag, int *status,
+                                              long long limit) {
+  return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag, status, limit));
+}
+
 // The MMA warp's: polled by the whole warp.
 __device__ __forceinline__ bool poll_bar(uint32_t bar, uint32_t parity, volatile int *abort_flag,
                                          int *status, long long limit) {
@@ -322,7 +329,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < p.NS; ++i) {
-      mbar_init(smem_u32(&full[i]), kProducerThreads);
+      mbar_init(smem_u32(&full[i]), kWarps - 1);
       mbar_init(smem_u32(&empty[i]), 1);
     }
     mbar_init(smem_u32(acc_full), 1);
@@ -377,14 +384,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
       if (!stage_round<KIND>(stg, p.a_bytes, p.b_bytes, A, B, k0, k_end, p.s2d, tid, sp, fast,
                              wide, i,
                              [&] {
-            return wait_bar(smem_u32(&empty[st]), (uint32_t)(((i / p.NS) & 1) ^ 1), abort_flag,
+            return wait_bar_warp(smem_u32(&empty[st]), (uint32_t)(((i / p.NS) & 1) ^ 1), abort_flag,
                             p.status, p.spin_limit);
           })) {
         staged = false;
         break;
       }
       fence_proxy_async();
-      mbar_arrive(smem_u32(&full[st]));
+      mbar_arrive_warp(smem_u32(&full[st]), lane);
     }
     if (staged && warp >= kEpiWarp0) {
       // ===================== epilogue: TMEM -> C =====================
