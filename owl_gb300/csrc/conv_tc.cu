@@ -108,11 +108,13 @@ struct TcParams {
   int T;  // plan: taps of the longest segment
   int n_table;  // taps of all segments
   int sw, su, sv;          // strides along w, u, v
-  int HW, HU, HV, HVR, HP, PS;  // halo rows along w, u; pixels per u-row (= sv * HVR)
-  // Halo rows that some tap reads, for the row table: NHU u rows of the n_ures
-  // residues mod su in ures, n_vres residue rows mod sv in vres (a 1x1 kernel of
-  // stride 2 reads a quarter of its footprint); nrows in all.
+  // Halo: HW x HU input rows, of which the stage holds those that some tap reads:
+  // NHU u rows, of the n_ures residues mod su in ures, each as n_vres rows of HVR
+  // pixels, the residues mod sv in vres (a 1x1 kernel of stride 2 reads a quarter of
+  // its footprint); nrows rows and HP pixels in all, PS with padding.
+  int HW, HU, HVR, HP, PS;
   int n_ures, n_vres, NHU, nrows;
+  unsigned sbo;  // bytes from a tile's row (u) to the next in the stage
   unsigned char ures[8], vres[8];
   int n_tiles;
   int NCT, n_groups;  // output-channel tiles per CTA tile (1 or 2), and tile groups
@@ -221,46 +223,13 @@ using stage::pack_bf16;
 using stage::pack_rest;
 using stage::to_tf32;
 
-// One producer warp's staging of a channel block in whole 32-byte chunks: the
-// rows of the row table from `first` on, every kProducerWarps * ROWS, ROWS rows
-// of STEPS loads per lane a round (ROWS * STEPS <= 6 loads in flight).  What a
-// slot needs is constant for the lane or advances by an add.  `ready` waits for
-// the stage, after the first round's loads are issued.
-template <int KIND, int STEPS, int ROWS, class Ready>
-__device__ __forceinline__ bool stage_lanes(const TcParams &p, const int4 *rows, int first,
-                                            const stage::Lane &L, int steps, int n_lane,
-                                            const float *xt, int iw0, int iu0, int iv0,
-                                            uint8_t *dst, Ready ready) {
-  const long long pix = (long long)p.sv * p.xsv * p.Cin;  // floats between row pixels
-  bool waited = false;
-  for (int r0 = first * ROWS; r0 < p.nrows; r0 += kProducerWarps * ROWS) {
-    // (steps > STEPS only in the one-row form: a row in several rounds)
-    for (int k = 0; k < steps; k += STEPS) {
-      float v[ROWS][STEPS][8];
-#pragma unroll
-      for (int a = 0; a < ROWS; ++a) {
-        const int4 e = rows[min(r0 + a, p.nrows - 1)];
-        const int hw = e.z & 0xffff, hu = e.z >> 16;
-        const bool ok = r0 + a < p.nrows && (unsigned)(iw0 + hw) < (unsigned)p.IW &&
-                        (unsigned)(iu0 + hu) < (unsigned)p.IU && L.on;
-        stage::lane_load<STEPS>(xt + (long long)e.x * p.Cin + (long long)k * L.di * pix,
-                                L.di * pix, iv0 + e.w + (L.i0 + k * L.di) * p.sv, L.di * p.sv,
-                                ok ? (unsigned)p.IV : 0u, steps - k, v[a]);
-      }
-      if (!waited) {
-        if (!ready()) return false;
-        waited = true;
-      }
-#pragma unroll
-      for (int a = 0; a < ROWS; ++a) {
-        const int row = rows[min(r0 + a, p.nrows - 1)].y;
-        stage::lane_store<KIND, STEPS>(dst + (uint32_t)(row + k * L.di) * 16u,
-                                       (uint32_t)L.di * 16u, p.halo_bytes,
-                                       r0 + a < p.nrows ? n_lane - k : 0, v[a]);
-      }
-    }
-  }
-  return waited || ready();
+// Row r of the stage: residue row hr of input row (hw, hu) of the tile.
+__device__ __forceinline__ void halo_row(const TcParams &p, int r, int &hr, int &hu, int &hw) {
+  const int t = r / p.n_vres;
+  hr = p.vres[r - t * p.n_vres];
+  hw = t / p.NHU;
+  const int hi = t - hw * p.NHU, uq = hi / p.n_ures;
+  hu = uq * p.su + p.ures[hi - uq * p.n_ures];
 }
 
 // MULTI: the launch has several segments (else segment 0 only, read at a
@@ -280,7 +249,10 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
   constexpr bool SEP = (KIND == K_BF16X3);
   extern __shared__ __align__(1024) uint8_t smem[];
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (the shuffle shows the compiler that a warp takes one side of the role branches
+  // as a whole: the MMA loop keeps its descriptors in uniform registers)
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
   uint8_t *halo = smem;
   uint8_t *bring = smem + (size_t)p.NH * PARTS * p.halo_bytes;
   uint64_t *bars = reinterpret_cast<uint64_t *>(bring + (size_t)p.NB * PARTS * p.b_bytes);
@@ -294,50 +266,65 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   uint32_t *tap_off = tmem_slot + 2;  // per-tap start pixel in the halo (16-byte units)
-  // LANES, the rows to stage: {pixel offset from the tile's first input pixel,
-  // first pixel in the stage, hw | hu << 16, hr}
-  int4 *rows = reinterpret_cast<int4 *>((reinterpret_cast<uintptr_t>(tap_off + p.n_table) + 15) &
-                                        ~(uintptr_t)15);
-  if (LANES) {
-    for (int i = threadIdx.x; i < p.nrows; i += blockDim.x) {
-      const int q = i / p.n_vres, hr = p.vres[i - q * p.n_vres];
-      const int hw = q / p.NHU, hi = q - hw * p.NHU;
-      const int uq = hi / p.n_ures, hu = uq * p.su + p.ures[hi - uq * p.n_ures];
-      rows[i] = make_int4((int)(hw * p.xsw + hu * p.xsu + hr * p.xsv),
-                          ((hw * p.HU + hu) * p.sv + hr) * p.HVR, hw | hu << 16, hr);
-    }
-  }
-
-  // tap offsets of every segment, segment c's at tap_off[seg[c].toff ..]
-  for (int c = 0; c < (MULTI ? p.nseg : 1); ++c) {
-    const Seg &sg = p.seg[c];
-    for (int tap = threadIdx.x; tap < sg.T; tap += blockDim.x) {
-      const int kv = tap % sg.KV, ku = (tap / sg.KV) % sg.KU, kw = tap / (sg.KV * sg.KU);
-      const int qv = kv * sg.dv;
-      tap_off[sg.toff + tap] = (uint32_t)((kw * sg.dw * p.HU + ku * sg.du) * p.HV +
-                                          (qv % p.sv) * p.HVR + qv / p.sv);
-    }
-  }
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < p.NH; ++i) {
-      mbar_init(smem_u32(&halo_full[i]), kProducerWarps);
-      mbar_init(smem_u32(&halo_empty[i]), 1);
-    }
-    for (int i = 0; i < p.NB; ++i) {
-      mbar_init(smem_u32(&b_full[i]), 1);
-      mbar_init(smem_u32(&b_empty[i]), 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&acc_full[i]), 1);
-      mbar_init(smem_u32(&acc_empty[i]), 128);
-    }
-    mbar_init(smem_u32(drain), 1);
-    *abort_flag = 0;
-    fence_barrier_init();
-  }
+  // LANES: where the stage's pixels lie, {offset in floats from the tile's first input
+  // pixel, position}, and one past the end that is outside any bounds
+  int2 *ptab = reinterpret_cast<int2 *>((reinterpret_cast<uintptr_t>(tap_off + p.n_table) + 7) &
+                                        ~(uintptr_t)7);
+  // The setup is a call's latency, so its parts run side by side: the barriers and
+  // TMEM in the MMA warp, the tap table in the epilogue's, the pixel table in the rest.
+  // (Quotients of fewer than 2^21 by reciprocals, which are shorter than divisions.)
+  auto quot = [](int a, float r) { return (int)(((float)a + 0.5f) * r); };
   if (warp == kMmaWarp) {
+    if (lane == 0) {
+      for (int i = 0; i < p.NH; ++i) {
+        mbar_init(smem_u32(&halo_full[i]), kProducerWarps);
+        mbar_init(smem_u32(&halo_empty[i]), 1);
+      }
+      for (int i = 0; i < p.NB; ++i) {
+        mbar_init(smem_u32(&b_full[i]), 1);
+        mbar_init(smem_u32(&b_empty[i]), 1);
+      }
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(smem_u32(&acc_full[i]), 1);
+        mbar_init(smem_u32(&acc_empty[i]), 128);
+      }
+      mbar_init(smem_u32(drain), 1);
+      *abort_flag = 0;
+      fence_barrier_init();
+    }
+    __syncwarp();
     tmem_alloc(smem_u32(tmem_slot), p.tmem_cols);
     tmem_relinquish();
+  } else if (warp >= kEpiWarp0) {
+    // tap offsets of every segment, segment c's at tap_off[seg[c].toff ..]
+    const float r_su = __frcp_rn((float)p.su), r_sv = __frcp_rn((float)p.sv);
+    for (int c = 0; c < (MULTI ? p.nseg : 1); ++c) {
+      const Seg &sg = p.seg[c];
+      const float r_kv = __frcp_rn((float)sg.KV), r_ku = __frcp_rn((float)sg.KU);
+      for (int tap = threadIdx.x - kEpiWarp0 * 32; tap < sg.T; tap += kThreads - kEpiWarp0 * 32) {
+        const int tu = quot(tap, r_kv), kv = tap - tu * sg.KV;
+        const int kw = quot(tu, r_ku), ku = tu - kw * sg.KU;
+        const int qu = ku * sg.du, qv = kv * sg.dv, iu = quot(qu, r_su), iv = quot(qv, r_sv);
+        int hu = iu * p.n_ures, hv = 0;
+        for (int i = 0; i < p.n_ures; ++i) hu += p.ures[i] < qu - iu * p.su;
+        for (int i = 0; i < p.n_vres; ++i) hv += p.vres[i] < qv - iv * p.sv;
+        tap_off[sg.toff + tap] =
+            (uint32_t)(((kw * sg.dw * p.NHU + hu) * p.n_vres + hv) * p.HVR + iv);
+      }
+    }
+  } else if (LANES) {
+    const float r_hvr = __frcp_rn((float)p.HVR), r_nv = __frcp_rn((float)p.n_vres),
+                r_nhu = __frcp_rn((float)p.NHU), r_nu = __frcp_rn((float)p.n_ures);
+    for (int i = threadIdx.x - 32; i < p.HP; i += (kEpiWarp0 - 1) * 32) {
+      const int row = quot(i, r_hvr), t = quot(row, r_nv);
+      const int hr = p.vres[row - t * p.n_vres] + (i - row * p.HVR) * p.sv;
+      const int hw = quot(t, r_nhu), hi = t - hw * p.NHU, uq = quot(hi, r_nu);
+      const int hu = uq * p.su + p.ures[hi - uq * p.n_ures];
+      ptab[i] = make_int2((int)((hw * p.xsw + hu * p.xsu + hr * p.xsv) * p.Cin),
+                          (int)(stage::position(hr, hu, hw) | stage::kGuard));
+    }
+    if (threadIdx.x == 32)
+      ptab[p.HP] = make_int2(0, (int)(stage::position(stage::kMaxV + 1, 0, 0) | stage::kGuard));
   }
   tc_fence_before();
   __syncthreads();
@@ -347,48 +334,85 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
   const int pidx = producer_index(warp);
   if (LANES && pidx >= 0) {
     // ===================== halo producers, whole chunks =====================
+    // A lane keeps one 32-byte chunk of the channel block and takes every
+    // lanes/chunks-th pixel of the halo, whose place comes from the table, kB a
+    // batch.  Two batches are in registers, across stages and tiles: the loads of
+    // one are in flight while the other is converted and stored.
     if constexpr (LANES) {
-      const stage::Lane L(p.NCH, lane);
-      const int steps = (p.HVR + L.di - 1) / L.di;
-      const int n_lane = L.on ? (p.HVR - L.i0 + L.di - 1) / L.di : 0;  // the lane's pixels
-      const uint32_t lane_off = (uint32_t)L.j * (uint32_t)p.PS * 16u + (uint32_t)L.i0 * 16u;
-      int hs = 0, sc = 0;
+      constexpr int kB = 4;
+      const int lg = 32 - __clz(p.NCH - 1);  // (clz(0) = 32)
+      const int id = pidx * 32 + lane, j = id & ((1 << lg) - 1);
+      const int px = id >> lg, dpx = (kProducerWarps * 32) >> lg;
+      const int batches = (p.HP + kB * dpx - 1) / (kB * dpx);  // of a stage
+      const uint32_t lane_off = (uint32_t)(j * p.PS + px) * 16u;
+      const int n_px = j < p.NCH ? p.HP - px : 0;
+      // the next batch to load: batch lb of channel block lc of tile t
+      long long t = blockIdx.x;
+      int lb = 0, lc = 0, sc = 0;
+      const float *xt = nullptr;
+      unsigned lo = 0, hi = 0;
+      auto tile_begin = [&] {
+        if (t < p.total_tiles) {
+          sc = MULTI ? seg_of(p, t, sc) : 0;
+          const Tile tl = decode_tile(p, t, sc);
+          const int iw0 = tl.ow * p.sw - p.seg[sc].pw, iu0 = tl.u0 * p.su - p.seg[sc].pu,
+                    iv0 = tl.v0 * p.sv - p.seg[sc].pv;
+          xt = p.x + ((long long)tl.b * p.xsb + (long long)iw0 * p.xsw + (long long)iu0 * p.xsu +
+                      (long long)iv0 * p.xsv) * p.Cin + j * EPC;
+          unsigned l, h;
+          stage::field(iv0, p.IV, stage::kMaxV, lo, hi);
+          stage::field(iu0, p.IU, stage::kMaxU, l, h);
+          lo |= l << 11;
+          hi |= h << 11;
+          stage::field(iw0, p.IW, stage::kMaxW, l, h);
+          lo |= l << 22;
+          hi |= h << 22;
+        } else {
+          lo = stage::kMaxV;  // nothing left to load
+          hi = 0;
+        }
+      };
+      auto load = [&](float(&v)[kB][8]) {
+        // (chunks past the channels, of a ragged last block, are zeros)
+        const bool real = lc * p.CPB + j * EPC < p.Cin;
+        stage::table_load<kB>(ptab, px + lb * kB * dpx, dpx, p.HP, xt + lc * p.CPB,
+                              real ? lo : (unsigned)stage::kMaxV, real ? hi : 0u, v);
+        if (++lb == batches) {
+          lb = 0;
+          if (++lc == p.NCB) {
+            lc = 0;
+            t += gridDim.x;
+            tile_begin();
+          }
+        }
+      };
+      int hs = 0, sb = 0;  // stage and batch to store
       uint32_t hph = 1;
-      bool ok = true;
-      for (long long t = blockIdx.x; ok && t < p.total_tiles; t += gridDim.x) {
-        sc = MULTI ? seg_of(p, t, sc) : 0;
-        const Tile tl = decode_tile(p, t, sc);
-        const int iw0 = tl.ow * p.sw - p.seg[sc].pw, iu0 = tl.u0 * p.su - p.seg[sc].pu,
-                  iv0 = tl.v0 * p.sv - p.seg[sc].pv;
-        const float *xt = p.x + ((long long)tl.b * p.xsb + (long long)iw0 * p.xsw +
-                                 (long long)iu0 * p.xsu +
-                                 (long long)(iv0 + L.i0 * p.sv) * p.xsv) * p.Cin + L.j * EPC;
-        for (int cb = 0; cb < p.NCB; ++cb, xt += p.CPB) {
-          // chunks past the channels (a ragged last block) are zeros
-          stage::Lane Lb = L;
-          const bool real = (cb * p.CPB + L.j * EPC) < p.Cin;
-          auto ready = [&] {
-            return wait_bar_warp(smem_u32(&halo_empty[hs]), hph, abort_flag, p.status, p.spin_limit);
-          };
-          Lb.on = L.on && real;
-          uint8_t *dst = halo + (size_t)hs * PARTS * p.halo_bytes + lane_off;
-          if (steps == 1)
-            ok = stage_lanes<KIND, 1, 6>(p, rows, pidx, Lb, steps, n_lane, xt, iw0, iu0, iv0, dst,
-                                         ready);
-          else if (steps == 2)
-            ok = stage_lanes<KIND, 2, 3>(p, rows, pidx, Lb, steps, n_lane, xt, iw0, iu0, iv0, dst,
-                                         ready);
-          else if (steps == 3)
-            ok = stage_lanes<KIND, 3, 2>(p, rows, pidx, Lb, steps, n_lane, xt, iw0, iu0, iv0, dst,
-                                         ready);
-          else
-            ok = stage_lanes<KIND, 6, 1>(p, rows, pidx, Lb, steps, n_lane, xt, iw0, iu0, iv0, dst,
-                                         ready);
-          if (!ok) break;
+      auto store = [&](const float(&v)[kB][8]) {
+        if (sb == 0 && !wait_bar_warp(smem_u32(&halo_empty[hs]), hph, abort_flag, p.status,
+                                      p.spin_limit))
+          return false;
+        stage::table_store<KIND, kB>(halo + (uint32_t)hs * PARTS * p.halo_bytes + lane_off +
+                                         (uint32_t)(sb * kB * dpx) * 16u,
+                                     dpx, p.halo_bytes, n_px - sb * kB * dpx, v);
+        if (++sb == batches) {
+          sb = 0;
           fence_proxy_async();
           mbar_arrive_warp(smem_u32(&halo_full[hs]), lane);
           if (++hs == p.NH) { hs = 0; hph ^= 1; }
         }
+        return true;
+      };
+      long long left = (p.total_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x * p.NCB * batches;
+      float va[kB][8], vb[kB][8];
+      tile_begin();
+      load(va);
+      load(vb);
+      for (; left > 0; left -= 2) {
+        if (!store(va)) break;
+        load(va);
+        if (left == 1 || !store(vb)) break;
+        load(vb);
       }
     }
   } else if (!LANES && pidx >= 0) {
@@ -398,7 +422,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
     // bounds are checked once and each lane only adds offsets.  A pass takes
     // one or two rows and deals their chunk slots flat over the lanes, up to
     // six loads in flight per lane.
-    const int nrows = p.HW * p.HU * p.sv;
+    const int nrows = p.nrows;
     const int S = p.HVR * p.NCH;  // chunk slots per row
     // rows per producer pass: two when both rows' slots fit 6 per lane
     const int rpp = 2 * S <= 32 * 6 ? 2 : 1;
@@ -424,9 +448,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
           int ivs0, ivs1;
           auto row_setup = [&](int rr, const float *&rp, bool &ok, int &ivs) {
             const int r = r0 + rr;
-            // row -> (w row, u row, residue class)
-            const int hr = r % p.sv, t3 = r / p.sv;
-            const int hu = t3 % p.HU, hw = t3 / p.HU;
+            int hr, hu, hw;
+            halo_row(p, r, hr, hu, hw);
             const int iw = tl.ow * p.sw - pw + hw, iu = tl.u0 * p.su - pu + hu;
             ivs = tl.v0 * p.sv - pv + hr;  // global v of the row's pixel 0
             ok = rr < rpp && r < nrows && iw >= 0 && iw < p.IW && iu >= 0 && iu < p.IU;
@@ -491,8 +514,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
             const int r = r0 + rr;
             if (r >= nrows) break;
             for (int sl = lane + 32 * kSlots; sl < S; sl += 32) {
-              const int hr = r % p.sv, t3 = r / p.sv;
-              const int hu = t3 % p.HU, hw = t3 / p.HU;
+              int hr, hu, hw;
+              halo_row(p, r, hr, hu, hw);
               const int iw = tl.ow * p.sw - pw + hw, iu = tl.u0 * p.su - pu + hu;
               const int hc = sl / p.NCH, j = sl - hc * p.NCH;
               const int iv = tl.v0 * p.sv - pv + hr + hc * p.sv;
@@ -539,7 +562,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
       uint32_t hph = 0, bph = 0;
       int tc = 0;
       const uint32_t halo0 = smem_u32(halo), b0 = smem_u32(bring);
-      const uint32_t a_lbo = (uint32_t)p.PS * 16, a_sbo = (uint32_t)(p.su * p.HV) * 16;
+      const uint32_t a_lbo = (uint32_t)p.PS * 16, a_sbo = p.sbo;
       const uint32_t b_lbo = (uint32_t)p.BN * 16;
       const int ksteps = p.NCH / 2;
       // descriptor increments in 16-byte units
@@ -1044,11 +1067,11 @@ struct PlanSeg {
 };
 
 // What a plan's time is made of, in us (measured on GB300; the choice needs
-// their ratios only): an MMA with one and with two accumulators in turn, and per
-// column of N; a round of the producers' loads; weight bytes and output bytes
-// per us and SM; the hand-off of a weight slot.
+// their ratios only): a tile; an MMA with one and with two accumulators in turn, and per
+// column of N; a stage and a batch of the producers' loads; weight bytes and output
+// bytes per us and SM; the hand-off of a weight slot.
 constexpr double kMma1 = 0.056, kMma2 = 0.0485, kMmaCol = 0.00027;
-constexpr double kRound = 1.15, kWeightRate = 100e3, kStoreRate = 45e3, kSlot = 0.2;
+constexpr double kTile = 0.6, kStage = 0.2, kBatch = 0.25, kWeightRate = 100e3, kStoreRate = 45e3, kSlot = 0.2;
 
 // Choose tile and pipeline sizes; false if no configuration fits.
 //
@@ -1085,7 +1108,7 @@ bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const P
   const int max_tu = std::min(32, max_ou);
 
   // q: the sizes of one configuration; false when it does not fit
-  auto fit = [&](TcParams &q, int nh, int tu, int cb, int nct) {
+  auto fit = [&](TcParams &q, int nh, int tu, int cb, int nct, bool lean = false) {
     q = p;
     q.NH = nh;
     q.TU = tu;
@@ -1101,23 +1124,24 @@ bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const P
     q.HW = (v.KW - 1) * v.dw + 1;
     q.HU = (tu - 1) * v.su + (v.KU - 1) * v.du + 1;
     q.HVR = 8 + ((v.KV - 1) * v.dv) / v.sv;
-    q.HV = v.sv * q.HVR;
-    q.HP = q.HW * q.HU * q.HV;
     q.NHU = q.HU / v.su * q.n_ures;
     for (int i = 0; i < q.n_ures; ++i) q.NHU += q.ures[i] < q.HU % v.su;
     q.nrows = q.HW * q.NHU * q.n_vres;
+    q.HP = q.nrows * q.HVR;
+    q.sbo = (unsigned)(q.n_ures * q.n_vres * q.HVR) * 16u;
     q.PS = q.HP + (((1 - q.HP) % 8) + 8) % 8;  // plane stride = 1 (mod 8) pixels
-    if (q.PS >= 16384 || q.HV >= 16384) return false;
+    if (q.PS >= 16384) return false;
     q.halo_bytes = (unsigned)q.PS * 16u * (unsigned)q.NCH;
     const long long fixed =
-        (long long)q.NH * parts * q.halo_bytes + 512 + 4LL * t_table + 16LL * q.nrows + 16;
+        (long long)q.NH * parts * q.halo_bytes + 512 + 4LL * t_table + 8LL * (q.HP + 2);
     // Shared memory up to the step that leaves 60 KB of the SM's 256 for the L1
-    // cache where three taps per weight slot fit in that: the producers' loads in
-    // flight (up to 55 KB) wait for lines of a smaller one (57.3 us against 53.2
-    // for [64;56;56;128]x[3;3;128;128]).
+    // cache where a third of the taps (three at least) fit a weight slot in that: the
+    // producers' loads in flight (up to 74 KB) wait for lines of a smaller one (57.3
+    // us against 53.2 for [64;56;56;128]x[3;3;128;128]), but 27 taps in threes are
+    // waited for (36 us against 33).
     const long long slot = (long long)parts * q.NCT * q.tile_bytes;
     long long room = kSmemLean - fixed;
-    if (room < 2 * slot * std::min(3, q.T)) room = kSmemMax - fixed;
+    if (!lean && room < 2 * slot * std::min(q.T, std::max(3, q.T / 3))) room = kSmemMax - fixed;
     if (room <= 0) return false;
     // the most taps per weight slot (fewer barrier polls between MMAs) that
     // leaves at least two slots
@@ -1154,19 +1178,18 @@ bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const P
     const double mmas = taps * q.NCB * (q.NCH / 2) * q.NCT * (parts == 2 ? 3 : 1);
     const double mma = mmas * std::max(q.NCT * parts == 1 ? kMma1 : kMma2, kMmaCol * q.TN) +
                        q.NCB * std::max(1.0, taps / q.TPS) * kSlot;
-    // a row of the halo in 32-lane loads, six loads a lane and round
+    // the producers' batches of four chunks a lane
     int chunks = 1;
     while (chunks < q.NCH) chunks *= 2;
-    const int steps = (q.HVR * chunks + 31) / 32;
-    const int per_round = kProducerWarps * std::max(1, 6 / steps);
-    const double stage = kRound * ((q.nrows + per_round - 1) / per_round) * ((steps + 5) / 6) *
-                         (parts == 2 ? 1.3 : 1.0);
+    const int lanes = kProducerWarps * 32 * 4;
+    const double stage = kStage + kBatch * ((q.HP * chunks + lanes - 1) / lanes) *
+                                      (parts == 2 ? 1.3 : 1.0);
     const double weights = taps * q.NCB * q.tile_bytes * (parts * q.NCT) / kWeightRate;
     const double store = (double)q.TN * std::min(v.Cout, q.BN * q.NCT) * 4 / kStoreRate;
     const double fill = q.NCB * stage;
     const double work = std::max(weights, q.NH >= 2 ? std::max(mma, fill) : mma + fill);
-    return q.nbuf == 2 ? stage + rounds * std::max(work, store) + store
-                       : stage + rounds * (work + store);
+    return q.nbuf == 2 ? stage + rounds * (std::max(work, store) + kTile) + store
+                       : stage + rounds * (work + store + kTile);
   };
 
   // channel blocks, the least padded first (a block's own cost counts as half a
@@ -1181,10 +1204,12 @@ bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const P
     return n * (cb + 16);
   };
   std::stable_sort(cbs, cbs + ncb, [&](int a, int b) { return padded(a) < padded(b); });
-  // the first of them that fits with two halo stages (staging overlaps the MMAs)
-  // and the tallest tile, 32-byte ones with one half as tall: a tall tile's fewer
-  // MMAs outweigh a wide block ([64;56;56;128]x[3;3;128;128] at rate 2 in split
-  // BF16 takes 155 us with 128 bytes and TU <= 20, 122 with 64 and TU = 28).
+  // the first of them that fits the leaner shared memory with two halo stages
+  // (staging overlaps the MMAs), the tallest tile and its co tiles, 32-byte ones with
+  // one half as tall: a tall tile's fewer MMAs outweigh a wide block
+  // ([64;56;56;128]x[3;3;128;128] at rate 2 in split BF16 takes 155 us with 128 bytes
+  // and TU <= 20, 122 with 64 and TU = 28), and so do the loads in flight
+  // ([64;28;28;256]x[3;3;256;256] at stride 2: 39 us with 128 bytes, 31 with 64).
   // Else the first that fits with the lowest tile, then with one stage.
   TcParams q;
   int nh = 0, cb = 0;
@@ -1192,7 +1217,8 @@ bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const P
     for (int i = 0; i < ncb && !cb; ++i) {
       const int tall = form == 0 ? max_tu : (form == 1 ? std::min(16, max_tu) : 2);
       if (form == 0 && cbs[i] == 32 && all > 32) continue;
-      if (fit(q, form < 3 ? 2 : 1, tall, cbs[i], 1)) {
+      const int nct = form == 0 && tall <= 16 ? std::min(2, p.n_tiles) : 1;
+      if (fit(q, form < 3 ? 2 : 1, tall, cbs[i], nct, form == 0)) {
         nh = form < 3 ? 2 : 1;
         cb = cbs[i];
       }
@@ -1529,12 +1555,15 @@ int run_segs(int prec, int nseg_in, const SegSpec *sp, bool bwd_input, int Ci, i
     }
   }
   const size_t smem = (size_t)p.NH * parts * p.halo_bytes + (size_t)p.NB * parts * p.b_bytes +
-                      (2 * p.NH + 2 * p.NB + 5) * 8 + 16 + 4 * (size_t)t_table + 16 +
-                      16 * (size_t)p.nrows;
+                      (2 * p.NH + 2 * p.NB + 5) * 8 + 16 + 4 * (size_t)t_table +
+                      8 * (size_t)(p.HP + 2);
   const bool multi = p.nseg > 1;
   const bool pdl = prep && !build_cached;
-  // (the row table's pixel offsets are 32-bit)
-  const bool lanes = p.vec_in == 2 && p.HW * p.xsw + p.HU * p.xsu + p.HV * p.xsv < (1LL << 31);
+  // (the table's offsets are 32-bit, its positions' fields 10, 10 and 9 bits)
+  const long long span_v = (long long)p.HVR * p.sv;
+  const bool lanes = p.vec_in == 2 && span_v <= stage::kMaxV && p.HU <= stage::kMaxU &&
+                     p.HW <= stage::kMaxW &&
+                     (p.HW * p.xsw + p.HU * p.xsu + span_v * p.xsv) * p.Cin < (1LL << 31);
   if (kind == K_TF32)
     rc = multi ? launch<K_TF32, true, false>(p, smem, s, pdl)
                : launch<K_TF32, false, false>(p, smem, s, pdl);

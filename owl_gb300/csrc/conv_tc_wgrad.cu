@@ -149,7 +149,10 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
   // and dY may be its output) before any global access
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (the shuffle shows the compiler that a warp takes one side of the role branches
+  // as a whole: the MMA loop keeps its descriptors in uniform registers)
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
   const int YPL = p.BN * EB / 16;
 
   // ---- work unit of this CTA ----

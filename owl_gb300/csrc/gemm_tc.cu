@@ -312,7 +312,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
   // launched with launch_pdl: the operands may be the previous kernel's output
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (the shuffle shows the compiler that a warp takes one side of the role branches
+  // as a whole: the MMA loop keeps its descriptors in uniform registers)
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
   const long long m0 = (long long)blockIdx.x * kBM, n0 = (long long)blockIdx.y * p.BN;
   const long long k_begin = (long long)blockIdx.z * p.kps;
   const long long k_end = min(p.K, k_begin + p.kps);

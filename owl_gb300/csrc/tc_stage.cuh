@@ -226,51 +226,12 @@ load_vec<EPC>(src, vec, vb[q]);
   }
 }
 
-// ---- staging whole 32-byte chunks with little arithmetic per slot -----------
-// (32-byte aligned arrays, channels a multiple of 8.)  A lane keeps one chunk of
-// every row (lane mod the chunks, rounded up to a power of two) and takes pixels
-// i0, i0 + di, ..: what a slot needs is constant for the lane or advances by an
-// add.  Out-of-range pixels load from a row of zeros instead of branching.
+// ---- staging whole 32-byte chunks from a table of a tile's pixels -----------
+// (32-byte aligned arrays, channels a multiple of 8.)  Where a pixel lies relative
+// to its tile is the same for every tile; those outside the array load from a row
+// of zeros instead of branching.
 
 __device__ __align__(32) const float g_zero_chunk[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-
-struct Lane {
-  int j, i0, di;  // chunk, first pixel, pixel step
-  bool on;        // the chunk exists
-  __device__ __forceinline__ Lane(int nch, int lane) {
-    int lg = 0;
-    while ((1 << lg) < nch) ++lg;  // nch <= 32
-    j = lane & ((1 << lg) - 1);
-    i0 = lane >> lg;
-    di = 32 >> lg;
-    on = j < nch;
-  }
-};
-
-// The first n of Q loads of a row (n the same for the warp): the lane's pixels
-// i0 + q*di at src + q*step, in range while (unsigned)(vv + q*vstep) < vlim
-// (vlim 0: a row outside the array).
-template <int Q>
-__device__ __forceinline__ void lane_load(const float *src, long long step, int vv, int vstep,
-                                          unsigned vlim, int n, float (&v)[Q][8]) {
-#pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    if (q < n) ld8((unsigned)vv < vlim ? src : g_zero_chunk, v[q]);
-    src += step;
-    vv += vstep;
-  }
-}
-
-// Convert and store them at dst + q*dstep, those of the `n` pixels that exist.
-template <int KIND, int Q>
-__device__ __forceinline__ void lane_store(uint8_t *dst, uint32_t dstep, uint32_t lo_off, int n,
-                                           const float (&v)[Q][8]) {
-#pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    if (q < n) put_chunk<KIND, 8>(dst, lo_off, v[q]);
-    dst += dstep;
-  }
-}
 
 // A position in a tile as one word, fields v (10 bits), u (10) and w (9) with a guard
 // bit above each: inside the bounds when no field of (position - low) or of (high -
