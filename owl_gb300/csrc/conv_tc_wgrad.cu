@@ -76,6 +76,7 @@ struct WgParams {
   unsigned idesc, tmem_cols;
   unsigned small_off;  // BF16X3: TMEM column of the cross-term accumulators (TG * BN)
   int vec_x, vec_y;
+  int pk_nch;  // PACK: chunk rows of a halo row (a power of two), else 16
   // LANES: floats from a tile's first pixel to the next tile's along v; from there
   // to the next row of tiles; and so on along w and b
   long long x_dv, x_du, x_dw, x_db, y_dv, y_du, y_dw, y_db;
@@ -130,9 +131,23 @@ __device__ __forceinline__ bool poll_bar(uint32_t bar, uint32_t parity, volatile
   return true;
 }
 
+// Pixels from one chunk row of a packed X stage to the next: as many as a halo row
+// has, or the few more that put the 16-byte chunks that eight lanes store together
+// into different banks.
+__host__ __device__ inline int chunk_row(int hvr, int nch) {
+  const int step = 8 / nch > 0 ? 8 / nch : 1;  // nch rows x step pixels
+  while (nch > 1 && (hvr % (2 * step)) != step) ++hvr;
+  return hvr;
+}
+
 // LANES: the operands are staged as whole 32-byte chunks (both arrays 32-byte
 // aligned, their channels multiples of 8), else element by element where needed.
-template <int KIND, bool LANES>
+// PACK: at most 64 input channels, of which an MMA's 128 rows hold
+// those of several taps, ku, ku + su, ..: the X stage keeps, halo row after halo row,
+// `pk` chunk rows of PSR pixels, so that one stride of PSR pixels walks the chunks of
+// a halo row and on into the next one's, the next tap's operand.  With a tap to an
+// MMA, 32 channels used a quarter of each: [4;32;32;32;32]x[3;3;3;32;64] took 77 us.
+template <int KIND, bool LANES, bool PACK>
 __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_constant__ WgParams p) {
   constexpr int EB = (KIND == K_TF32) ? 4 : 2;
   constexpr int EPC = 16 / EB;
@@ -165,7 +180,9 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
   const long long t_end = min(p.total_tiles, t_begin + p.tiles_per_range);
   const int gbeg = p.ordered ? (int)p.gstart[tg] : tg * p.TG;
   const int ntap = p.ordered ? (int)p.gstart[tg + 1] - gbeg : min(p.TG, p.T - gbeg);
+  // (PACK: the first tap of each pack)
   auto tap_of = [&](int i) { return p.ordered ? (int)p.tap_order[gbeg + i] : gbeg + i; };
+  const int pk = p.pk_nch, pk_taps = PACK ? XPL / pk : 1;
 
   // bounding box of this group's tap offsets -> halo extents
   int minw = 1 << 30, minu = 1 << 30, minv = 1 << 30, maxw = -1, maxu = -1, maxv = -1;
@@ -173,7 +190,8 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
     const int t = tap_of(i);
     const int kv = t % p.KV, ku = (t / p.KV) % p.KU, kw = t / (p.KV * p.KU);
     minw = min(minw, kw * p.dw); maxw = max(maxw, kw * p.dw);
-    minu = min(minu, ku * p.du); maxu = max(maxu, ku * p.du);
+    minu = min(minu, ku * p.du);
+    maxu = max(maxu, (PACK ? ku + min(pk_taps - 1, (p.KU - 1 - ku) / p.su) * p.su : ku) * p.du);
     minv = min(minv, kv * p.dv); maxv = max(maxv, kv * p.dv);
   }
   // X halo of a phase-uniform group: input rows and columns of the group's
@@ -182,11 +200,15 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
   // column: 8 consecutive output columns are 8 consecutive stored pixels.
   const int HW = (maxw - minw) / p.sw + 1, HU = p.TU + (maxu - minu) / p.su;
   const int HVR = 8 + (maxv - minv) / p.sv;
+  // PACK: pixels from a chunk row to the next, and from a halo row to the next; else
+  // pixels from one chunk plane to the next, and the halo rows lie in one plane
+  const int PSR = PACK ? chunk_row(HVR, pk) : p.PS, row_px = PACK ? pk * PSR : HVR;
   // X halo rows; when both operand tiles have at most one row per producer
   // warp, each warp stages its X row and dY row together in a single pass
   const int xrows = HW * HU;
+  const int nch = PACK ? pk : XPL;  // chunks of X staged element by element
   const bool paired = xrows <= kProducerWarps && p.TU <= kProducerWarps &&
-                      HVR * XPL <= 32 * 5 && 8 * YPL <= 32 * 4;
+                      HVR * nch <= 32 * 5 && 8 * YPL <= 32 * 4;
 
   uint8_t *xs = smem;
   uint8_t *ys = smem + (size_t)p.NS * PARTS * p.x_bytes;
@@ -202,8 +224,9 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
   for (int i = threadIdx.x; i < ntap; i += blockDim.x) {
     const int tt = tap_of(i);
     const int kv = tt % p.KV, ku = (tt / p.KV) % p.KU, kw = tt / (p.KV * p.KU);
-    tap_off[i] = (uint32_t)((((kw * p.dw - minw) / p.sw) * HU + (ku * p.du - minu) / p.su) * HVR +
-                            (kv * p.dv - minv) / p.sv);
+    tap_off[i] =
+        (uint32_t)((((kw * p.dw - minw) / p.sw) * HU + (ku * p.du - minu) / p.su) * row_px +
+                   (kv * p.dv - minv) / p.sv);
   }
 
   // LANES: where the tile's pixels lie, X's then dY's: {offset in floats from the
@@ -211,10 +234,12 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
   int2 *xtab = reinterpret_cast<int2 *>((reinterpret_cast<uintptr_t>(tap_off + p.TG) + 7) &
                                         ~(uintptr_t)7);
   int2 *ytab = xtab + xrows * HVR + 1;
+  uint16_t *xdst = reinterpret_cast<uint16_t *>(ytab + p.TP + 1);  // PACK: places in the stage
   if (LANES) {
     const int n = xrows * HVR, out = (int)(stage::position(stage::kMaxV + 1, 0, 0) | stage::kGuard);
     for (int i = threadIdx.x; i <= n; i += blockDim.x) {
       const int hv = i % HVR, hu = (i / HVR) % HU, hw = i / (HVR * HU);
+      if (PACK && i < n) xdst[i] = (uint16_t)(i / HVR * row_px + hv);
       xtab[i] =
           i < n ? make_int2((int)((hw * p.sw * p.xsw + hu * p.su * p.xsu + hv * p.sv * p.xsv) * p.Ci),
                             (int)(stage::position(hv * p.sv, hu * p.su, hw * p.sw) | stage::kGuard))
@@ -295,7 +320,7 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
       const int py = id >> lgy, dpy = (kProducerWarps * 32) >> lgy, npy = p.TP;
       const bool onx = jx < nchx, ony = jy < nchy;  // (others load chunk 0 and store nothing)
       const int rounds_x = (npx + dpx - 1) / dpx, rounds_y = (npy + dpy - 1) / dpy;
-      const uint32_t lane_x = (uint32_t)(jx * p.PS + px) * 16u, lane_y = (uint32_t)(jy * p.YPS + py) * 16u;
+      const uint32_t lane_x = (uint32_t)(jx * PSR + (PACK ? 0 : px)) * 16u, lane_y = (uint32_t)(jy * p.YPS + py) * 16u;
       int iw0 = ow * p.sw - p.pw + minw, iu0 = u0 * p.su - p.pu + minu, iv0 = v0 * p.sv - p.pv + minv;
       const float *xt = p.x + ((long long)b * p.xsb + (long long)iw0 * p.xsw + (long long)iu0 * p.xsu +
                                (long long)iv0 * p.xsv) * p.Ci + mb * 128 + (onx ? jx * 8 : 0);
@@ -341,8 +366,12 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
           const int kx = k * dpx * QX, ky = k * dpy * QY;
           uint8_t *yd = ys + (uint32_t)st * PARTS * p.y_bytes + lane_y + (uint32_t)ky * 16u;
           const int ny = ony ? npy - py - ky : 0;
-          stage::table_store<KIND, QX>(xs + (uint32_t)st * PARTS * p.x_bytes + lane_x + (uint32_t)kx * 16u,
-                                       dpx, p.x_bytes, onx ? npx - px - kx : 0, vx);
+          uint8_t *xd = xs + (uint32_t)st * PARTS * p.x_bytes + lane_x;
+          const int nx = onx ? npx - px - kx : 0;
+          if (PACK)
+            stage::table_store_at<KIND, QX>(xd, xdst + px + kx, dpx, p.x_bytes, nx, vx);
+          else
+            stage::table_store<KIND, QX>(xd + (uint32_t)kx * 16u, dpx, p.x_bytes, nx, vx);
           ++k;
           const bool last = k * QX >= rounds_x && k * QY >= rounds_y;  // the tile's last round
           if (last) {
@@ -428,15 +457,15 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
         };
         if (paired) {
           // at most one row of each per warp: both rows in one pass
-          stage::RowSet sx{xd, p.x_bytes, (uint32_t)p.PS * 16, xrows, HVR, XPL, p.Ci - xcb};
-          stage::RowSet sy{yd, p.y_bytes, (uint32_t)p.YPS * 16, p.TU, 8, YPL, p.Co - ycb};
+          stage::RowSet sx{xd, p.x_bytes, (uint32_t)PSR * 16, xrows, HVR, row_px, nch, p.Ci - xcb};
+          stage::RowSet sy{yd, p.y_bytes, (uint32_t)p.YPS * 16, p.TU, 8, 8, YPL, p.Co - ycb};
           stage::stage_rows2<KIND, EPC, 5, 4>(sx, xrow, sy, yrow, min(p.vec_x, p.vec_y),
                                               pidx, kProducerWarps, lane);
         } else {
-          stage::stage_rows<KIND, EPC, 6>(xd, p.x_bytes, (uint32_t)p.PS * 16, xrows, HVR, XPL,
+          stage::stage_rows<KIND, EPC, 6>(xd, p.x_bytes, (uint32_t)PSR * 16, xrows, HVR, row_px, nch,
                                           p.Ci - xcb, p.vec_x, pidx, kProducerWarps, lane,
                                           xrow);
-          stage::stage_rows<KIND, EPC, 4>(yd, p.y_bytes, (uint32_t)p.YPS * 16, p.TU, 8, YPL,
+          stage::stage_rows<KIND, EPC, 4>(yd, p.y_bytes, (uint32_t)p.YPS * 16, p.TU, 8, 8, YPL,
                                           p.Co - ycb, p.vec_y, pidx, kProducerWarps, lane,
                                           yrow);
         }
@@ -451,11 +480,14 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
       // warps take every kEpiParts-th 16 columns)
       const int q = warp & 3;
       int mine = (warp - kEpiWarp0) >> 2;
-      const int ci = mb * 128 + q * 32 + lane;
+      const int row = q * 32 + lane, pt = PACK ? row / (pk * 8) : 0;  // tap of the pack
+      const int ci = PACK ? row - pt * pk * 8 : mb * 128 + row;
       if (wait_bar(smem_u32(acc_full), 0, abort_flag, p.status, p.spin_limit)) {
         tc_fence_after();
         for (int i = 0; i < ntap; ++i) {
-          const int tt = tap_of(i);
+          const int tt = tap_of(i) + pt * p.su * p.KV;
+          const bool real =
+              ci < p.Ci && (!PACK || tap_of(i) / p.KV % p.KU + pt * p.su < p.KU);
           float *out = p.out + (((long long)r * p.T + tt) * p.Ci + ci) * p.Co + nb * p.BN;
           const uint32_t tcol = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(i * p.BN);
           for (int c0 = 0; c0 < p.BN; c0 += 16) {
@@ -476,7 +508,7 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
             } else {
               tmem_ld_wait();
             }
-            if (ci < p.Ci) {
+            if (real) {
               const int n0 = nb * p.BN + c0;
               if (p.vec_y == 2 && n0 + 16 <= p.Co && ((uintptr_t)(out + c0) % 32 == 0)) {
                 stage::st8(out + c0, rr);
@@ -503,12 +535,12 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
     {
       const uint32_t lead = elect_one();
       const uint32_t x0 = smem_u32(xs), y0 = smem_u32(ys);
-      const uint32_t a_lbo = (uint32_t)HVR * 16, a_sbo = (uint32_t)p.PS * 16;
+      const uint32_t a_lbo = (uint32_t)row_px * 16, a_sbo = (uint32_t)PSR * 16;
       const uint32_t b_lbo = 128, b_sbo = (uint32_t)p.YPS * 16;
       const uint32_t xlo16 = p.x_bytes >> 4, ylo16 = p.y_bytes >> 4;
       // per K step: 16 pixels = two halo rows further into the X halo, 16
       // pixels further into the dY tile (16-byte units)
-      const uint32_t xk16 = (uint32_t)(KSTEP_PIX / 8) * (uint32_t)HVR;
+      const uint32_t xk16 = (uint32_t)(KSTEP_PIX / 8) * (uint32_t)row_px;
       const int nks = p.TP / KSTEP_PIX;
       // up to four taps' A offsets in registers (the common tap groups)
       const bool few = ntap <= 4;
@@ -631,17 +663,17 @@ int *status_word() {
   return p[dev];
 }
 
-template <int KIND, bool LANES>
+template <int KIND, bool LANES, bool PACK>
 int launch(const WgParams &p, size_t smem, int grid, cudaStream_t s) {
   static bool attr[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr[dev]) {
-    OWL_CUDA(cudaFuncSetAttribute(wgrad_tc_kernel<KIND, LANES>,
+    OWL_CUDA(cudaFuncSetAttribute(wgrad_tc_kernel<KIND, LANES, PACK>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
     attr[dev] = true;
   }
-  cudaError_t e = launch_pdl(wgrad_tc_kernel<KIND, LANES>, dim3(grid), dim3(kThreads), smem, s,
+  cudaError_t e = launch_pdl(wgrad_tc_kernel<KIND, LANES, PACK>, dim3(grid), dim3(kThreads), smem, s,
                              p);
   if (e == cudaSuccess) e = cudaGetLastError();
   note_launch();
@@ -714,6 +746,40 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
     cls_begin[n_cls] = p.T;
     for (int i = 0; i < p.T; ++i) p.tap_order[i] = (unsigned short)order[i];
   }
+  // 1: 16-byte vector loads; 2: 32-byte aligned chunks (one load per chunk)
+  auto vec_of = [](const float *a, long long ch) {
+    if ((uintptr_t)a % 32 == 0 && ch % 8 == 0) return 2;
+    return ((uintptr_t)a % 16 == 0 && ch % 4 == 0) ? 1 : 0;
+  };
+  p.vec_x = vec_of(x, p.Ci);
+  p.vec_y = vec_of(dy, p.Co);
+  // (the tables' offsets are 32-bit, their positions' fields 10, 10 and 9 bits; tiles
+  // have at most 16 rows)
+  const long long fw = (long long)p.KW * p.dw + p.sw, fu = 16LL * p.su + (long long)p.KU * p.du,
+                  fv = 8LL * p.sv + (long long)p.KV * p.dv;
+  const bool lanes = p.vec_x == 2 && p.vec_y == 2 && fw <= stage::kMaxW && fu <= stage::kMaxU &&
+                     fv <= stage::kMaxV &&
+                     (fw * p.xsw + fu * p.xsu + fv * p.xsv) * p.Ci < (1LL << 31) &&
+                     (16 * p.ysu + 8 * p.ysv) * p.Co < (1LL << 31);
+  // Packs of taps along u where the channels leave room for them in an MMA's 128
+  // rows; from here on a "tap" of a group is a pack.
+  p.pk_nch = 16;
+  int n_ent = p.T;
+  if (p.ordered && p.Ci <= 64 && p.du == 1 && p.KU > p.su) {
+    p.pk_nch = 1;
+    while (p.pk_nch * 8 < p.Ci) p.pk_nch *= 2;
+    const int taps = 16 / p.pk_nch;
+    int n = 0, begin = 0;
+    for (int c = 0; c < n_cls; ++c) {
+      const int end = cls_begin[c + 1];
+      cls_begin[c] = n;
+      for (int i = begin; i < end; ++i)
+        if (order[i] / p.KV % p.KU / p.su % taps == 0) p.tap_order[n++] = (unsigned short)order[i];
+      begin = end;
+    }
+    cls_begin[n_cls] = n_ent = n;
+  }
+  const bool pack = p.pk_nch < 16;
   // Groups of at most tg taps: each class split into the fewest groups,
   // sizes as even as possible.  Returns the number of groups and fills
   // gstart (ordered) or sets the contiguous split (unordered).
@@ -734,7 +800,7 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
         widest = std::max(widest, sz);
       }
     }
-    p.gstart[n] = (unsigned short)p.T;
+    p.gstart[n] = (unsigned short)n_ent;
     p.TG = widest;
     return n;
   };
@@ -763,7 +829,7 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
   double least = -1;
   int best_tg = 0, last_n = -1;
   WgParams best = p;
-  for (int tg = std::min(p.T, 16); tg >= 1; --tg) {
+  for (int tg = std::min(n_ent, 16); tg >= 1; --tg) {
     const int n = p.n_tg = make_groups(tg);
     if (n == last_n) continue;
     last_n = n;
@@ -777,7 +843,9 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
         const int t = p.ordered ? p.tap_order[i] : i;
         const int kv = t % p.KV, ku = (t / p.KV) % p.KU, kw = t / (p.KV * p.KU);
         mnw = std::min(mnw, kw * p.dw); mxw = std::max(mxw, kw * p.dw);
-        mnu = std::min(mnu, ku * p.du); mxu = std::max(mxu, ku * p.du);
+        mnu = std::min(mnu, ku * p.du);
+        mxu = std::max(
+            mxu, (pack ? ku + std::min(16 / p.pk_nch - 1, (p.KU - 1 - ku) / p.su) * p.su : ku) * p.du);
         mnv = std::min(mnv, kv * p.dv); mxv = std::max(mxv, kv * p.dv);
       }
       const Halo h{(mxw - mnw) / p.sw + 1, (mxu - mnu) / p.su, (mxv - mnv) / p.sv};
@@ -800,20 +868,28 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
       last_bn = p.BN;
       for (int ti = 0; ti < ntu; ++ti) {
         const int tu = tus[ti];
-        int HP = 0;
-        for (int i = 0; i < nh; ++i)
-          HP = std::max(HP, halo[i].w * (tu + halo[i].u) * (8 + halo[i].v));
+        int HP = 0, packed = 0;  // pixels of the largest halo; PACK: of its stage
+        for (int i = 0; i < nh; ++i) {
+          const int hvr = 8 + halo[i].v, hu = tu + halo[i].u;
+          HP = std::max(HP, halo[i].w * hu * hvr);
+          // (an MMA reads on past the last halo row, into rows of no tap)
+          if (pack)
+            packed = std::max(packed, (halo[i].w * hu + 16 / p.pk_nch - 1) * p.pk_nch *
+                                              chunk_row(hvr, p.pk_nch) + 8);
+        }
         p.TU = tu;
         p.TP = tu * 8;
         p.YPS = p.TP + 1;
         p.PS = HP + (((1 - HP) % 8) + 8) % 8;
         if (p.PS >= 16384) continue;
-        p.x_bytes = (unsigned)(128 * EB / 16) * (unsigned)p.PS * 16u;
+        if (packed >= 16384 || (packed > 0 && HP >= 65536)) continue;
+        p.x_bytes = pack ? (unsigned)((packed + 15) / 16 * 16) * 16u
+                         : (unsigned)(128 * EB / 16) * (unsigned)p.PS * 16u;
         p.y_bytes = (unsigned)(p.BN * EB / 16) * (unsigned)p.YPS * 16u;
         p.NS = 2;
         p.n_tab = HP + p.TP;
         const size_t need = (size_t)p.NS * parts * (p.x_bytes + p.y_bytes) + 256 +
-                            8 * (size_t)(p.n_tab + 3);
+                            8 * (size_t)(p.n_tab + 3) + 2 * (size_t)p.n_tab;
         if (need > (size_t)kSmemMax) continue;
         p.u_tiles = (p.OU + tu - 1) / tu;
         p.v_tiles = (p.OV + 7) / 8;
@@ -844,13 +920,6 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
   uint32_t idesc = instr_desc(kind == K_TF32 ? 2u : 1u, (uint32_t)p.BN);
   idesc |= (1u << 15) | (1u << 16);  // A and B MN-major
   p.idesc = idesc;
-  // 1: 16-byte vector loads; 2: 32-byte aligned chunks (one load per chunk)
-  auto vec_of = [](const float *a, long long ch) {
-    if ((uintptr_t)a % 32 == 0 && ch % 8 == 0) return 2;
-    return ((uintptr_t)a % 16 == 0 && ch % 4 == 0) ? 1 : 0;
-  };
-  p.vec_x = vec_of(x, p.Ci);
-  p.vec_y = vec_of(dy, p.Co);
   p.spin_limit = wait_limit();
   p.status = status_word();
   if (!p.status) {
@@ -868,17 +937,9 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
   }
   const size_t smem =
       (size_t)p.NS * parts * (p.x_bytes + p.y_bytes) + (2 * p.NS + 2) * 8 + 16 + 4 * (size_t)p.TG +
-      8 * (size_t)(p.n_tab + 3);
+      8 * (size_t)(p.n_tab + 3) + 2 * (size_t)p.n_tab;
   const int grid = (int)(units * p.R);
   int rc;
-  // (the tables' offsets are 32-bit, their positions' fields 10, 10 and 9 bits)
-  const long long fw = (long long)p.KW * p.dw + p.sw,
-                  fu = (long long)p.TU * p.su + (long long)p.KU * p.du,
-                  fv = 8LL * p.sv + (long long)p.KV * p.dv;
-  const bool lanes = p.vec_x == 2 && p.vec_y == 2 && fw <= stage::kMaxW && fu <= stage::kMaxU &&
-                     fv <= stage::kMaxV &&
-                     (fw * p.xsw + fu * p.xsu + fv * p.xsv) * p.Ci < (1LL << 31) &&
-                     (p.TU * p.ysu + 8 * p.ysv) * p.Co < (1LL << 31);
   p.x_dv = 8LL * p.sv * p.xsv * p.Ci;
   p.x_du = (long long)p.TU * p.su * p.xsu * p.Ci - p.v_tiles * p.x_dv;
   p.x_dw = p.sw * p.xsw * p.Ci - (long long)p.u_tiles * p.TU * p.su * p.xsu * p.Ci;
@@ -888,9 +949,15 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
   p.y_dw = p.ysw * p.Co - (long long)p.u_tiles * p.TU * p.ysu * p.Co;
   p.y_db = p.ysb * p.Co - (long long)p.OW * p.ysw * p.Co;
   if (kind == K_BF16X3)
-    rc = lanes ? launch<K_BF16X3, true>(p, smem, grid, s) : launch<K_BF16X3, false>(p, smem, grid, s);
+    rc = lanes ? (pack ? launch<K_BF16X3, true, true>(p, smem, grid, s)
+                       : launch<K_BF16X3, true, false>(p, smem, grid, s))
+               : (pack ? launch<K_BF16X3, false, true>(p, smem, grid, s)
+                       : launch<K_BF16X3, false, false>(p, smem, grid, s));
   else
-    rc = lanes ? launch<K_BF16, true>(p, smem, grid, s) : launch<K_BF16, false>(p, smem, grid, s);
+    rc = lanes ? (pack ? launch<K_BF16, true, true>(p, smem, grid, s)
+                       : launch<K_BF16, true, false>(p, smem, grid, s))
+               : (pack ? launch<K_BF16, false, true>(p, smem, grid, s)
+                       : launch<K_BF16, false, false>(p, smem, grid, s));
   if (rc == kOk && p.R > 1) rc = sum_partials_f32(part, dw, welems, p.R, s);
   if (part) scratch_free(part, s);
   return rc;

@@ -87,18 +87,18 @@ struct Row {
 
 // Stage nrows rows (this warp takes rows warp, warp + nwarps, ...), each
 // npix pixels x nch chunks of EPC channels; chunk j of row pixel i goes to
-// dst + j*plane_bytes + (r*npix + i)*16.  `clim` = channels available from
+// dst + j*plane_bytes + (r*row + i)*16.  `clim` = channels available from
 // the block start (chunks past it are zero).  Loads are issued BATCH slots
 // per lane at a time before any conversion, so each lane keeps BATCH
 // requests in flight.
 template <int KIND, int EPC, int BATCH, class RowFn>
 __device__ __forceinline__ void stage_rows(uint8_t *dst, uint32_t lo_off, uint32_t plane_bytes,
-                                           int nrows, int npix, int nch, int clim, int vec,
+                                           int nrows, int npix, int row, int nch, int clim, int vec,
                                            int warp, int nwarps, int lane, RowFn rowfn) {
   const int S = npix * nch;
   const int nsh = (nch & (nch - 1)) == 0 ? __ffs(nch) - 1 : -1;
   for (int r = warp; r < nrows; r += nwarps) {
-    const Row row = rowfn(r);
+    const Row in = rowfn(r);
     for (int s0 = 0; s0 < S; s0 += 32 * BATCH) {
       float v[BATCH][EPC];
       int off[BATCH];
@@ -111,11 +111,11 @@ __device__ __forceinline__ void stage_rows(uint8_t *dst, uint32_t lo_off, uint32
         if (sl < S) {
           const int i = nsh >= 0 ? (sl >> nsh) : sl / nch;
           const int j = sl - i * nch;
-          off[q] = (int)(j * plane_bytes) + (r * npix + i) * 16;
-          const int vv = row.vfirst + i * row.vstride;
+          off[q] = (int)(j * plane_bytes) + (r * row + i) * 16;
+          const int vv = in.vfirst + i * in.vstride;
           const int c = j * EPC;
-          if (row.ok && vv >= 0 && vv < row.vlim && c < clim) {
-            const float *src = row.rowp + (long long)i * row.pstep + c;
+          if (in.ok && vv >= 0 && vv < in.vlim && c < clim) {
+            const float *src = in.rowp + (long long)i * in.pstep + c;
             if (vec && c + EPC <= clim) {
 load_vec<EPC>(src, vec, v[q]);
             } else {
@@ -140,11 +140,11 @@ namespace owlgpu {
 namespace stage {
 
 // One operand tile for stage_rows2: nrows rows of npix pixels x nch chunks,
-// chunk j of row r pixel i at dst + j*plane_bytes + (r*npix + i)*16.
+// chunk j of row r pixel i at dst + j*plane_bytes + (r*row + i)*16.
 struct RowSet {
   uint8_t *dst;
   uint32_t lo_off, plane_bytes;
-  int nrows, npix, nch, clim;
+  int nrows, npix, row, nch, clim;
 };
 
 // Stage two row sets in the same passes: warp w takes row w (+ k*nwarps)
@@ -179,7 +179,7 @@ __device__ __forceinline__ void stage_rows2(const RowSet &A, FnA rowa, const Row
         if (hasA && sl < SA) {
           const int i = nshA >= 0 ? (sl >> nshA) : sl / A.nch;
           const int j = sl - i * A.nch;
-          oa[q] = (int)(j * A.plane_bytes) + (r * A.npix + i) * 16;
+          oa[q] = (int)(j * A.plane_bytes) + (r * A.row + i) * 16;
           const int vv = ra.vfirst + i * ra.vstride, c = j * EPC;
           if (ra.ok && vv >= 0 && vv < ra.vlim && c < A.clim) {
             const float *src = ra.rowp + (long long)i * ra.pstep + c;
@@ -202,7 +202,7 @@ load_vec<EPC>(src, vec, va[q]);
         if (hasB && sl < SB) {
           const int i = nshB >= 0 ? (sl >> nshB) : sl / Bs.nch;
           const int j = sl - i * Bs.nch;
-          ob[q] = (int)(j * Bs.plane_bytes) + (r * Bs.npix + i) * 16;
+          ob[q] = (int)(j * Bs.plane_bytes) + (r * Bs.row + i) * 16;
           const int vv = rb.vfirst + i * rb.vstride, c = j * EPC;
           if (rb.ok && vv >= 0 && vv < rb.vlim && c < Bs.clim) {
             const float *src = rb.rowp + (long long)i * rb.pstep + c;
@@ -274,6 +274,15 @@ __device__ __forceinline__ void table_store(uint8_t *dst, int d, uint32_t lo_off
 #pragma unroll
   for (int q = 0; q < Q; ++q)
     if (q * d < n) put_chunk<KIND, 8>(dst + (uint32_t)(q * d) * 16u, lo_off, v[q]);
+}
+
+// The same at dst + at[q*d]*16.
+template <int KIND, int Q>
+__device__ __forceinline__ void table_store_at(uint8_t *dst, const uint16_t *at, int d,
+                                               uint32_t lo_off, int n, const float (&v)[Q][8]) {
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+    if (q * d < n) put_chunk<KIND, 8>(dst + (uint32_t)at[q * d] * 16u, lo_off, v[q]);
 }
 
 }  // namespace stage
