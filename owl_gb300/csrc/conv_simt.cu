@@ -83,6 +83,19 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
   int64_t kt_begin = -KT;  // k of the table's first entry
 
   const int tid = threadIdx.x;
+  // Pixels and taps are decoded in 32 bits where the sizes allow: the decode of a
+  // slab is a serial chain of divisions that every thread waits for.
+  const bool narrow = g.M < (1LL << 31) && g.K < (1LL << 31);
+  auto split = [&](int64_t &p, int64_t d) -> int64_t {  // p / d in place; the remainder
+    if (narrow) {
+      const uint32_t a = (uint32_t)p, q = a / (uint32_t)d;
+      p = q;
+      return a - q * (uint32_t)d;
+    }
+    const int64_t q = p / d, r = p - q * d;
+    p = q;
+    return r;
+  };
   const int64_t m0 = (int64_t)blockIdx.x * BM;
   // BWDK: a thread's A elements all sit in row m0 + tid % BM (NT is a
   // multiple of BM), so its tap and channel are decoded once.
@@ -93,12 +106,10 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
     const int64_t m = m0 + tid % BM;
     a_mval = m < g.M;
     if (a_mval) {
-      int64_t tap = m / g.Ci;
-      a_ci = (int)(m - tap * g.Ci);
-      const int kd = (int)(tap % g.KD);
-      tap /= g.KD;
-      const int kr = (int)(tap % g.KR), kc = (int)(tap / g.KR);
-      a_dc = kc * g.dc;
+      int64_t kc = m;
+      a_ci = (int)split(kc, g.Ci);
+      const int kd = (int)split(kc, g.KD), kr = (int)split(kc, g.KR);
+      a_dc = (int)kc * g.dc;
       a_dr = kr * g.dr;
       a_dd = kd * g.dd;
     }
@@ -114,9 +125,8 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
   auto decode_pixel = [&](int64_t p, int slot, int buf) {
     if (MODE == BWDI) {
       if (p < g.M) {
-        int64_t id = p % g.ID, t = p / g.ID;
-        int64_t ir = t % g.IR; t /= g.IR;
-        int64_t ic = t % g.IC, b = t / g.IC;
+        int64_t b = p;
+        const int64_t id = split(b, g.ID), ir = split(b, g.IR), ic = split(b, g.IC);
         s_base[buf][slot] = b * g.OC * g.OR * g.OD;
         s_c[buf][slot] = (int)ic + g.pc;
         s_r[buf][slot] = (int)ir + g.pr;
@@ -127,9 +137,8 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
     } else {
       int64_t lim = (MODE == FWD) ? g.M : g.K;
       if (p < lim) {
-        int64_t od = p % g.OD, t = p / g.OD;
-        int64_t orr = t % g.OR; t /= g.OR;
-        int64_t oc = t % g.OC, b = t / g.OC;
+        int64_t b = p;
+        const int64_t od = split(b, g.OD), orr = split(b, g.OR), oc = split(b, g.OC);
         s_base[buf][slot] = b * g.IC * g.IR * g.ID;
         s_c[buf][slot] = (int)(oc * g.sc) - g.pc;
         s_r[buf][slot] = (int)(orr * g.sr) - g.pr;
@@ -169,11 +178,8 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
         for (int i = tid; i < KT; i += NT) {
           const int64_t k = k0 + i;
           if (k >= k_end) break;
-          int64_t tap = k / g.Ci;
-          const int64_t ci = k - tap * g.Ci;
-          const int64_t kd = tap % g.KD;
-          tap /= g.KD;
-          const int64_t kr = tap % g.KR, kc = tap / g.KR;
+          int64_t kc = k;
+          const int64_t ci = split(kc, g.Ci), kd = split(kc, g.KD), kr = split(kc, g.KR);
           s_kc[i] = (int)(kc * g.dc);
           s_kr[i] = (int)(kr * g.dr);
           s_kd[i] = (int)(kd * g.dd);
@@ -216,10 +222,11 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
       int kc = 0, kr = 0, kd = 0, co = 0;
       bool kval = k < k_end;
       if (kval) {
-        int64_t tap = k / g.Co;
-        co = (int)(k - tap * g.Co);
-        kd = (int)(tap % g.KD); tap /= g.KD;
-        kr = (int)(tap % g.KR); kc = (int)(tap / g.KR);
+        int64_t t = k;
+        co = (int)split(t, g.Co);
+        kd = (int)split(t, g.KD);
+        kr = (int)split(t, g.KR);
+        kc = (int)t;
       }
 #pragma unroll
       for (int i = 0; i < A_PER; ++i) {
@@ -246,7 +253,8 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
         int64_t kq = k0 + kk2, n = n0 + nn;
         T v = T(0);
         if (kq < k_end && n < g.N) {
-          int64_t tap = kq / g.Co, co = kq - tap * g.Co;
+          int64_t tap = kq;
+          const int64_t co = split(tap, g.Co);
           v = B0[(tap * g.Ci + n) * g.Co + co];
         }
         b_reg[i] = v;
@@ -1147,11 +1155,14 @@ int splitk_t(Dtype dt, const ConvGeom &g, const T *A, const T *B, T *C, cudaStre
     return kOk;
   }
   // Split the reduction so that ~4 waves of CTAs cover 152 SMs, with
-  // each split at least 8 K-tiles deep.
+  // each split at least 8 K-tiles deep.  A small result is worth more splits (one
+  // tile's CTAs are all there are: [256;28;28;1] x [5;5;1;32] 55 us with 256 of them,
+  // 40 with 598, their sums 5.5 and 10).
   int64_t tiles = ceil_div(d.M, tile_m<T>(d)) * ceil_div(d.N, tile_n<T>(d));
   int64_t want = ceil_div(4 * 152, tiles);
   int64_t max_by_k = ceil_div(d.K, 64);
-  int splits = (int)std::max<int64_t>(1, std::min<int64_t>(want, std::min<int64_t>(max_by_k, 256)));
+  const int64_t most = d.M * d.N <= 4096 ? 4 * 152 : 256;
+  int splits = (int)std::max<int64_t>(1, std::min<int64_t>(want, std::min<int64_t>(max_by_k, most)));
   int64_t kps = ceil_div(ceil_div(d.K, splits), 16) * 16;
   splits = (int)ceil_div(d.K, kps);
   if (splits == 1) {

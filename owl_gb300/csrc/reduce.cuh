@@ -1,14 +1,12 @@
-// reduce.cuh -- the sum of split reductions' partials in split order, with an
-// optional bias and activation: out[i] = act((((p0 + p1) + p2) + ...)[i] +
-// bias[i % C]).  Deterministic: every element is summed by one thread in
-// increasing split, whatever the kernel below.
+// reduce.cuh -- the sum of split reductions' partials, with an optional bias and
+// activation: out[i] = act((p0 + p1 + ...)[i] + bias[i % C]).  Deterministic: an
+// element's partials are added in an order that its kernel below fixes.
 //
 // Bound: reading the partials once (HBM / L2).  A thread that adds partials
 // as it loads them keeps one load in flight and waits a memory round trip per
 // split (256 partials of 800 elements took 95 us); so the loads are issued
-// ahead of the ordered adds: 16 at a time per thread where there are enough
-// elements to fill the GPU, and by a whole block into shared memory where
-// there are few.
+// ahead of the ordered adds, 16 at a time per thread, and where there are too few
+// elements to fill the GPU eight threads share one.
 #pragma once
 
 #include "../../include/owlgpu.h"
@@ -77,9 +75,12 @@ __global__ void __launch_bounds__(256) sum_splits_kernel(const T *__restrict__ p
   }
 }
 
-// 32 elements a block: 8 rows of 32 threads load kRows partials at a time into
-// shared memory (the next batch already in flight), one row adds them in order.
-constexpr int kSumRows = 64;
+// 32 elements a block: row r of its 8 rows of 32 threads adds the partials r, r + 8, ..
+// in order, kSumAhead loads at a time, then one row adds the 8 sums in order.  (One row
+// adding all of them from shared memory took as long, 10 us for 800 elements x 598
+// partials, and its rounding grew with their number: a training step's gradients were
+// 3.7e-7 off 64 bits where they are 1.9e-7 off so.)
+constexpr int kSumAhead = 16;
 template <typename T>
 __global__ void __launch_bounds__(256) sum_splits_few_kernel(const T *__restrict__ part,
                                                              T *__restrict__ out, long long n,
@@ -87,40 +88,33 @@ __global__ void __launch_bounds__(256) sum_splits_few_kernel(const T *__restrict
                                                              const T *__restrict__ bias,
                                                              long long C, int act) {
   asm volatile("griddepcontrol.wait;" ::: "memory");  // launched with launch_pdl
-  __shared__ T buf[kSumRows][32];
+  __shared__ T rows[8][32];
   const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
   const long long i = (long long)blockIdx.x * 32 + lane;
-  constexpr int PER = kSumRows / 8;
-  T v[PER];
-  auto load = [&](int z0) {
-#pragma unroll
-    for (int u = 0; u < PER; ++u) {
-      const int z = z0 + row + 8 * u;
-      if (z < splits && i < n) v[u] = part[(long long)z * n + i];
-    }
-  };
-  load(0);
   T s{};
-  for (int z0 = 0; z0 < splits; z0 += kSumRows) {
+  if (i < n && row < splits) {
+    s = part[(long long)row * n + i];
+    for (int z0 = row + 8; z0 < splits; z0 += 8 * kSumAhead) {
+      T v[kSumAhead];
 #pragma unroll
-    for (int u = 0; u < PER; ++u) buf[row + 8 * u][lane] = v[u];
-    __syncthreads();
-    if (z0 + kSumRows < splits) load(z0 + kSumRows);
-    if (row == 0) {
-      const int m = min(kSumRows, splits - z0);
-      for (int z = 0; z < m; ++z) {
-        if (z0 + z == 0) s = buf[0][lane];
-        else s += buf[z][lane];
-      }
+      for (int u = 0; u < kSumAhead; ++u)
+        if (z0 + 8 * u < splits) v[u] = part[(long long)(z0 + 8 * u) * n + i];
+#pragma unroll
+      for (int u = 0; u < kSumAhead; ++u)
+        if (z0 + 8 * u < splits) s += v[u];
     }
-    __syncthreads();
   }
-  if (row == 0 && i < n) out[i] = finish_sum(s, bias, i, C, act);
+  rows[row][lane] = s;
+  __syncthreads();
+  if (row == 0 && i < n) {
+    for (int r = 1; r < min(8, splits); ++r) s += rows[r][lane];
+    out[i] = finish_sum(s, bias, i, C, act);
+  }
 }
 
 // Fewer than 152 * 128 elements do not fill the GPU one thread each: the
 // block form reads them (measured on 800 elements x 256 partials: 95 us as
-// one thread per element adding as it loads, 5.6 us here).
+// one thread per element adding as it loads, 5.5 us here).
 template <typename T>
 int sum_splits(const T *part, T *out, long long n, int splits, const T *bias, long long C, int act,
                cudaStream_t s) {
