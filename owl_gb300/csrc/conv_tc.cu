@@ -8,9 +8,8 @@
 //     another (v): N = 8*TU pixels (TU even, up to 32), each group of 8
 //     v-positions one 8-row core-matrix band of the MMA's N dimension.  The
 //     kernel tile (128 output channels) is the M = 128 operand.  tcgen05.mma
-//     costs the same number of cycles for any N at M = 128, so the pixel
-//     dimension goes on N, the tile is as tall as the fewest tiles along u
-//     allow, and no taller (less halo).
+//     costs about the same number of cycles for any N at M = 128, so the pixel
+//     dimension goes on N; plan() picks the tile for the batch.
 //   * Producer warps load the input halo the tile needs for one block of
 //     channels -- once -- from the float32 activation, convert it (bf16 RN,
 //     tf32 RNA, or bf16 hi + lo) and store it in shared memory as
@@ -337,7 +336,9 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
     // A lane keeps one 32-byte chunk of the channel block and takes every
     // lanes/chunks-th pixel of the halo, whose place comes from the table, kB a
     // batch.  Two batches are in registers, across stages and tiles: the loads of
-    // one are in flight while the other is converted and stored.
+    // one are in flight while the other is converted and stored.  (Rows dealt to
+    // warps left up to half the lanes idle on rows of 9 pixels: [64;28;28;256] x
+    // [3;3;256;256] at stride 2 takes 29 us, 39 with rows.)
     if constexpr (LANES) {
       constexpr int kB = 4;
       const int lg = 32 - __clz(p.NCH - 1);  // (clz(0) = 32)
