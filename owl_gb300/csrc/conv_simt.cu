@@ -409,7 +409,11 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 // pairs, B's values duplicated into both halves.  Blocks of 128 threads (three an
 // SM) instead of 256 (one) let one block's barrier and loads overlap another's
 // arithmetic: [32;56;56;128] x [3;3;128;128] 43 -> 48 TFLOP/s.
+//
+// WIDE: the column tiles lie along grid.x and the row tiles along grid.y, for
+// products of more columns than 65535 tiles hold.
 constexpr int kVBK = 16;
+constexpr int64_t kMaxGridY = 65535;
 
 __device__ __forceinline__ float4 ldg4(const float *p) {
   return __ldg(reinterpret_cast<const float4 *>(p));
@@ -427,7 +431,7 @@ __device__ __forceinline__ void ffma2(uint64_t &d, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
 
-template <int MODE, int BM, int BN, int TM, int TN, bool BT>
+template <int MODE, int BM, int BN, int TM, int TN, bool BT, bool WIDE>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
     conv_f32v_kernel(Dev g, const float *__restrict__ A0, const float *__restrict__ B0,
                      float *__restrict__ C, int64_t k_per_split) {
@@ -450,7 +454,8 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
   constexpr int CW = BN / TN / 4;  // warps along the columns
   const int lane = tid & 31, warp = tid >> 5;
   const int ty = (warp / CW) * 8 + (lane >> 2), tx = (warp % CW) * 4 + (lane & 3);
-  const int64_t m0 = (int64_t)blockIdx.x * BM, n0 = (int64_t)blockIdx.y * BN;
+  const int64_t m0 = (int64_t)(WIDE ? blockIdx.y : blockIdx.x) * BM,
+                n0 = (int64_t)(WIDE ? blockIdx.x : blockIdx.y) * BN;
   const int64_t k_begin = (int64_t)blockIdx.z * k_per_split;
   const int64_t k_end = min(g.K, k_begin + k_per_split);
   const int64_t img = g.IC * g.IR * g.ID;  // pixels per batch image of X
@@ -824,11 +829,12 @@ bool f32v_ok(int mode, const Dev &d, const void *A, const void *B, const void *C
          d.Co % kVBK == 0 && kps % kVBK == 0;
 }
 
-template <int MODE, int BM, int BN, int TM, int TN, bool BT>
+template <int MODE, int BM, int BN, int TM, int TN, bool BT, bool WIDE = false>
 cudaError_t launch_f32v_tile(const Dev &d, const float *A, const float *B, float *C, int splits,
                              int64_t kps, cudaStream_t s) {
-  dim3 grid((unsigned)ceil_div(d.M, BM), (unsigned)ceil_div(d.N, BN), (unsigned)splits);
-  return launch_pdl(conv_f32v_kernel<MODE, BM, BN, TM, TN, BT>, grid,
+  const unsigned mt = (unsigned)ceil_div(d.M, BM), nt = (unsigned)ceil_div(d.N, BN);
+  const dim3 grid(WIDE ? nt : mt, WIDE ? mt : nt, (unsigned)splits);
+  return launch_pdl(conv_f32v_kernel<MODE, BM, BN, TM, TN, BT, WIDE>, grid,
                     dim3((BM / TM) * (BN / TN)), 0, s, d, A, B, C, kps);
 }
 
@@ -840,10 +846,14 @@ cudaError_t launch_f32v_tile(const Dev &d, const float *A, const float *B, float
 // w warps (by registers 3 blocks of 128 x 64 fit, 4 of 128 x 32, 6 of 64 x 32).
 // Measured against each tile forced: it takes the fastest on wide, ragged (N =
 // 160, 96), 5x5x32x64, 3-D and [8;32;32;16] x [3;3;16;32] layers in all three passes,
-// or one within 3 %.
+// or one within 3 %.  Where the 32-column tiles are more than a grid's y axis takes,
+// the 64-column one; where those are too, that one with its grid turned (3: a kernel of
+// its own, for choosing the axis in the kernel cost the ragged float32 layers 2 %).
 int pick_f32v(const Dev &d, int splits) {
   static const struct { int bm, bn, most; double cost; } t[] = {
       {128, 64, 3, 1.0}, {128, 32, 4, 1.13}, {64, 32, 6, 1.33}};
+  if (ceil_div(d.N, 64) > kMaxGridY) return 3;
+  if (ceil_div(d.N, 32) > kMaxGridY) return 0;
   int best = 0;
   double least = 0;
   for (int i = 0; i < 3; ++i) {
@@ -864,7 +874,8 @@ int launch_f32v(const Dev &d, const float *A, const float *B, float *C, int spli
   switch (pick_f32v(d, splits)) {
     case 0: e = launch_f32v_tile<MODE, 128, 64, 8, 8, BT>(d, A, B, C, splits, kps, s); break;
     case 1: e = launch_f32v_tile<MODE, 128, 32, 8, 4, BT>(d, A, B, C, splits, kps, s); break;
-    default: e = launch_f32v_tile<MODE, 64, 32, 4, 4, BT>(d, A, B, C, splits, kps, s);
+    case 2: e = launch_f32v_tile<MODE, 64, 32, 4, 4, BT>(d, A, B, C, splits, kps, s); break;
+    default: e = launch_f32v_tile<MODE, 128, 64, 8, 8, BT, true>(d, A, B, C, splits, kps, s);
   }
   if (e == cudaSuccess) e = cudaGetLastError();
   note_launch();
@@ -907,7 +918,8 @@ int launch_cfg(const Dev &d, const T *A, const T *B, T *C, int splits, int64_t k
 // 8- and 16-byte elements: the FP64 pipe is slow enough that any tile feeds
 // it, so the smallest busiest SM wins, ceil(tiles / SMs) tiles of BM x BN, the
 // larger tile on a tie ([8;28;28;32] x [5;5;32;64]: 98 tiles of 64 x 64 leave a
-// third of the SMs idle, 883 us; 392 of 32 x 32, 625 us).
+// third of the SMs idle, 883 us; 392 of 32 x 32, 625 us).  No tile of 32 columns where
+// N has more of them than a grid's y axis takes.
 template <typename T, int MODE>
 int launch_any(const Dev &d, const T *A, const T *B, T *C, int splits, int64_t kps,
                cudaStream_t s) {
@@ -921,9 +933,10 @@ int launch_any(const Dev &d, const T *A, const T *B, T *C, int splits, int64_t k
       return launch_f32v<FWD, true>(f, A, B, C, splits, kps, s);
     }
   }
+  const bool wide = ceil_div(d.N, 32) > kMaxGridY;
   if constexpr (sizeof(T) == 4) {
     if constexpr (MODE == BWDK) {
-      if (d.M <= 32) return launch_cfg<T, MODE, 32, 32, 32, 2, 2>(d, A, B, C, splits, kps, s);
+      if (d.M <= 32 && !wide) return launch_cfg<T, MODE, 32, 32, 32, 2, 2>(d, A, B, C, splits, kps, s);
     }
     if (d.N > 64) return launch_cfg<T, MODE, 128, 128, 8, 8, 8>(d, A, B, C, splits, kps, s);
     if (d.N > 32) return launch_cfg<T, MODE, 128, 64, 8, 8, 4>(d, A, B, C, splits, kps, s);
@@ -933,9 +946,9 @@ int launch_any(const Dev &d, const T *A, const T *B, T *C, int splits, int64_t k
       return ceil_div(ceil_div(d.M, bm) * ceil_div(d.N, bn) * splits, 152) * bm * bn;
     };
     const int64_t big = d.N > 32 ? busiest(64, 64) : busiest(64, 32), mid = busiest(32, 32);
-    if (busiest(16, 32) < std::min(big, mid))
+    if (!wide && busiest(16, 32) < std::min(big, mid))
       return launch_cfg<T, MODE, 16, 32, 16, 1, 2>(d, A, B, C, splits, kps, s);
-    if (mid < big) return launch_cfg<T, MODE, 32, 32, 8, 2, 2>(d, A, B, C, splits, kps, s);
+    if (!wide && mid < big) return launch_cfg<T, MODE, 32, 32, 8, 2, 2>(d, A, B, C, splits, kps, s);
     if (d.N > 32) return launch_cfg<T, MODE, 64, 64, 8, 4, 4>(d, A, B, C, splits, kps, s);
     return launch_cfg<T, MODE, 64, 32, 8, 4, 2>(d, A, B, C, splits, kps, s);
   }
