@@ -42,6 +42,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <cstring>
 #include <mutex>
 #include <vector>
@@ -75,6 +76,10 @@ constexpr int kSmemMax = 232448;  // 227 KB opt-in dynamic shared memory
 constexpr int kSmemLean = 195 * 1024;  // the carve-out step below it, less the block's 1 KB
 constexpr long long kSpinLimit = 4000000000LL;  // cycles (~2 s) before a wait gives up
 
+// How the producers find the halo's pixels: element by element along its rows (any
+// operand), or whole 32-byte chunks (32-byte aligned, channels a multiple of 8) from a
+// table of its pixels or of its rows.
+enum Stage { S_ELEMENT = 0, S_PIXELS = 1, S_ROWS = 2 };
 enum Kind { K_BF16 = 0, K_TF32 = 1, K_BF16X3 = 2 };
 
 // A launch covers up to kMaxSeg segments: convolutions that share the input,
@@ -105,6 +110,7 @@ struct TcParams {
   // column stride of the accumulators of a tile's co tiles and buffers).
   int TU, TN, TNA;
   int T;  // plan: taps of the longest segment
+  int stage;  // plan: how the halo is staged (Stage)
   int n_table;  // taps of all segments
   int sw, su, sv;          // strides along w, u, v
   // Halo: HW x HU input rows, of which the stage holds those that some tap reads:
@@ -232,9 +238,8 @@ __device__ __forceinline__ void halo_row(const TcParams &p, int r, int &hr, int 
 }
 
 // MULTI: the launch has several segments (else segment 0 only, read at a
-// constant offset of the parameters).  LANES: the input is staged as whole
-// 32-byte chunks (32-byte aligned, channels a multiple of 8).
-template <int KIND, bool MULTI, bool LANES>
+// constant offset of the parameters).  STAGE: see Stage.
+template <int KIND, bool MULTI, int STAGE>
 __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_constant__ TcParams p) {
   if (p.wait_all) asm volatile("griddepcontrol.wait;" ::: "memory");
   constexpr int EPC = (KIND == K_TF32) ? 4 : 8;  // channels per 16-byte chunk
@@ -265,8 +270,10 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   uint32_t *tap_off = tmem_slot + 2;  // per-tap start pixel in the halo (16-byte units)
-  // LANES: where the stage's pixels lie, {offset in floats from the tile's first input
-  // pixel, position}, and one past the end that is outside any bounds
+  constexpr bool LANES = STAGE != S_ELEMENT;
+  // LANES: where the stage's pixels (or first pixels of its rows) lie, {offset in floats
+  // from the tile's first input pixel, position}, and one past the end that is outside
+  // any bounds
   int2 *ptab = reinterpret_cast<int2 *>((reinterpret_cast<uintptr_t>(tap_off + p.n_table) + 7) &
                                         ~(uintptr_t)7);
   // The setup is a call's latency, so its parts run side by side: the barriers and
@@ -314,16 +321,18 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
   } else if (LANES) {
     const float r_hvr = __frcp_rn((float)p.HVR), r_nv = __frcp_rn((float)p.n_vres),
                 r_nhu = __frcp_rn((float)p.NHU), r_nu = __frcp_rn((float)p.n_ures);
-    for (int i = threadIdx.x - 32; i < p.HP; i += (kEpiWarp0 - 1) * 32) {
-      const int row = quot(i, r_hvr), t = quot(row, r_nv);
-      const int hr = p.vres[row - t * p.n_vres] + (i - row * p.HVR) * p.sv;
+    const int n = STAGE == S_PIXELS ? p.HP : p.nrows;
+    for (int i = threadIdx.x - 32; i < n; i += (kEpiWarp0 - 1) * 32) {
+      const int row = STAGE == S_PIXELS ? quot(i, r_hvr) : i, t = quot(row, r_nv);
+      const int hr = p.vres[row - t * p.n_vres] +
+                     (STAGE == S_PIXELS ? (i - row * p.HVR) * p.sv : 0);
       const int hw = quot(t, r_nhu), hi = t - hw * p.NHU, uq = quot(hi, r_nu);
       const int hu = uq * p.su + p.ures[hi - uq * p.n_ures];
       ptab[i] = make_int2((int)((hw * p.xsw + hu * p.xsu + hr * p.xsv) * p.Cin),
                           (int)(stage::position(hr, hu, hw) | stage::kGuard));
     }
     if (threadIdx.x == 32)
-      ptab[p.HP] = make_int2(0, (int)(stage::position(stage::kMaxV + 1, 0, 0) | stage::kGuard));
+      ptab[n] = make_int2(0, (int)(stage::position(stage::kMaxV + 1, 0, 0) | stage::kGuard));
   }
   tc_fence_before();
   __syncthreads();
@@ -334,8 +343,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
   if (LANES && pidx >= 0) {
     // ===================== halo producers, whole chunks =====================
     // A lane keeps one 32-byte chunk of the channel block and takes every
-    // lanes/chunks-th pixel of the halo, whose place comes from the table, kB a
-    // batch.  Two batches are in registers, across stages and tiles: the loads of
+    // lanes/chunks-th pixel of the halo, whose place comes from the table (of rows:
+    // from its row's, the row and the pixel in it advancing by constants), kB a batch.  Two batches are in registers, across stages and tiles: the loads of
     // one are in flight while the other is converted and stored.  (Rows dealt to
     // warps left up to half the lanes idle on rows of 9 pixels: [64;28;28;256] x
     // [3;3;256;256] at stride 2 takes 29 us, 39 with rows.)
@@ -350,6 +359,11 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
       // the next batch to load: batch lb of channel block lc of tile t
       long long t = blockIdx.x;
       int lb = 0, lc = 0, sc = 0;
+      // S_ROWS: the lane's next pixel as row and place in it
+      const int row0 = px / p.HVR, at0 = px - row0 * p.HVR;
+      const int drow = dpx / p.HVR, dat = dpx - drow * p.HVR;
+      const int pix_off = (int)(p.sv * p.xsv * p.Cin);
+      int row = row0, at = at0;
       const float *xt = nullptr;
       unsigned lo = 0, hi = 0;
       auto tile_begin = [&] {
@@ -376,10 +390,30 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_kernel(const __grid_const
       auto load = [&](float(&v)[kB][8]) {
         // (chunks past the channels, of a ragged last block, are zeros)
         const bool real = lc * p.CPB + j * EPC < p.Cin;
-        stage::table_load<kB>(ptab, px + lb * kB * dpx, dpx, p.HP, xt + lc * p.CPB,
-                              real ? lo : (unsigned)stage::kMaxV, real ? hi : 0u, v);
+        const unsigned l = real ? lo : (unsigned)stage::kMaxV, h = real ? hi : 0u;
+        if (STAGE == S_PIXELS) {
+          stage::table_load<kB>(ptab, px + lb * kB * dpx, dpx, p.HP, xt + lc * p.CPB, l, h, v);
+        } else {
+          int2 e[kB];
+#pragma unroll
+          for (int q = 0; q < kB; ++q) {
+            const int a = row < p.nrows ? at : 0;
+            e[q] = ptab[min(row, p.nrows)];
+            e[q].x += a * pix_off;
+            e[q].y += a * p.sv;
+            row += drow;
+            at += dat;
+            if (at >= p.HVR) {
+              at -= p.HVR;
+              ++row;
+            }
+          }
+          stage::entry_load<kB>(e, xt + lc * p.CPB, l, h, v);
+        }
         if (++lb == batches) {
           lb = 0;
+          row = row0;
+          at = at0;
           if (++lc == p.NCB) {
             lc = 0;
             t += gridDim.x;
@@ -1069,10 +1103,17 @@ struct PlanSeg {
 
 // What a plan's time is made of, in us (measured on GB300; the choice needs
 // their ratios only): a tile; an MMA with one and with two accumulators in turn, and per
-// column of N; a stage and a batch of the producers' loads; weight bytes and output
-// bytes per us and SM; the hand-off of a weight slot.
+// column of N; a stage and a batch of the producers' loads (S_ELEMENT, S_PIXELS,
+// S_ROWS); weight bytes and output bytes per us and SM; the hand-off of a weight slot,
+// and, where shared memory is tight, of one with a single tap and one more in flight.
 constexpr double kMma1 = 0.056, kMma2 = 0.0485, kMmaCol = 0.00027;
-constexpr double kTile = 0.6, kStage = 0.2, kBatch = 0.25, kWeightRate = 100e3, kStoreRate = 45e3, kSlot = 0.2;
+constexpr double kTile = 0.6, kStage = 0.2, kBatch[3] = {1.25, 0.25, 0.3};
+constexpr double kWeightRate = 100e3, kStoreRate = 45e3, kSlot = 0.2, kLoneSlot = 0.3;
+
+// Shared memory of the staging table.
+long long table_bytes(const TcParams &p) {
+  return p.stage == S_PIXELS ? 8LL * (p.HP + 2) : (p.stage == S_ROWS ? 8LL * (p.nrows + 2) : 0);
+}
 
 // Choose tile and pipeline sizes; false if no configuration fits.
 //
@@ -1096,8 +1137,9 @@ constexpr double kTile = 0.6, kStage = 0.2, kBatch = 0.25, kWeightRate = 100e3, 
 // `v` holds the largest halo extents of the launch's segments; t_slot is the
 // most taps of one segment (weight slots), t_table the taps of all segments
 // (the shared-memory tap table).
+// `chunks`: the input is aligned for staging whole 32-byte chunks.
 bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const PlanSeg *segs,
-          int nseg) {
+          int nseg, bool chunks) {
   const int EB = (kind == K_TF32) ? 4 : 2;
   const int parts = (kind == K_BF16X3) ? 2 : 1;
   const int sms = num_sms();
@@ -1109,8 +1151,9 @@ bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const P
   const int max_tu = std::min(32, max_ou);
 
   // q: the sizes of one configuration; false when it does not fit
-  auto fit = [&](TcParams &q, int nh, int tu, int cb, int nct, bool lean = false) {
+  auto fit = [&](TcParams &q, int stage, int nh, int tu, int cb, int nct, bool lean = false) {
     q = p;
+    q.stage = stage;
     q.NH = nh;
     q.TU = tu;
     q.TN = 8 * tu;
@@ -1133,8 +1176,14 @@ bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const P
     q.PS = q.HP + (((1 - q.HP) % 8) + 8) % 8;  // plane stride = 1 (mod 8) pixels
     if (q.PS >= 16384) return false;
     q.halo_bytes = (unsigned)q.PS * 16u * (unsigned)q.NCH;
+    // (the tables' offsets are 32-bit, their positions' fields 10, 10 and 9 bits)
+    const long long span_v = (long long)q.HVR * v.sv;
+    if (stage != S_ELEMENT && kind != K_TF32 &&
+        (span_v > stage::kMaxV || q.HU > stage::kMaxU || q.HW > stage::kMaxW ||
+         (q.HW * v.xsw + q.HU * v.xsu + span_v * v.xsv) * v.Cin >= (1LL << 31)))
+      return false;
     const long long fixed =
-        (long long)q.NH * parts * q.halo_bytes + 512 + 4LL * t_table + 8LL * (q.HP + 2);
+        (long long)q.NH * parts * q.halo_bytes + 512 + 4LL * t_table + table_bytes(q);
     // Shared memory up to the step that leaves 60 KB of the SM's 256 for the L1
     // cache where a third of the taps (three at least) fit a weight slot in that: the
     // producers' loads in flight (up to 74 KB) wait for lines of a smaller one (57.3
@@ -1165,6 +1214,7 @@ bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const P
     return true;
   };
   // estimated time of a configuration (the start that all share left out)
+  double lone_slot = kSlot;
   auto estimate = [&](const TcParams &q) {
     long long tiles = 0, taps_sum = 0;
     for (int c = 0; c < nseg; ++c) {
@@ -1178,12 +1228,13 @@ bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const P
     const double rounds = (double)((tiles + sms - 1) / sms);
     const double mmas = taps * q.NCB * (q.NCH / 2) * q.NCT * (parts == 2 ? 3 : 1);
     const double mma = mmas * std::max(q.NCT * parts == 1 ? kMma1 : kMma2, kMmaCol * q.TN) +
-                       q.NCB * std::max(1.0, taps / q.TPS) * kSlot;
+                       q.NCB * std::max(1.0, taps / q.TPS) *
+                           (q.TPS == 1 && q.NB == 2 ? lone_slot : kSlot);
     // the producers' batches of four chunks a lane
-    int chunks = 1;
-    while (chunks < q.NCH) chunks *= 2;
+    int pow2 = 1;
+    while (pow2 < q.NCH) pow2 *= 2;
     const int lanes = kProducerWarps * 32 * 4;
-    const double stage = kStage + kBatch * ((q.HP * chunks + lanes - 1) / lanes) *
+    const double stage = kStage + kBatch[q.stage] * ((q.HP * pow2 + lanes - 1) / lanes) *
                                       (parts == 2 ? 1.3 : 1.0);
     const double weights = taps * q.NCB * q.tile_bytes * (parts * q.NCT) / kWeightRate;
     const double store = (double)q.TN * std::min(v.Cout, q.BN * q.NCT) * 4 / kStoreRate;
@@ -1212,30 +1263,47 @@ bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const P
   // and TU <= 20, 122 with 64 and TU = 28), and so do the loads in flight
   // ([64;28;28;256]x[3;3;256;256] at stride 2: 39 us with 128 bytes, 31 with 64).
   // Else the first that fits with the lowest tile, then with one stage.
+  // The pixel table takes 8 bytes of shared memory a pixel; where no block fits beside
+  // it (3x3 at rate 36) the first that fits beside the row table, and where a position
+  // does not fit the tables' fields, without one.  (TF32 halos are staged element by
+  // element, and where nothing fits beside a pixel table the CUDA cores are faster:
+  // [4;65;65;256]x[3;3;256;256] at rate 36 takes 1360 us here and 442 there.)
   TcParams q;
-  int nh = 0, cb = 0;
-  for (int form = 0; form < 4 && !cb; ++form)
-    for (int i = 0; i < ncb && !cb; ++i) {
-      const int tall = form == 0 ? max_tu : (form == 1 ? std::min(16, max_tu) : 2);
-      if (form == 0 && cbs[i] == 32 && all > 32) continue;
-      const int nct = form == 0 && tall <= 16 ? std::min(2, p.n_tiles) : 1;
-      if (fit(q, form < 3 ? 2 : 1, tall, cbs[i], nct, form == 0)) {
-        nh = form < 3 ? 2 : 1;
-        cb = cbs[i];
+  int cb = 0, form = 0, stage = S_PIXELS;
+  for (;;) {
+    for (form = 0; form < 4 && !cb; form += !cb)
+      for (int i = 0; i < ncb && !cb; ++i) {
+        const int tall = form == 0 ? max_tu : (form == 1 ? std::min(16, max_tu) : 2);
+        if (form == 0 && cbs[i] == 32 && all > 32) continue;
+        const int nct = form == 0 && tall <= 16 ? std::min(2, p.n_tiles) : 1;
+        if (fit(q, stage, form < 3 ? 2 : 1, tall, cbs[i], nct, form == 0)) cb = cbs[i];
       }
-    }
+    if (cb || stage == S_ELEMENT || kind == K_TF32) break;
+    stage = stage == S_PIXELS ? S_ROWS : S_ELEMENT;
+  }
   if (!cb) return false;
+  // Where the pixel table leaves no two stages of a tall tile, plans with the row table
+  // (the same channel block, and so the same sums) and with one stage are weighed too:
+  // a pixel's place costs a few instructions more, low tiles far more.  The same layer
+  // in BF16 at rate 25 takes 99 us with one stage and TU = 18, 960 with TU = 2, and at
+  // rate 34 197 us from the row table, 1210 from the pixel table and TU = 2.
+  const bool tight = form >= 2 || stage != S_PIXELS;
+  if (tight) lone_slot = kLoneSlot;
+  int stages[2] = {chunks && kind != K_TF32 ? stage : S_ELEMENT, S_ROWS};
+  const int nstages = tight && stages[0] == S_PIXELS ? 2 : 1;
   double least = -1;
   TcParams best = p;
-  for (int tu = max_tu; tu >= 2; tu -= 2)
-    for (int nct = std::min(2, p.n_tiles); nct >= 1; --nct) {
-      if (!fit(q, nh, tu, cb, nct)) continue;
-      const double t = estimate(q);
-      if (least < 0 || t < least) {
-        least = t;
-        best = q;
-      }
-    }
+  for (int si = 0; si < nstages; ++si)
+    for (int nh = 2; nh >= (tight ? 1 : 2); --nh)
+      for (int tu = max_tu; tu >= 2; tu -= 2)
+        for (int nct = std::min(2, p.n_tiles); nct >= 1; --nct) {
+          if (!fit(q, stages[si], nh, tu, cb, nct)) continue;
+          const double t = estimate(q);
+          if (least < 0 || t < least) {
+            least = t;
+            best = q;
+          }
+        }
   p = best;
   return true;
 }
@@ -1301,13 +1369,13 @@ int drop_images(int dev, const void *w, bool all) {
   return kOk;
 }
 
-template <int KIND, bool MULTI, bool LANES>
+template <int KIND, bool MULTI, int STAGE>
 int launch(const TcParams &p, size_t smem, cudaStream_t s, bool after_prep) {
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    OWL_CUDA(cudaFuncSetAttribute(conv_tc_kernel<KIND, MULTI, LANES>,
+    OWL_CUDA(cudaFuncSetAttribute(conv_tc_kernel<KIND, MULTI, STAGE>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
     attr_set[dev] = true;
   }
@@ -1327,7 +1395,7 @@ int launch(const TcParams &p, size_t smem, cudaStream_t s, bool after_prep) {
   // then every thread waits for the earlier work (wait_all)
   TcParams q = p;
   q.wait_all = after_prep ? 0 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, conv_tc_kernel<KIND, MULTI, LANES>, q);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, conv_tc_kernel<KIND, MULTI, STAGE>, q);
   note_launch();
   note_tc_launch();
   if (e != cudaSuccess) return cuda_fail(e, "conv_tc_kernel");
@@ -1402,8 +1470,12 @@ int run_segs(int prec, int nseg_in, const SegSpec *sp, bool bwd_input, int Ci, i
     const View &v = sp[idx[k]].v;
     psegs[k] = {v.OW, v.OU, v.OV, v.KW * v.KU * v.KV};
   }
+  // 1: 16-byte vector loads; 2: 32-byte aligned chunks (one load per chunk)
+  p.vec_in = ((uintptr_t)x % 32 == 0 && pv.Cin % 8 == 0)
+                 ? 2
+                 : (((uintptr_t)x % 16 == 0) && (pv.Cin % 4 == 0) ? 1 : 0);
   if (pv.Cin == 0 || p.n_ures == 0 || p.n_vres == 0 ||
-      !plan(p, pv, kind, t_slot, t_table, psegs, nseg))
+      !plan(p, pv, kind, t_slot, t_table, psegs, nseg, p.vec_in == 2))
     return kErrUnsupported;
   p.n_table = t_table;
   p.x = x; p.y = y;
@@ -1443,10 +1515,6 @@ int run_segs(int prec, int nseg_in, const SegSpec *sp, bool bwd_input, int Ci, i
   if (tiles >= (1LL << 31)) return kErrUnsupported;
   p.total_tiles = tiles;
   p.idesc = instr_desc(kind == K_TF32 ? 2u : 1u, (uint32_t)p.TN);
-  // 1: 16-byte vector loads; 2: 32-byte aligned chunks (one load per chunk)
-  p.vec_in = ((uintptr_t)x % 32 == 0 && pv.Cin % 8 == 0)
-                 ? 2
-                 : (((uintptr_t)x % 16 == 0) && (pv.Cin % 4 == 0) ? 1 : 0);
   p.spin_limit = wait_limit();
   p.status = status_ptr();
   if (!p.status) {
@@ -1557,27 +1625,25 @@ int run_segs(int prec, int nseg_in, const SegSpec *sp, bool bwd_input, int Ci, i
   }
   const size_t smem = (size_t)p.NH * parts * p.halo_bytes + (size_t)p.NB * parts * p.b_bytes +
                       (2 * p.NH + 2 * p.NB + 5) * 8 + 16 + 4 * (size_t)t_table +
-                      8 * (size_t)(p.HP + 2);
+                      (size_t)table_bytes(p);
   const bool multi = p.nseg > 1;
   const bool pdl = prep && !build_cached;
-  // (the table's offsets are 32-bit, its positions' fields 10, 10 and 9 bits)
-  const long long span_v = (long long)p.HVR * p.sv;
-  const bool lanes = p.vec_in == 2 && span_v <= stage::kMaxV && p.HU <= stage::kMaxU &&
-                     p.HW <= stage::kMaxW &&
-                     (p.HW * p.xsw + p.HU * p.xsu + span_v * p.xsv) * p.Cin < (1LL << 31);
-  if (kind == K_TF32)
-    rc = multi ? launch<K_TF32, true, false>(p, smem, s, pdl)
-               : launch<K_TF32, false, false>(p, smem, s, pdl);
-  else if (kind == K_BF16X3)
-    rc = lanes ? (multi ? launch<K_BF16X3, true, true>(p, smem, s, pdl)
-                        : launch<K_BF16X3, false, true>(p, smem, s, pdl))
-               : (multi ? launch<K_BF16X3, true, false>(p, smem, s, pdl)
-                        : launch<K_BF16X3, false, false>(p, smem, s, pdl));
-  else
-    rc = lanes ? (multi ? launch<K_BF16, true, true>(p, smem, s, pdl)
-                        : launch<K_BF16, false, true>(p, smem, s, pdl))
-               : (multi ? launch<K_BF16, true, false>(p, smem, s, pdl)
-                        : launch<K_BF16, false, false>(p, smem, s, pdl));
+  auto go = [&](auto k) {
+    constexpr int KIND = decltype(k)::value;
+    if constexpr (KIND != K_TF32) {
+      if (p.stage == S_PIXELS)
+        return multi ? launch<KIND, true, S_PIXELS>(p, smem, s, pdl)
+                     : launch<KIND, false, S_PIXELS>(p, smem, s, pdl);
+      if (p.stage == S_ROWS)
+        return multi ? launch<KIND, true, S_ROWS>(p, smem, s, pdl)
+                     : launch<KIND, false, S_ROWS>(p, smem, s, pdl);
+    }
+    return multi ? launch<KIND, true, S_ELEMENT>(p, smem, s, pdl)
+                 : launch<KIND, false, S_ELEMENT>(p, smem, s, pdl);
+  };
+  if (kind == K_TF32) rc = go(std::integral_constant<int, K_TF32>{});
+  else if (kind == K_BF16X3) rc = go(std::integral_constant<int, K_BF16X3>{});
+  else rc = go(std::integral_constant<int, K_BF16>{});
   if (!cached) scratch_free(wt, s);
   return rc;
 }

@@ -249,22 +249,27 @@ __device__ __forceinline__ void field(int f0, int n, int top, unsigned &lo, unsi
   hi = (unsigned)max(h, 0);
 }
 
-// Q loads of a table's pixels i, i + d, .. (past its end the one at n, outside any
-// bounds): {offset in floats from `base`, position | kGuard}, those outside [lo, hi]
-// from a row of zeros.  No branches: a load that may or may not happen keeps its
-// registers' old values alive and costs their copies.
+// Q loads of entries {offset in floats from `base`, position | kGuard}, those outside
+// [lo, hi] from a row of zeros; table_load: a table's entries i, i + d, .. (past its
+// end the one at n, outside any bounds).  No branches: a load that may or may not
+// happen keeps its registers' old values alive and costs their copies.
 template <int Q>
-__device__ __forceinline__ void table_load(const int2 *tab, int i, int d, int n, const float *base,
-                                           unsigned lo, unsigned hi, float (&v)[Q][8]) {
-  int2 e[Q];
-#pragma unroll
-  for (int q = 0; q < Q; ++q) e[q] = tab[min(i + q * d, n)];
+__device__ __forceinline__ void entry_load(const int2 (&e)[Q], const float *base, unsigned lo,
+                                           unsigned hi, float (&v)[Q][8]) {
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     const unsigned pos = (unsigned)e[q].y;
     const bool ok = ((pos - lo) & (hi + 2 * kGuard - pos) & kGuard) == kGuard;
     ld8(ok ? base + e[q].x : g_zero_chunk, v[q]);
   }
+}
+template <int Q>
+__device__ __forceinline__ void table_load(const int2 *tab, int i, int d, int n, const float *base,
+                                           unsigned lo, unsigned hi, float (&v)[Q][8]) {
+  int2 e[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) e[q] = tab[min(i + q * d, n)];
+  entry_load<Q>(e, base, lo, hi, v);
 }
 
 // Convert and store those of pixels q*d < n at dst + q*d*16.
