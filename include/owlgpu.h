@@ -81,8 +81,9 @@ int owlgpu_last_conv_path(void);
 int owlgpu_device_status(void);
 /* Device ordinal used by the host drop-in entry points (default 0). */
 int owlgpu_set_device(int device);
-/* Release cached device/pinned staging memory held by the host drop-in,
- * and every cached weight image (below). */
+/* Release cached device/pinned staging memory held by the host drop-in, the
+ * workspaces that the library keeps for its calls (up to 256 MB a device) and
+ * every cached weight image (below). */
 int owlgpu_trim(void);
 /* Weight-image cache (no counterpart in Owl, whose stubs re-pack their
  * kernel operand on every call too).  The tensor-core convolutions re-lay

@@ -39,17 +39,19 @@ int cuda_fail(cudaError_t e, const char *where) {
 // pool gives everything back at each one, and a call after it then took 250-400
 // us longer to map its workspace again.  The bound covers the workspaces of the
 // measured layers (at most 40 MB each) on several streams at once; what is above
-// it goes back at the next synchronisation, and all of it when an allocation
-// fails.
+// it goes back at the next synchronisation, and all of it to owlgpu_trim and when an
+// allocation of the library fails.
 constexpr uint64_t kScratchKeep = 256ull << 20;
 
-static cudaMemPool_t scratch_pool() {
+// The scratch pool of device `dev` (-1: the current one), made when first asked for
+// unless `existing`; null when there is none.
+static cudaMemPool_t scratch_pool(int dev = -1, bool existing = false) {
   static cudaMemPool_t pools[64] = {};
   static std::mutex mu;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  if (dev < 0 && cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  if (dev < 0 || dev >= 64) return nullptr;
   std::lock_guard<std::mutex> lk(mu);
-  if (!pools[dev]) {
+  if (!pools[dev] && !existing) {
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -66,25 +68,25 @@ static cudaMemPool_t scratch_pool() {
   return pools[dev];
 }
 
+void trim_pools() {
+  int dev = 0;
+  cudaMemPool_t pool = scratch_pool(-1, true);
+  if (pool) cudaMemPoolTrimTo(pool, 0);
+  if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
+    cudaMemPoolTrimTo(pool, 0);
+  cudaGetLastError();
+}
+
 int scratch_alloc(void **p, size_t bytes, cudaStream_t s) {
   *p = nullptr;
   if (bytes == 0) return kOk;
   cudaMemPool_t pool = scratch_pool();
-  auto get = [&] {
+  const cudaError_t e = retry_trimmed([&] {
     return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
-  };
-  cudaError_t e = get();
-  if (e == cudaErrorMemoryAllocation && pool) {
-    cudaGetLastError();
-    cudaMemPoolTrimTo(pool, 0);
-    e = get();
-  }
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    *p = nullptr;
-    return cuda_fail(e, "cudaMallocAsync(scratch)");
-  }
-  return kOk;
+  });
+  if (e == cudaSuccess) return kOk;
+  *p = nullptr;
+  return cuda_fail(e, "cudaMallocAsync(scratch)");
 }
 
 // Memory that callers hold or that a host drop-in call stages its arrays in:
@@ -92,12 +94,10 @@ int scratch_alloc(void **p, size_t bytes, cudaStream_t s) {
 static int device_alloc(void **p, size_t bytes, cudaStream_t s) {
   *p = nullptr;
   if (bytes == 0) return kOk;
-  cudaError_t e = cudaMallocAsync(p, bytes, s);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return cuda_fail(e, "cudaMallocAsync");
-  }
-  return kOk;
+  const cudaError_t e = retry_trimmed([&] { return cudaMallocAsync(p, bytes, s); });
+  if (e == cudaSuccess) return kOk;
+  *p = nullptr;
+  return cuda_fail(e, "cudaMallocAsync");
 }
 
 void scratch_free(void *p, cudaStream_t s) {
@@ -678,6 +678,7 @@ int owlgpu_trim(void) {
   OWL_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
   OWL_CUDA(cudaDeviceSynchronize());
   OWL_CUDA(cudaMemPoolTrimTo(pool, 0));
+  if (cudaMemPool_t scratch = scratch_pool(dev, true)) OWL_CUDA(cudaMemPoolTrimTo(scratch, 0));
   return weights_drop_all();
 }
 int owlgpu_weights_declare(const void *kernel, uint64_t version) {

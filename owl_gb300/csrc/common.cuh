@@ -176,6 +176,21 @@ cudaError_t launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, 
 
 // Stream-ordered scratch allocation used by kernels that need workspace.
 int scratch_alloc(void **p, size_t bytes, cudaStream_t s);
+// Give back what the current device's pools keep and nothing uses: the scratch pool,
+// and the default pool, which the drop-in path has keep its staging memory.
+void trim_pools();
+// Run an allocation; when it lacks memory, once more after trim_pools().
+template <class F>
+cudaError_t retry_trimmed(F alloc) {
+  cudaError_t e = alloc();
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    trim_pools();
+    e = alloc();
+  }
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
 void scratch_free(void *p, cudaStream_t s);
 
 // ---- compute entry points (device pointers, asynchronous) --------------

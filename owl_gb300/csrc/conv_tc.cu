@@ -1562,13 +1562,11 @@ int run_segs(int prec, int nseg_in, const SegSpec *sp, bool bwd_input, int Ci, i
       if (!present && cudaStreamIsCapturing(s, &cs) == cudaSuccess &&
           cs == cudaStreamCaptureStatusNone) {
         void *buf = nullptr;
-        if (cudaMalloc(&buf, wt_bytes * parts) == cudaSuccess) {
+        if (retry_trimmed([&] { return cudaMalloc(&buf, wt_bytes * parts); }) == cudaSuccess) {
           g_images.push_back({key, ver, (uint8_t *)buf, wt_bytes * parts, false});
           cached = (uint8_t *)buf;
           build_cached = true;
-        } else {
-          cudaGetLastError();  // no room for an image: per-call scratch instead
-        }
+        }  // (else no room for an image: per-call scratch instead)
       }
     }
   }
