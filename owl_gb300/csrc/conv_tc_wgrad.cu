@@ -25,6 +25,7 @@
 
 #include <algorithm>
 #include <type_traits>
+#include <vector>
 
 #include "../../include/owlgpu.h"
 #include "common.cuh"
@@ -75,6 +76,11 @@ struct WgParams {
   int NS;
   unsigned idesc, tmem_cols;
   unsigned small_off;  // BF16X3: TMEM column of the cross-term accumulators (TG * BN)
+  // Accumulator sets, set_cols TMEM columns each: the pixel tiles go to them in turn and
+  // the epilogue adds them.  The tensor core rounds an accumulator toward zero at every
+  // MMA, so the error of a sum grows with its length, and sets shorten it for nothing.
+  int sets;
+  unsigned set_cols;
   int vec_x, vec_y;
   int pk_nch;  // PACK: chunk rows of a halo row (a power of two), else 16
   // LANES: floats from a tile's first pixel to the next tile's along v; from there
@@ -147,7 +153,9 @@ __host__ __device__ inline int chunk_row(int hvr, int nch) {
 // `pk` chunk rows of PSR pixels, so that one stride of PSR pixels walks the chunks of
 // a halo row and on into the next one's, the next tap's operand.  With a tap to an
 // MMA, 32 channels used a quarter of each: [4;32;32;32;32]x[3;3;3;32;64] took 77 us.
-template <int KIND, bool LANES, bool PACK>
+// SETS: several accumulator sets may be in use (a kernel of its own for whole chunks,
+// where the choice in the loops cost layers with one set 1 to 3 %).
+template <int KIND, bool LANES, bool PACK, bool SETS>
 __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_constant__ WgParams p) {
   constexpr int EB = (KIND == K_TF32) ? 4 : 2;
   constexpr int EPC = 16 / EB;
@@ -479,6 +487,7 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
       // (a warp reaches the TMEM lanes of its quadrant, warp % 4; the quadrant's
       // warps take every kEpiParts-th 16 columns)
       const int q = warp & 3;
+      const int n_sets = (int)min((long long)p.sets, t_end - t_begin);
       int mine = (warp - kEpiWarp0) >> 2;
       const int row = q * 32 + lane, pt = PACK ? row / (pk * 8) : 0;  // tap of the pack
       const int ci = PACK ? row - pt * pk * 8 : mb * 128 + row;
@@ -496,18 +505,27 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
               continue;
             }
             mine = kEpiParts - 1;
-            uint32_t rr[16];
-            tmem_ld16(tcol + (uint32_t)c0, rr);
-            if (SEP) {
-              uint32_t r2[16];
-              tmem_ld16(tcol + p.small_off + (uint32_t)c0, r2);
-              tmem_ld_wait();
+            uint32_t rr[16], r2[16];
+            auto add = [](uint32_t(&a)[16], const uint32_t(&b)[16]) {
 #pragma unroll
               for (int e = 0; e < 16; ++e)
-                rr[e] = __float_as_uint(__uint_as_float(rr[e]) + __uint_as_float(r2[e]));
-            } else {
+                a[e] = __float_as_uint(__uint_as_float(a[e]) + __uint_as_float(b[e]));
+            };
+            tmem_ld16(tcol + (uint32_t)c0, rr);
+            if (SEP) tmem_ld16(tcol + p.small_off + (uint32_t)c0, r2);
+            tmem_ld_wait();
+            for (int k = 1; SETS && k < n_sets; ++k) {
+              uint32_t more[16];
+              tmem_ld16(tcol + (uint32_t)k * p.set_cols + (uint32_t)c0, more);
               tmem_ld_wait();
+              add(rr, more);
+              if (SEP) {
+                tmem_ld16(tcol + (uint32_t)k * p.set_cols + p.small_off + (uint32_t)c0, more);
+                tmem_ld_wait();
+                add(r2, more);
+              }
             }
+            if (SEP) add(rr, r2);
             if (real) {
               const int n0 = nb * p.BN + c0;
               if (p.vec_y == 2 && n0 + 16 <= p.Co && ((uintptr_t)(out + c0) % 32 == 0)) {
@@ -544,17 +562,24 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
       const int nks = p.TP / KSTEP_PIX;
       // up to four taps' A offsets in registers (the common tap groups)
       const bool few = ntap <= 4;
-      uint32_t to[4], dc[4];
+      uint32_t to[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        to[i] = i < ntap ? tap_off[i] : 0u;
-        dc[i] = tmem_base + (uint32_t)(i * p.BN);
-      }
+      for (int i = 0; i < 4; ++i) to[i] = i < ntap ? tap_off[i] : 0u;
       int st = 0;
       uint32_t ph = 0;
       uint32_t acc = 0;
       bool ok = true;
+      int set = 0;
       for (long long t = t_begin; t < t_end; ++t) {
+        uint32_t d0 = tmem_base;
+        if (SETS) {
+          acc = t - t_begin >= p.sets;  // the first tile of a set overwrites it
+          d0 += (uint32_t)set * p.set_cols;
+          if (++set == p.sets) set = 0;
+        }
+        uint32_t dc[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dc[i] = d0 + (uint32_t)(i * p.BN);
         if (!poll_bar(smem_u32(&full[st]), ph, abort_flag, p.status, p.spin_limit)) {
           ok = false;
           break;
@@ -586,7 +611,7 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
           } else {
             for (int i = 0; i < ntap; ++i) {
               const uint64_t ad = xs_ + (uint64_t)tap_off[i];
-              const uint32_t d = tmem_base + (uint32_t)(i * p.BN);
+              const uint32_t d = d0 + (uint32_t)(i * p.BN);
               if (KIND == K_TF32) {
                 mma_tf32(lead, d, ad, bd, p.idesc, acc);
               } else {
@@ -621,7 +646,7 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
 // Estimated time of a plan in cycles, from a fit to 950 plans of twelve layers on
 // GB300 (3% off on average; the choice needs the ratios only).  A tile costs its
 // rounds of staging slots, its bytes and its MMAs, which overlap little; each wave
-// of CTAs an epilogue; the partial sums their writing and reading.
+// of CTAs a start and an epilogue; the partial sums their writing and reading.
 double estimate(const WgParams &p, int halo_pixels, int parts, long long ctas, int sms) {
   auto pow2 = [](int n) {
     int q = 1;
@@ -640,7 +665,7 @@ double estimate(const WgParams &p, int halo_pixels, int parts, long long ctas, i
                       p.TP / 16 * p.TG * (parts == 2 ? 3 : 1) * std::max(mma, 0.26 * p.BN);
   const double waves = (double)((ctas + sms - 1) / sms);
   const double sums = p.R > 1 ? 1.3e-3 * p.T * p.Ci * (double)p.Co * p.R : 0.0;
-  return waves * ((double)p.tiles_per_range * tile + 25.0 * p.TG * p.BN * parts) + sums;
+  return waves * ((double)p.tiles_per_range * tile + 25.0 * p.TG * p.BN * parts + 8e3) + sums;
 }
 
 int sm_count() {
@@ -663,18 +688,18 @@ int *status_word() {
   return p[dev];
 }
 
-template <int KIND, bool LANES, bool PACK>
+template <int KIND, bool LANES, bool PACK, bool SETS>
 int launch(const WgParams &p, size_t smem, int grid, cudaStream_t s) {
   static bool attr[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr[dev]) {
-    OWL_CUDA(cudaFuncSetAttribute(wgrad_tc_kernel<KIND, LANES, PACK>,
+    OWL_CUDA(cudaFuncSetAttribute(wgrad_tc_kernel<KIND, LANES, PACK, SETS>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
     attr[dev] = true;
   }
-  cudaError_t e = launch_pdl(wgrad_tc_kernel<KIND, LANES, PACK>, dim3(grid), dim3(kThreads), smem, s,
-                             p);
+  cudaError_t e = launch_pdl(wgrad_tc_kernel<KIND, LANES, PACK, SETS>, dim3(grid), dim3(kThreads),
+                             smem, s, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   note_launch();
   note_tc_launch();
@@ -804,6 +829,59 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
     p.TG = widest;
     return n;
   };
+  // The groupings by at most 16 taps and their groups' halos beyond a tile, those that
+  // lie within another left out.
+  struct Halo {
+    int w, u, v;
+  };
+  constexpr int kMaxHalos = 32;
+  struct Grouping {
+    int tg, n, widest, nh;  // asked for, groups, taps of the widest, halos
+    Halo halo[kMaxHalos];
+  } grouping[16];
+  int n_grouping = 0;
+  struct Reach {
+    int w, u, v, u1;  // a tap's offsets; PACK: the u offset of its pack's last tap
+  };
+  Reach few_taps[kMaxOrderedTaps];
+  std::vector<Reach> many_taps(p.T > kMaxOrderedTaps ? p.T : 0);
+  Reach *reach = p.T > kMaxOrderedTaps ? many_taps.data() : few_taps;
+  for (int t = 0; t < p.T; ++t) {
+    const int tu = t / p.KV, kv = t - tu * p.KV, kw = tu / p.KU, ku = tu - kw * p.KU;
+    const int last = pack ? ku + std::min(16 / p.pk_nch - 1, (p.KU - 1 - ku) / p.su) * p.su : ku;
+    reach[t] = {kw * p.dw, ku * p.du, kv * p.dv, last * p.du};
+  }
+  for (int tg = std::min(n_ent, 16); tg >= 1; --tg) {
+    const int n = make_groups(tg);
+    if (n_grouping > 0 && n == grouping[n_grouping - 1].n) continue;
+    Grouping &gr = grouping[n_grouping++];
+    gr.tg = tg;
+    gr.n = n;
+    gr.widest = p.TG;
+    gr.nh = 0;
+    for (int gi = 0; gi < n; ++gi) {
+      const int b0 = p.ordered ? p.gstart[gi] : gi * p.TG;
+      const int b1 = p.ordered ? p.gstart[gi + 1] : std::min(p.T, b0 + p.TG);
+      int mnw = 1 << 30, mnu = 1 << 30, mnv = 1 << 30, mxw = -1, mxu = -1, mxv = -1;
+      for (int i = b0; i < b1; ++i) {
+        const Reach &o = reach[p.ordered ? p.tap_order[i] : i];
+        mnw = std::min(mnw, o.w); mxw = std::max(mxw, o.w);
+        mnu = std::min(mnu, o.u); mxu = std::max(mxu, o.u1);
+        mnv = std::min(mnv, o.v); mxv = std::max(mxv, o.v);
+      }
+      const Halo h{(mxw - mnw) / p.sw + 1, (mxu - mnu) / p.su, (mxv - mnv) / p.sv};
+      bool seen = false;
+      for (int i = 0; i < gr.nh && !seen; ++i)
+        seen = gr.halo[i].w >= h.w && gr.halo[i].u >= h.u && gr.halo[i].v >= h.v;
+      if (seen) continue;
+      if (gr.nh < kMaxHalos) {
+        gr.halo[gr.nh++] = h;
+      } else {  // one that holds both
+        Halo &l = gr.halo[gr.nh - 1];
+        l = {std::max(l.w, h.w), std::max(l.u, h.u), std::max(l.v, h.v)};
+      }
+    }
+  }
   // Plan: BN output channels and TG taps per CTA (TG*BN <= 512 TMEM columns, or
   // 2*TG*BN with split-BF16's separate cross-term accumulators) and tiles of TU (even,
   // so that TU*8 pixels fill whole 16-pixel K steps) rows, two stages of which fit
@@ -820,92 +898,114 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
     if (t > 16 || t >= tu) continue;
     tus[ntu++] = tu = t;
   }
-  struct Halo {
-    int w, u, v;
-  };
-  constexpr int kMaxHalos = 32;
-  Halo halo[kMaxHalos];
   const long long rows = (long long)p.B * p.OW;
-  double least = -1;
-  int best_tg = 0, last_n = -1;
-  WgParams best = p;
-  for (int tg = std::min(n_ent, 16); tg >= 1; --tg) {
-    const int n = p.n_tg = make_groups(tg);
-    if (n == last_n) continue;
-    last_n = n;
-    // the groups' halos beyond a tile, those that lie within another left out
-    int nh = 0;
-    for (int gi = 0; gi < n; ++gi) {
-      const int b0 = p.ordered ? p.gstart[gi] : gi * p.TG;
-      const int b1 = p.ordered ? p.gstart[gi + 1] : std::min(p.T, b0 + p.TG);
-      int mnw = 1 << 30, mnu = 1 << 30, mnv = 1 << 30, mxw = -1, mxu = -1, mxv = -1;
-      for (int i = b0; i < b1; ++i) {
-        const int t = p.ordered ? p.tap_order[i] : i;
-        const int kv = t % p.KV, ku = (t / p.KV) % p.KU, kw = t / (p.KV * p.KU);
-        mnw = std::min(mnw, kw * p.dw); mxw = std::max(mxw, kw * p.dw);
-        mnu = std::min(mnu, ku * p.du);
-        mxu = std::max(
-            mxu, (pack ? ku + std::min(16 / p.pk_nch - 1, (p.KU - 1 - ku) / p.su) * p.su : ku) * p.du);
-        mnv = std::min(mnv, kv * p.dv); mxv = std::max(mxv, kv * p.dv);
-      }
-      const Halo h{(mxw - mnw) / p.sw + 1, (mxu - mnu) / p.su, (mxv - mnv) / p.sv};
-      bool seen = false;
-      for (int i = 0; i < nh && !seen; ++i)
-        seen = halo[i].w >= h.w && halo[i].u >= h.u && halo[i].v >= h.v;
-      if (seen) continue;
-      if (nh < kMaxHalos) {
-        halo[nh++] = h;
-      } else {  // one that holds both
-        Halo &l = halo[nh - 1];
-        l = {std::max(l.w, h.w), std::max(l.u, h.u), std::max(l.v, h.v)};
-      }
+  int HP = 0;  // pixels of the largest halo
+  // the sizes of one configuration, one wave of pixel ranges; false when it does not fit
+  auto fit = [&](const Grouping &gr, int bn, int tu, bool tables = true) {
+    p.n_tg = gr.n;
+    p.TG = gr.widest;
+    p.BN = std::min(bn, (p.Co + 15) / 16 * 16);
+    p.set_cols = (unsigned)(parts * p.TG * p.BN);
+    if (p.set_cols > 512) return false;
+    HP = 0;
+    int packed = 0;  // PACK: pixels of the largest halo's stage
+    for (int i = 0; i < gr.nh; ++i) {
+      const int hvr = 8 + gr.halo[i].v, hu = tu + gr.halo[i].u;
+      HP = std::max(HP, gr.halo[i].w * hu * hvr);
+      // (an MMA reads on past the last halo row, into rows of no tap)
+      if (pack)
+        packed = std::max(packed, (gr.halo[i].w * hu + 16 / p.pk_nch - 1) * p.pk_nch *
+                                          chunk_row(hvr, p.pk_nch) + 8);
     }
+    p.TU = tu;
+    p.TP = tu * 8;
+    p.YPS = p.TP + 1;
+    p.PS = HP + (((1 - HP) % 8) + 8) % 8;
+    if (p.PS >= 16384) return false;
+    if (packed >= 16384 || (packed > 0 && HP >= 65536)) return false;
+    p.x_bytes = pack ? (unsigned)((packed + 15) / 16 * 16) * 16u
+                     : (unsigned)(128 * EB / 16) * (unsigned)p.PS * 16u;
+    p.y_bytes = (unsigned)(p.BN * EB / 16) * (unsigned)p.YPS * 16u;
+    p.NS = 2;
+    p.n_tab = HP + p.TP;
+    const size_t need = (size_t)p.NS * parts * (p.x_bytes + p.y_bytes) + 256 +
+                        (tables ? 8 * (size_t)(p.n_tab + 3) + 2 * (size_t)p.n_tab : 0);
+    if (need > (size_t)kSmemMax) return false;
+    p.u_tiles = (p.OU + tu - 1) / tu;
+    p.v_tiles = (p.OV + 7) / 8;
+    p.total_tiles = rows * p.u_tiles * p.v_tiles;
+    p.n_nb = (p.Co + p.BN - 1) / p.BN;
+    return true;
+  };
+  auto set_ranges = [&](long long R) {
+    R = std::max<long long>(1, std::min(R, p.total_tiles));
+    p.tiles_per_range = (p.total_tiles + R - 1) / R;
+    p.R = (int)((p.total_tiles + p.tiles_per_range - 1) / p.tiles_per_range);
+  };
+  auto units = [&] { return (long long)p.n_tg * p.n_nb * p.n_mb; };
+  // MMAs that follow one another in an accumulator
+  auto chain = [&](int sets) {
+    const long long tiles =
+        sets == 1 ? p.tiles_per_range : (p.tiles_per_range + sets - 1) / sets;
+    return tiles * (p.TP / 16);
+  };
+  // The longest accumulation that is allowed, in MMAs: that of the widest block, the
+  // height that stages the fewest rows (a tile counts as four more) and the fewest
+  // groups, whose CTAs have about the most pixel ranges that fill the GPU once.  Plans by
+  // time alone took 1.3 to 4 times as many for split BF16, and its error, which is
+  // theirs, grew as much (64 x 7x7x512: 4.9e-6 to 6.7e-6 of the largest element, with
+  // values of one sign 3.3e-6 to 7.2e-6).  Beside the rounding of BF16's operands to 2^-9
+  // 128 MMAs (some 2^-17) do not show, nor does an eighth more.
+  long long shortest = -1;
+  int heights[8] = {14, 12, 10, 16, 8, 6, 4, 2};
+  long long staged[8];
+  for (int i = 0; i < 8; ++i) {  // sorted by the rows they stage
+    const int tu = heights[i];
+    const long long n =
+        (p.OU + tu - 1) / tu * (tu + 4LL) + (tu > kProducerWarps ? 1LL << 40 : 0);
+    int k = i;
+    for (; k > 0 && staged[k - 1] > n; --k) {
+      staged[k] = staged[k - 1];
+      heights[k] = heights[k - 1];
+    }
+    staged[k] = n;
+    heights[k] = tu;
+  }
+  for (int bn = 256; bn >= 16 && shortest < 0; bn /= 2)
+    for (int ti = 0; ti < 8 && shortest < 0; ++ti)
+      for (int gi = 0; gi < n_grouping && shortest < 0; ++gi)
+        if (fit(grouping[gi], bn, heights[ti], false)) {
+          set_ranges(sms / units());
+          shortest = chain(1);
+        }
+  const long long bound =
+      kind == K_BF16X3 ? shortest : std::max(shortest + shortest / 8, 128LL);
+  double least = -1;
+  int best_tg = 0;
+  WgParams best = p;
+  for (int gi = 0; gi < n_grouping; ++gi) {
     int last_bn = 0;
     for (int bn : {256, 128, 64, 32, 16}) {
-      p.BN = std::min(bn, (p.Co + 15) / 16 * 16);
-      if (p.BN == last_bn || parts * p.TG * p.BN > 512) continue;
+      if (std::min(bn, (p.Co + 15) / 16 * 16) == last_bn) continue;
       if (bn < 64 && least >= 0) continue;  // (narrow blocks waste the tensor core)
-      last_bn = p.BN;
       for (int ti = 0; ti < ntu; ++ti) {
-        const int tu = tus[ti];
-        int HP = 0, packed = 0;  // pixels of the largest halo; PACK: of its stage
-        for (int i = 0; i < nh; ++i) {
-          const int hvr = 8 + halo[i].v, hu = tu + halo[i].u;
-          HP = std::max(HP, halo[i].w * hu * hvr);
-          // (an MMA reads on past the last halo row, into rows of no tap)
-          if (pack)
-            packed = std::max(packed, (halo[i].w * hu + 16 / p.pk_nch - 1) * p.pk_nch *
-                                              chunk_row(hvr, p.pk_nch) + 8);
-        }
-        p.TU = tu;
-        p.TP = tu * 8;
-        p.YPS = p.TP + 1;
-        p.PS = HP + (((1 - HP) % 8) + 8) % 8;
-        if (p.PS >= 16384) continue;
-        if (packed >= 16384 || (packed > 0 && HP >= 65536)) continue;
-        p.x_bytes = pack ? (unsigned)((packed + 15) / 16 * 16) * 16u
-                         : (unsigned)(128 * EB / 16) * (unsigned)p.PS * 16u;
-        p.y_bytes = (unsigned)(p.BN * EB / 16) * (unsigned)p.YPS * 16u;
-        p.NS = 2;
-        p.n_tab = HP + p.TP;
-        const size_t need = (size_t)p.NS * parts * (p.x_bytes + p.y_bytes) + 256 +
-                            8 * (size_t)(p.n_tab + 3) + 2 * (size_t)p.n_tab;
-        if (need > (size_t)kSmemMax) continue;
-        p.u_tiles = (p.OU + tu - 1) / tu;
-        p.v_tiles = (p.OV + 7) / 8;
-        p.total_tiles = rows * p.u_tiles * p.v_tiles;
-        p.n_nb = (p.Co + p.BN - 1) / p.BN;
-        // pixel ranges: enough CTAs to fill the GPU once
-        const long long units = (long long)n * p.n_nb * p.n_mb;
-        long long R = std::min(std::max<long long>(1, sms / units), p.total_tiles);
-        p.tiles_per_range = (p.total_tiles + R - 1) / R;
-        R = (p.total_tiles + p.tiles_per_range - 1) / p.tiles_per_range;
-        p.R = (int)R;
-        const double t = estimate(p, HP, parts, units * R, sms);
+        if (!fit(grouping[gi], bn, tus[ti])) continue;
+        last_bn = p.BN;
+        // pixel ranges: enough CTAs to fill the GPU once; accumulator sets, which cost
+        // nothing, and beyond them ranges for several waves of CTAs where an accumulation
+        // is too long (each wave an epilogue more)
+        set_ranges(sms / units());
+        p.sets = 1;
+        while (chain(p.sets) > shortest && p.sets < p.tiles_per_range &&
+               2 * p.sets * p.set_cols <= 512)
+          p.sets *= 2;
+        for (int waves = 2; chain(p.sets) > bound && p.tiles_per_range > p.sets; ++waves)
+          set_ranges(std::max<long long>(waves, waves * sms / units()));
+        const double t = estimate(p, HP, parts, units() * p.R, sms);
         if (least < 0 || t < least) {
           least = t;
           best = p;
-          best_tg = tg;
+          best_tg = grouping[gi].tg;
         }
       }
     }
@@ -915,8 +1015,7 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
   p.n_tg = make_groups(best_tg);
   p.small_off = (unsigned)(p.TG * p.BN);
   p.tmem_cols = 32;
-  while (p.tmem_cols < (unsigned)(parts * p.TG * p.BN)) p.tmem_cols <<= 1;
-  const long long units = (long long)p.n_tg * p.n_nb * p.n_mb;
+  while (p.tmem_cols < p.set_cols * (unsigned)p.sets) p.tmem_cols <<= 1;
   uint32_t idesc = instr_desc(kind == K_TF32 ? 2u : 1u, (uint32_t)p.BN);
   idesc |= (1u << 15) | (1u << 16);  // A and B MN-major
   p.idesc = idesc;
@@ -938,7 +1037,7 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
   const size_t smem =
       (size_t)p.NS * parts * (p.x_bytes + p.y_bytes) + (2 * p.NS + 2) * 8 + 16 + 4 * (size_t)p.TG +
       8 * (size_t)(p.n_tab + 3) + 2 * (size_t)p.n_tab;
-  const int grid = (int)(units * p.R);
+  const int grid = (int)(units() * p.R);
   int rc;
   p.x_dv = 8LL * p.sv * p.xsv * p.Ci;
   p.x_du = (long long)p.TU * p.su * p.xsu * p.Ci - p.v_tiles * p.x_dv;
@@ -948,16 +1047,17 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
   p.y_du = (long long)p.TU * p.ysu * p.Co - p.v_tiles * p.y_dv;
   p.y_dw = p.ysw * p.Co - (long long)p.u_tiles * p.TU * p.ysu * p.Co;
   p.y_db = p.ysb * p.Co - (long long)p.OW * p.ysw * p.Co;
-  if (kind == K_BF16X3)
-    rc = lanes ? (pack ? launch<K_BF16X3, true, true>(p, smem, grid, s)
-                       : launch<K_BF16X3, true, false>(p, smem, grid, s))
-               : (pack ? launch<K_BF16X3, false, true>(p, smem, grid, s)
-                       : launch<K_BF16X3, false, false>(p, smem, grid, s));
-  else
-    rc = lanes ? (pack ? launch<K_BF16, true, true>(p, smem, grid, s)
-                       : launch<K_BF16, true, false>(p, smem, grid, s))
-               : (pack ? launch<K_BF16, false, true>(p, smem, grid, s)
-                       : launch<K_BF16, false, false>(p, smem, grid, s));
+  auto go = [&](auto k, auto packed) {
+    constexpr int KIND = decltype(k)::value;
+    constexpr bool PACK = decltype(packed)::value;
+    if (!lanes) return launch<KIND, false, PACK, true>(p, smem, grid, s);
+    return p.sets > 1 ? launch<KIND, true, PACK, true>(p, smem, grid, s)
+                      : launch<KIND, true, PACK, false>(p, smem, grid, s);
+  };
+  using X3 = std::integral_constant<int, K_BF16X3>;
+  using B1 = std::integral_constant<int, K_BF16>;
+  if (kind == K_BF16X3) rc = pack ? go(X3{}, std::true_type{}) : go(X3{}, std::false_type{});
+  else rc = pack ? go(B1{}, std::true_type{}) : go(B1{}, std::false_type{});
   if (rc == kOk && p.R > 1) rc = sum_partials_f32(part, dw, welems, p.R, s);
   if (part) scratch_free(part, s);
   return rc;
