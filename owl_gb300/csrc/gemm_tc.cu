@@ -20,6 +20,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "../../include/owlgpu.h"
 #include "common.cuh"
@@ -86,6 +87,11 @@ struct GemmParams {
   long long kps;              // k per split, a multiple of kBK
   unsigned a_bytes, b_bytes;  // one stage of each operand, per precision part
   unsigned idesc, tmem_cols, small_off;
+  // Accumulators of BN TMEM columns each: the k blocks go to them in turn and the epilogue
+  // adds them.  The tensor core rounds an accumulator toward zero at every MMA, so the
+  // error of a sum grows with its length, and sets shorten it for nothing.  (The one of
+  // BF16X3's cross terms, after them at small_off, holds 2^-8 of the sum.)
+  int sets;
   int *status;
   long long spin_limit;
 };
@@ -304,7 +310,8 @@ __device__ __forceinline__ bool stage_round(uint8_t *stage, uint32_t lo_a, uint3
   return true;
 }
 
-template <int KIND>
+// SETS: several accumulator sets.
+template <int KIND, bool SETS>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_constant__ GemmParams p) {
   constexpr int PARTS = (KIND == stage::K_BF16X3) ? 2 : 1;
   constexpr bool SEP = (KIND == stage::K_BF16X3);
@@ -406,18 +413,22 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         float *crow = p.c + (final_ ? 0 : (long long)blockIdx.z * p.M * p.N) + m * p.N;
         const uint32_t tcol = tmem_base + ((uint32_t)(q * 32) << 16);
         for (int c0 = 0; c0 < p.BN; c0 += 16) {
-          uint32_t r[16];
-          tmem_ld16(tcol + (uint32_t)c0, r);
-          if (SEP) {
-            uint32_t r2[16];
-            tmem_ld16(tcol + p.small_off + (uint32_t)c0, r2);
-            tmem_ld_wait();
+          uint32_t r[16], r2[16];
+          auto add = [](uint32_t(&a)[16], const uint32_t(&b)[16]) {
 #pragma unroll
             for (int e = 0; e < 16; ++e)
-              r[e] = __float_as_uint(__uint_as_float(r[e]) + __uint_as_float(r2[e]));
-          } else {
+              a[e] = __float_as_uint(__uint_as_float(a[e]) + __uint_as_float(b[e]));
+          };
+          tmem_ld16(tcol + (uint32_t)c0, r);
+          if (SEP) tmem_ld16(tcol + p.small_off + (uint32_t)c0, r2);
+          tmem_ld_wait();
+          for (int k = 1; SETS && k < min(p.sets, nkb); ++k) {
+            uint32_t more[16];
+            tmem_ld16(tcol + (uint32_t)(k * p.BN + c0), more);
             tmem_ld_wait();
+            add(r, more);
           }
+          if (SEP) add(r, r2);
           if (m < p.M) {
             const long long n = n0 + c0;
             float v[16];
@@ -457,11 +468,18 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     const uint32_t a_step = p.a_kmaj ? 2 * (kBM + 1) : 16,
                    b_step = p.b_kmaj ? 2 * (uint32_t)(p.BN + 1) : 16;
     const uint32_t alo = p.a_bytes >> 4, blo = p.b_bytes >> 4;
-    const uint32_t d = tmem_base, ds = tmem_base + p.small_off;
-    uint32_t acc = 0;
+    const uint32_t ds = tmem_base + p.small_off;
+    uint32_t acc = 0, acc_s = 0;
     bool ok = true;
+    int set = 0;
     for (int i = 0; i < nkb; ++i) {
       const int st = i % p.NS;
+      uint32_t d = tmem_base;
+      if (SETS) {
+        acc = i >= p.sets;  // the first block of a set overwrites it
+        d += (uint32_t)(set * p.BN);
+        if (++set == p.sets) set = 0;
+      }
       if (!poll_bar(smem_u32(&full[st]), (uint32_t)((i / p.NS) & 1), abort_flag, p.status,
                     p.spin_limit)) {
         ok = false;
@@ -475,8 +493,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         const uint64_t ad = ad0 + (uint64_t)(s * a_step), bd = bd0 + (uint64_t)(s * b_step);
         mma_bf16(lead, d, ad, bd, p.idesc, acc);
         if (SEP) {
-          mma_bf16(lead, ds, ad + (uint64_t)alo, bd, p.idesc, acc);
+          mma_bf16(lead, ds, ad + (uint64_t)alo, bd, p.idesc, SETS ? acc_s : acc);
           mma_bf16(lead, ds, ad, bd + (uint64_t)blo, p.idesc, 1);
+          acc_s = 1;
         }
         acc = 1;
       }
@@ -516,17 +535,17 @@ int num_sms() {
   return n > 0 ? n : 148;
 }
 
-template <int KIND>
+template <int KIND, bool SETS>
 int launch(const GemmParams &p, size_t smem, dim3 grid, cudaStream_t s) {
   static bool attr[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr[dev]) {
-    OWL_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kSmemMax));
+    OWL_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<KIND, SETS>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
     attr[dev] = true;
   }
-  cudaError_t e = launch_pdl(gemm_tc_kernel<KIND>, grid, dim3(kThreads), smem, s, p);
+  cudaError_t e = launch_pdl(gemm_tc_kernel<KIND, SETS>, grid, dim3(kThreads), smem, s, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   note_launch();
   note_tc_launch();
@@ -550,9 +569,18 @@ namespace {
 // always 256 wide and the split covered two waves: 256x1024x3136 (x w^T) took
 // 31.5 us in 208 CTAs of two k blocks each, 17.8 now; 3136x256x1024 31.6 and
 // 12.3, 256x3136x1024 17.8 and 15.8.
+//
+// No accumulation is longer than in 256-wide tiles split to cover two waves, each split
+// at least two k blocks: by time alone split BF16 took up to three times as many k
+// blocks in a row, and its error, which is theirs, grew as much (1024x1024x16384: 4.5e-6
+// to 6.3e-6 of the largest element; 2048^3 with values of one sign 1.8e-6 to 4.4e-6).
+// Four blocks (16 MMAs) do not show beside what split BF16 leaves out (3136x1024x256:
+// 5.0e-6 with two in a row and with four), nor beside the rounding of BF16's operands to
+// 2^-9 do 32 or an eighth more.
 struct Plan {
   int bn;
   long long kbs;  // k blocks per split
+  int sets;       // accumulator sets that the k blocks of a split go to in turn
 };
 
 Plan plan(long long M, long long N, long long nkb, long long mt, int parts) {
@@ -560,7 +588,13 @@ Plan plan(long long M, long long N, long long nkb, long long mt, int parts) {
   const double mma = (parts == 2 ? 3 : 1) * 4 * 0.085;
   const int sms = num_sms();
   const int n16 = (int)std::min<long long>(256, std::max<long long>(16, (N + 15) / 16 * 16));
-  Plan best{n16, nkb};
+  const long long tiles256 = mt * ((N + n16 - 1) / n16);
+  const long long splits256 = std::min<long long>(
+      std::min((2LL * sms + tiles256 - 1) / tiles256, std::max(1LL, nkb / 2)), 64);
+  const long long longest = (nkb + splits256 - 1) / splits256;
+  const long long bound =
+      parts == 2 ? std::max(longest, 4LL) : std::max(longest, 32LL) * 9 / 8;
+  Plan best{n16, longest, 1};
   double least = -1;
   for (int bn = n16; bn >= 16; bn = bn > 32 ? (bn - 1) / 32 * 32 : 0) {
     const long long tiles = mt * ((N + bn - 1) / bn);
@@ -568,12 +602,15 @@ Plan plan(long long M, long long N, long long nkb, long long mt, int parts) {
     for (long long splits = 1; splits <= std::min<long long>(nkb, 64); ++splits) {
       const long long kbs = (nkb + splits - 1) / splits, used = (nkb + kbs - 1) / kbs;
       if (used != splits) continue;
+      const long long sets =
+          std::max(1LL, std::min<long long>((kbs + bound - 1) / bound, 512 / bn - parts + 1));
+      if ((kbs + sets - 1) / sets > bound) continue;
       const long long waves = (tiles * splits + sms - 1) / sms;
       double t = waves * (kStart + kbs * kb + kBM * (double)bn * 4 / kStore);
       if (splits > 1) t += kSum + (splits + 1) * (double)M * N * 4 / kSumRate;
       if (least < 0 || t < least) {
         least = t;
-        best = {bn, kbs};
+        best = {bn, kbs, (int)sets};
       }
     }
   }
@@ -601,9 +638,10 @@ int gemm_run(int prec, GemmParams p, float *c, cudaStream_t s) {
   const long long nt = (N + p.BN - 1) / p.BN;
   p.kps = pl.kbs * kBK;
   p.splits = (int)((nkb + pl.kbs - 1) / pl.kbs);
-  p.small_off = (unsigned)p.BN;
+  p.sets = pl.sets;
+  p.small_off = (unsigned)(p.sets * p.BN);
   p.tmem_cols = 32;
-  while (p.tmem_cols < (unsigned)(parts * p.BN)) p.tmem_cols <<= 1;
+  while (p.tmem_cols < (unsigned)((p.sets + parts - 1) * p.BN)) p.tmem_cols <<= 1;
   p.idesc = instr_desc(1u, (uint32_t)p.BN) | ((p.a_kmaj ? 0u : 1u) << 15) |
             ((p.b_kmaj ? 0u : 1u) << 16);
   p.spin_limit = wait_limit();
@@ -622,8 +660,13 @@ int gemm_run(int prec, GemmParams p, float *c, cudaStream_t s) {
   }
   const size_t smem = (size_t)p.NS * stage_bytes + (2 * p.NS + 2) * 8 + 16;
   const dim3 grid((unsigned)mt, (unsigned)nt, (unsigned)p.splits);
-  int rc = kind == stage::K_BF16X3 ? launch<stage::K_BF16X3>(p, smem, grid, s)
-                                   : launch<stage::K_BF16>(p, smem, grid, s);
+  auto go = [&](auto k) {
+    constexpr int KIND = decltype(k)::value;
+    return p.sets > 1 ? launch<KIND, true>(p, smem, grid, s)
+                      : launch<KIND, false>(p, smem, grid, s);
+  };
+  int rc = kind == stage::K_BF16X3 ? go(std::integral_constant<int, stage::K_BF16X3>{})
+                                   : go(std::integral_constant<int, stage::K_BF16>{});
   if (rc == kOk && p.splits > 1)
     rc = sum_splits<float>(part, c, M * N, p.splits, bias, N, act, s);
   if (part) scratch_free(part, s);

@@ -1,7 +1,7 @@
 """Long sums in split BF16 against float64, at the mode's tolerance: <= 1e-5 of the
 largest element.  The tensor core rounds an accumulator toward zero at every MMA, so
 the error grows with the MMAs that one takes in turn; these are layers of many pixels
-and wide blocks."""
+and wide blocks, and products of long inner dimensions."""
 
 import pytest
 
@@ -41,3 +41,13 @@ def test_weight_gradient(gpu_lib, b, h, w, ci, co, k):
     ref = torch.stack([xp[:, i:i + h, j:j + w].reshape(-1, ci).T @ d
                        for i in range(k) for j in range(k)]).reshape(got.shape)
     assert rel(from_dev(got), from_dev(ref)) <= 1e-5
+
+
+@pytest.mark.parametrize("m,n,k", [(2048, 2048, 16384), (1024, 1024, 65536), (512, 1024, 3136)])
+def test_dense_product(gpu_lib, m, n, k):
+    from owl_gb300.dense import NN, GpuBackend
+    from owl_gb300.layers import Layers
+
+    a, b = _draw(m + n, (k, m), (k, n))
+    got = Layers(NN(GpuBackend("bf16x3"))).dot(a, b, trans_a=True)
+    assert rel(from_dev(got), from_dev(a.double().T @ b.double())) <= 1e-5
