@@ -75,10 +75,11 @@ struct WgParams {
   unsigned x_bytes, y_bytes;  // per stage, per precision part
   int NS;
   unsigned idesc, tmem_cols;
-  unsigned small_off;  // BF16X3: TMEM column of the cross-term accumulators (TG * BN)
-  // Accumulator sets, set_cols TMEM columns each: the pixel tiles go to them in turn and
-  // the epilogue adds them.  The tensor core rounds an accumulator toward zero at every
-  // MMA, so the error of a sum grows with its length, and sets shorten it for nothing.
+  unsigned small_off;  // BF16X3: TMEM column of the cross-term accumulators
+  // Accumulator sets, set_cols = TG * BN TMEM columns each: the pixel tiles go to them in
+  // turn and the epilogue adds them.  The tensor core rounds an accumulator toward zero at
+  // every MMA, so the error of a sum grows with its length, and sets shorten it for
+  // nothing.  (BF16X3's cross terms hold 2^-8 of a sum and have one set, the last.)
   int sets;
   unsigned set_cols;
   int vec_x, vec_y;
@@ -519,11 +520,6 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
               tmem_ld16(tcol + (uint32_t)k * p.set_cols + (uint32_t)c0, more);
               tmem_ld_wait();
               add(rr, more);
-              if (SEP) {
-                tmem_ld16(tcol + (uint32_t)k * p.set_cols + p.small_off + (uint32_t)c0, more);
-                tmem_ld_wait();
-                add(r2, more);
-              }
             }
             if (SEP) add(rr, r2);
             if (real) {
@@ -567,9 +563,10 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
       for (int i = 0; i < 4; ++i) to[i] = i < ntap ? tap_off[i] : 0u;
       int st = 0;
       uint32_t ph = 0;
-      uint32_t acc = 0;
+      uint32_t acc = 0, acc_s = 0;
       bool ok = true;
       int set = 0;
+      const uint32_t small0 = tmem_base + p.small_off;
       for (long long t = t_begin; t < t_end; ++t) {
         uint32_t d0 = tmem_base;
         if (SETS) {
@@ -602,8 +599,9 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
                 } else {
                   mma_bf16(lead, dc[i], ad, bd, p.idesc, acc);
                   if (KIND == K_BF16X3) {
-                    mma_bf16(lead, dc[i] + p.small_off, ad, bd + (uint64_t)ylo16, p.idesc, acc);
-                    mma_bf16(lead, dc[i] + p.small_off, ad + (uint64_t)xlo16, bd, p.idesc, 1);
+                    const uint32_t ds = SETS ? small0 + (uint32_t)(i * p.BN) : dc[i] + p.small_off;
+                    mma_bf16(lead, ds, ad, bd + (uint64_t)ylo16, p.idesc, SETS ? acc_s : acc);
+                    mma_bf16(lead, ds, ad + (uint64_t)xlo16, bd, p.idesc, 1);
                   }
                 }
               }
@@ -617,13 +615,14 @@ __global__ void __launch_bounds__(kThreads, 1) wgrad_tc_kernel(const __grid_cons
               } else {
                 mma_bf16(lead, d, ad, bd, p.idesc, acc);
                 if (KIND == K_BF16X3) {
-                  mma_bf16(lead, d + p.small_off, ad, bd + (uint64_t)ylo16, p.idesc, acc);
-                  mma_bf16(lead, d + p.small_off, ad + (uint64_t)xlo16, bd, p.idesc, 1);
+                  const uint32_t ds = SETS ? small0 + (uint32_t)(i * p.BN) : d + p.small_off;
+                  mma_bf16(lead, ds, ad, bd + (uint64_t)ylo16, p.idesc, SETS ? acc_s : acc);
+                  mma_bf16(lead, ds, ad + (uint64_t)xlo16, bd, p.idesc, 1);
                 }
               }
             }
           }
-          acc = 1;
+          acc = acc_s = 1;
         }
         mma_commit(lead, smem_u32(&empty[st]));
         if (++st == p.NS) { st = 0; ph ^= 1; }
@@ -905,8 +904,8 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
     p.n_tg = gr.n;
     p.TG = gr.widest;
     p.BN = std::min(bn, (p.Co + 15) / 16 * 16);
-    p.set_cols = (unsigned)(parts * p.TG * p.BN);
-    if (p.set_cols > 512) return false;
+    p.set_cols = (unsigned)(p.TG * p.BN);
+    if (parts * p.set_cols > 512) return false;
     HP = 0;
     int packed = 0;  // PACK: pixels of the largest halo's stage
     for (int i = 0; i < gr.nh; ++i) {
@@ -951,12 +950,13 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
   };
   // The longest accumulation that is allowed, in MMAs: that of the widest block, the
   // height that stages the fewest rows (a tile counts as four more) and the fewest
-  // groups, whose CTAs have about the most pixel ranges that fill the GPU once.  Plans by
-  // time alone took 1.3 to 4 times as many for split BF16, and its error, which is
-  // theirs, grew as much (64 x 7x7x512: 4.9e-6 to 6.7e-6 of the largest element, with
-  // values of one sign 3.3e-6 to 7.2e-6).  Beside the rounding of BF16's operands to 2^-9
-  // 128 MMAs (some 2^-17) do not show, nor does an eighth more.
-  long long shortest = -1;
+  // groups (PACK: those of single taps), whose CTAs have about the most pixel ranges that
+  // fill the GPU once.  Plans by time alone took 1.3 to 4 times as many for split BF16,
+  // and its error, which is theirs, grew as much (64 x 7x7x512: 4.9e-6 to 6.7e-6 of the
+  // largest element, with values of one sign 3.3e-6 to 7.2e-6).  16 MMAs do not show
+  // beside what split BF16 leaves out, nor 128 (some 2^-17) or an eighth more than either
+  // beside the rounding of BF16's operands to 2^-9.
+  long long bound = -1;
   int heights[8] = {14, 12, 10, 16, 8, 6, 4, 2};
   long long staged[8];
   for (int i = 0; i < 8; ++i) {  // sorted by the rows they stage
@@ -971,15 +971,16 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
     staged[k] = n;
     heights[k] = tu;
   }
-  for (int bn = 256; bn >= 16 && shortest < 0; bn /= 2)
-    for (int ti = 0; ti < 8 && shortest < 0; ++ti)
-      for (int gi = 0; gi < n_grouping && shortest < 0; ++gi)
+  for (int bn = 256; bn >= 16 && bound < 0; bn /= 2)
+    for (int ti = 0; ti < 8 && bound < 0; ++ti)
+      for (int gi = 0; gi < n_grouping && bound < 0; ++gi)
         if (fit(grouping[gi], bn, heights[ti], false)) {
-          set_ranges(sms / units());
-          shortest = chain(1);
+          const int tg = std::min(16, 512 / (parts * p.BN));
+          const long long groups = pack ? std::max(p.n_tg, (p.T + tg - 1) / tg) : p.n_tg;
+          set_ranges(sms / (groups * p.n_nb * p.n_mb));
+          bound = chain(1);
         }
-  const long long bound =
-      kind == K_BF16X3 ? shortest : std::max(shortest + shortest / 8, 128LL);
+  bound = kind == K_BF16X3 ? std::max(bound, 16LL) : std::max(bound, 128LL) * 9 / 8;
   double least = -1;
   int best_tg = 0;
   WgParams best = p;
@@ -995,10 +996,9 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
         // nothing, and beyond them ranges for several waves of CTAs where an accumulation
         // is too long (each wave an epilogue more)
         set_ranges(sms / units());
+        const long long most = std::min(512LL / p.set_cols - parts + 1, p.tiles_per_range);
         p.sets = 1;
-        while (chain(p.sets) > shortest && p.sets < p.tiles_per_range &&
-               2 * p.sets * p.set_cols <= 512)
-          p.sets *= 2;
+        while (chain(p.sets) > bound && p.sets < most) ++p.sets;
         for (int waves = 2; chain(p.sets) > bound && p.tiles_per_range > p.sets; ++waves)
           set_ranges(std::max<long long>(waves, waves * sms / units()));
         const double t = estimate(p, HP, parts, units() * p.R, sms);
@@ -1013,9 +1013,9 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
   if (least < 0) return kErrUnsupported;
   p = best;
   p.n_tg = make_groups(best_tg);
-  p.small_off = (unsigned)(p.TG * p.BN);
+  p.small_off = p.set_cols * (unsigned)p.sets;
   p.tmem_cols = 32;
-  while (p.tmem_cols < p.set_cols * (unsigned)p.sets) p.tmem_cols <<= 1;
+  while (p.tmem_cols < p.set_cols * (unsigned)(p.sets + parts - 1)) p.tmem_cols <<= 1;
   uint32_t idesc = instr_desc(kind == K_TF32 ? 2u : 1u, (uint32_t)p.BN);
   idesc |= (1u << 15) | (1u << 16);  // A and B MN-major
   p.idesc = idesc;
