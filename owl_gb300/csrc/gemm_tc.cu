@@ -222,10 +222,13 @@ __device__ __forceinline__ void ld8(const float *p, float (&v)[8]) {
 
 // A thread's slots, resolved once per tile: where slot q's 8 floats of the
 // first k block are, how far they move per k block, and its destination.
-// A slot whose row lies outside the matrix has base == nullptr (zeros).
+// A slot whose row lies outside the matrix has base == nullptr (zeros); bit q of `half`
+// is set when the matrix ends after the first four of slot q's rows (MN-major, rows 4
+// mod 8).
 struct Slots {
   const float *base[kQ];
   int off[kQ];
+  unsigned half;
   long long step_a, step_b;  // per k block, operand A's slots and B's
 };
 
@@ -250,6 +253,14 @@ __device__ __forceinline__ void slot_plan(const Operand &o, int sl, long long k_
   }
 }
 
+// The source of an MN-major slot that the matrix ends in after four rows, else nullptr.
+__device__ __forceinline__ const float *half_slot(const Operand &o, int sl, long long k_begin) {
+  const int nj = o.R >> 3;
+  const int kk = sl / nj, j = sl - kk * nj;
+  const long long row = o.row0 + 8 * j;
+  return row + 4 == o.rows ? o.src + (k_begin + kk) * o.s_k + row : nullptr;
+}
+
 // A whole stage (both operands) in one round per thread: every load of the
 // stage is issued first (up to kQ slots per thread, 2 x 16-byte loads
 // each), then `ready()` waits for the stage's buffer to be free, then the
@@ -258,7 +269,7 @@ __device__ __forceinline__ void slot_plan(const Operand &o, int sl, long long k_
 // through their strides and every source is 16-byte aligned, so each slot
 // is two vector loads at base + i*step; otherwise each slot is resolved in
 // full (matrix edges, the window gather).
-template <int KIND, class Ready>
+template <int KIND, bool HALF, class Ready>
 __device__ __forceinline__ bool stage_round(uint8_t *stage, uint32_t lo_a, uint32_t lo_b,
                                             const Operand &A, const Operand &B, long long k0,
                                             long long kend, const S2D &g, int tid,
@@ -279,7 +290,8 @@ __device__ __forceinline__ bool stage_round(uint8_t *stage, uint32_t lo_a, uint3
           ld8(src, v[q]);
         } else {
           const float4 *p4 = reinterpret_cast<const float4 *>(src);
-          const float4 x0 = __ldg(p4), x1 = __ldg(p4 + 1);
+          const float4 x0 = __ldg(p4);
+          const float4 x1 = HALF && ((sp.half >> q) & 1u) ? float4{} : __ldg(p4 + 1);
           v[q][0] = x0.x; v[q][1] = x0.y; v[q][2] = x0.z; v[q][3] = x0.w;
           v[q][4] = x1.x; v[q][5] = x1.y; v[q][6] = x1.z; v[q][7] = x1.w;
         }
@@ -310,8 +322,9 @@ __device__ __forceinline__ bool stage_round(uint8_t *stage, uint32_t lo_a, uint3
   return true;
 }
 
-// SETS: several accumulator sets.
-template <int KIND, bool SETS>
+// SETS: several accumulator sets.  HALF: an MN-major operand of 4 mod 8 rows, its last
+// chunk half outside (kernels of their own: the choice cost 1000^3 17.7 to 18.3 us).
+template <int KIND, bool SETS, bool HALF>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_constant__ GemmParams p) {
   constexpr int PARTS = (KIND == stage::K_BF16X3) ? 2 : 1;
   constexpr bool SEP = (KIND == stage::K_BF16X3);
@@ -367,6 +380,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     const int na = 8 * kBM, total = na + 8 * p.BN;
     sp.step_a = slot_step(A);
     sp.step_b = slot_step(B);
+    sp.half = 0;
 #pragma unroll
     for (int q = 0; q < kQ; ++q) {
       const int sl = tid + q * kProducerThreads;
@@ -375,15 +389,32 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
       if (sl < na) slot_plan(A, sl, k_begin, sp.base[q], sp.off[q]);
       else if (sl < total) slot_plan(B, sl - na, k_begin, sp.base[q], sp.off[q]);
     }
+    const bool half_a = !p.a_kmaj && p.M % 8 == 4 && m0 + kBM > p.M,
+               half_b = !p.b_kmaj && p.N % 8 == 4 && n0 + p.BN > p.N;
+    if (HALF && (half_a || half_b)) {
+#pragma unroll
+      for (int q = 0; q < kQ; ++q) {
+        const int sl = tid + q * kProducerThreads;
+        const float *src = nullptr;
+        if (half_a && sl < na) src = half_slot(A, sl, k_begin);
+        if (half_b && sl >= na && sl < total) src = half_slot(B, sl - na, k_begin);
+        if (src) {
+          sp.base[q] = src;
+          sp.half |= 1u << q;
+        }
+      }
+    }
     // plain strided operands whose rows start 16-byte aligned and, MN-major,
-    // fill whole 8-row chunks (the fast path: its slots load whole chunks)
-    const bool aligned = !p.s2d.on && (p.a_kmaj || p.M % 8 == 0) &&
-                         (p.b_kmaj || p.N % 8 == 0) && ((uintptr_t)p.a & 15) == 0 &&
+    // fill whole 8-row chunks, or halves (the fast path)
+    constexpr int kRows = HALF ? 4 : 8;
+    const bool aligned = !p.s2d.on && (p.a_kmaj || p.M % kRows == 0) &&
+                         (p.b_kmaj || p.N % kRows == 0) && ((uintptr_t)p.a & 15) == 0 &&
                          ((uintptr_t)p.b & 15) == 0 &&
                          (p.a_kmaj ? p.a_sm % 4 == 0 : p.a_sk % 4 == 0) &&
                          (p.b_kmaj ? p.b_sn % 4 == 0 : p.b_sk % 4 == 0);
     // ... and 32-byte aligned: one 32-byte load per slot
-    const bool wide = aligned && ((uintptr_t)p.a & 31) == 0 && ((uintptr_t)p.b & 31) == 0 &&
+    const bool wide = aligned && (p.a_kmaj || p.M % 8 == 0) && (p.b_kmaj || p.N % 8 == 0) &&
+                      ((uintptr_t)p.a & 31) == 0 && ((uintptr_t)p.b & 31) == 0 &&
                       (p.a_kmaj ? p.a_sm % 8 == 0 : p.a_sk % 8 == 0) &&
                       (p.b_kmaj ? p.b_sn % 8 == 0 : p.b_sk % 8 == 0);
     for (int i = 0; i < nkb; ++i) {
@@ -391,7 +422,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
       uint8_t *stg = smem + (size_t)st * stage_bytes;
       const long long k0 = k_begin + (long long)i * kBK;
       const bool fast = aligned && k0 + kBK <= k_end;
-      if (!stage_round<KIND>(stg, p.a_bytes, p.b_bytes, A, B, k0, k_end, p.s2d, tid, sp, fast,
+      if (!stage_round<KIND, HALF>(stg, p.a_bytes, p.b_bytes, A, B, k0, k_end, p.s2d, tid, sp, fast,
                              wide, i,
                              [&] {
             return wait_bar_warp(smem_u32(&empty[st]), (uint32_t)(((i / p.NS) & 1) ^ 1), abort_flag,
@@ -535,17 +566,17 @@ int num_sms() {
   return n > 0 ? n : 148;
 }
 
-template <int KIND, bool SETS>
+template <int KIND, bool SETS, bool HALF>
 int launch(const GemmParams &p, size_t smem, dim3 grid, cudaStream_t s) {
   static bool attr[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr[dev]) {
-    OWL_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<KIND, SETS>,
+    OWL_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<KIND, SETS, HALF>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
     attr[dev] = true;
   }
-  cudaError_t e = launch_pdl(gemm_tc_kernel<KIND, SETS>, grid, dim3(kThreads), smem, s, p);
+  cudaError_t e = launch_pdl(gemm_tc_kernel<KIND, SETS, HALF>, grid, dim3(kThreads), smem, s, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   note_launch();
   note_tc_launch();
@@ -662,8 +693,10 @@ int gemm_run(int prec, GemmParams p, float *c, cudaStream_t s) {
   const dim3 grid((unsigned)mt, (unsigned)nt, (unsigned)p.splits);
   auto go = [&](auto k) {
     constexpr int KIND = decltype(k)::value;
-    return p.sets > 1 ? launch<KIND, true>(p, smem, grid, s)
-                      : launch<KIND, false>(p, smem, grid, s);
+    if ((!p.a_kmaj && M % 8 == 4) || (!p.b_kmaj && N % 8 == 4))
+      return launch<KIND, true, true>(p, smem, grid, s);
+    return p.sets > 1 ? launch<KIND, true, false>(p, smem, grid, s)
+                      : launch<KIND, false, false>(p, smem, grid, s);
   };
   int rc = kind == stage::K_BF16X3 ? go(std::integral_constant<int, stage::K_BF16X3>{})
                                    : go(std::integral_constant<int, stage::K_BF16>{});
