@@ -891,11 +891,12 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
   // 7x7x512 72 where they take 46, and [64;56;56;128]x[3;3;128;128] at rate 2 in
   // split BF16, one tap per CTA, 250 where TU = 8 and two taps take 194.
   const int sms = sm_count();
-  int tus[8], ntu = 0;  // the heights that leave the fewest rows past the output
-  for (int tiles = 1, tu = 17; ntu < 5 && tu > 2; ++tiles) {
-    const int t = std::max(2, (p.OU + tiles - 1) / tiles + 1) / 2 * 2;
-    if (t > 16 || t >= tu) continue;
-    tus[ntu++] = tu = t;
+  // heights, tallest first: those that leave the fewest rows past the output, the least
+  // even ones that some number of tiles needs
+  int tus[8], ntu = 0;
+  for (int tu = 16; tu >= 2 && ntu < 5; tu -= 2) {
+    const int tiles = (p.OU + tu - 1) / tu;
+    if (std::max(2, (p.OU + tiles - 1) / tiles + 1) / 2 * 2 == tu) tus[ntu++] = tu;
   }
   const long long rows = (long long)p.B * p.OW;
   int HP = 0;  // pixels of the largest halo
