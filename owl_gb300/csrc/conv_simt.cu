@@ -954,7 +954,9 @@ int launch_any(const Dev &d, const T *A, const T *B, T *C, int splits, int64_t k
   }
 }
 
-// The tile that the split count of a reduction is planned for.
+// The tile that the split count of a reduction is planned for, not one that is
+// launched: the vector kernel's are smaller, several to an SM (four waves of these are
+// enough of those), and the FP64 ones follow the split count.
 template <typename T>
 int tile_m(const Dev &d) { return sizeof(T) == 4 ? (d.N <= 32 ? 256 : 128) : 64; }
 template <typename T>
