@@ -1304,6 +1304,7 @@ bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const P
             best = q;
           }
         }
+  if (least < 0) return false;
   p = best;
   return true;
 }
