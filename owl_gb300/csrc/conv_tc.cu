@@ -1267,7 +1267,7 @@ bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const P
   // it (3x3 at rate 36) the first that fits beside the row table, and where a position
   // does not fit the tables' fields, without one.  (TF32 halos are staged element by
   // element, and where nothing fits beside a pixel table the CUDA cores are faster:
-  // [4;65;65;256]x[3;3;256;256] at rate 36 takes 1360 us here and 442 there.)
+  // [4;65;65;256]x[3;3;256;256] at rate 35 takes 1363 us here and 443 there.)
   TcParams q;
   int cb = 0, form = 0, stage = S_PIXELS;
   for (;;) {
@@ -1287,9 +1287,11 @@ bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const P
   // a pixel's place costs a few instructions more, low tiles far more.  The same layer
   // in BF16 at rate 25 takes 99 us with one stage and TU = 18, 960 with TU = 2, and at
   // rate 34 197 us from the row table, 1210 from the pixel table and TU = 2.
+  // (Elsewhere operands that are staged element by element keep the pixel table's plan.)
   const bool tight = form >= 2 || stage != S_PIXELS;
+  const bool table = chunks && kind != K_TF32;
   if (tight) lone_slot = kLoneSlot;
-  int stages[2] = {chunks && kind != K_TF32 ? stage : S_ELEMENT, S_ROWS};
+  int stages[2] = {table || !tight ? stage : S_ELEMENT, S_ROWS};
   const int nstages = tight && stages[0] == S_PIXELS ? 2 : 1;
   double least = -1;
   TcParams best = p;
@@ -1306,6 +1308,7 @@ bool plan(TcParams &p, const View &v, int kind, int t_slot, int t_table, const P
         }
   if (least < 0) return false;
   p = best;
+  if (!table) p.stage = S_ELEMENT;
   return true;
 }
 
