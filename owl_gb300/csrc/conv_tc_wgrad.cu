@@ -954,9 +954,13 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
   // groups (PACK: those of single taps), whose CTAs have about the most pixel ranges that
   // fill the GPU once.  Plans by time alone took 1.3 to 4 times as many for split BF16,
   // and its error, which is theirs, grew as much (64 x 7x7x512: 4.9e-6 to 6.7e-6 of the
-  // largest element, with values of one sign 3.3e-6 to 7.2e-6).  16 MMAs do not show
-  // beside what split BF16 leaves out, nor 128 (some 2^-17) or an eighth more than either
-  // beside the rounding of BF16's operands to 2^-9.
+  // largest element, with values of one sign 3.3e-6 to 7.2e-6).  What does not show is
+  // allowed: beside what split BF16 leaves out (4e-6) 16 MMAs, or an eighth more than the
+  // bound up to 128; beside the rounding of BF16's operands to 2^-9 144 MMAs, or a
+  // quarter more up to 512 ([53;68;11;144]x[3;3;144;192]: 315 instead of 252 in a row give
+  // 2.65e-5 instead of 2.62e-5 rms with values of one sign, the same with both).  Held to
+  // the bound itself [15;15;101;112]x[3;3;112;208] in split BF16 took 61 us instead of
+  // 43, for 100 MMAs instead of 104.
   long long bound = -1;
   int heights[8] = {14, 12, 10, 16, 8, 6, 4, 2};
   long long staged[8];
@@ -981,7 +985,8 @@ int tc_conv_bwd_kernel(int prec, const ConvGeom &g, const float *x, float *dw, c
           set_ranges(sms / (groups * p.n_nb * p.n_mb));
           bound = chain(1);
         }
-  bound = kind == K_BF16X3 ? std::max(bound, 16LL) : std::max(bound, 128LL) * 9 / 8;
+  bound = kind == K_BF16X3 ? std::max({bound, std::min(bound * 9 / 8, 128LL), 16LL})
+                           : std::max({bound, std::min(bound * 5 / 4, 512LL), 144LL});
   double least = -1;
   int best_tg = 0;
   WgParams best = p;
